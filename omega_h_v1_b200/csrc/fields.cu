@@ -67,50 +67,129 @@ __device__ void invert_jacobian(u32 dim, double in[3][3], double out[3][3])
   }
 }
 
-__global__ void k_element_gradients(u32 dim, u32 ne, u32 const* __restrict__ voe,
+// Gradients of one element's fields: the inverse Jacobian and, per component,
+// the sum over the edges from vertex 0 in their order (element_gradients.cpp).
+// NC: the components at compile time (0: nc of them), so that a gradient is
+// summed in registers; `put` takes value k of the element's nc * 3.
+template <u32 NC, class Put>
+__device__ inline void element_gradient(u32 dim, u32 const* ve, double const* __restrict__ x,
+    u32 nc_any, double const* __restrict__ f, Put put)
+{
+  u32 const vpe = dim + 1, nc = NC ? NC : nc_any;
+  double ex[4][3];
+#pragma unroll
+  for (u32 j = 0; j < 4; ++j)
+    if (j < vpe) load3(x, ve[j], ex[j]);
+  // element_jacobian: column j is x[j+1] - x[0]
+  double jac[3][3];
+#pragma unroll
+  for (u32 a = 0; a < 3; ++a)
+#pragma unroll
+    for (u32 b = 0; b < 3; ++b) jac[b][a] = a < dim ? ex[a + 1][b] - ex[0][b] : 0;
+  double jaci[3][3];
+  invert_jacobian(dim, jac, jaci);
+#pragma unroll
+  for (u32 k = 0; k < (NC ? NC : nc); ++k) {
+    double fv[4];
+#pragma unroll
+    for (u32 j = 0; j < 4; ++j) fv[j] = j < vpe ? f[(size_t)ve[j] * nc + k] : 0;
+#pragma unroll
+    for (u32 l = 0; l < 3; ++l) {
+      double g = 0;
+#pragma unroll
+      for (u32 j = 0; j < 3; ++j)
+        if (j < dim) g += jaci[j][l] * (fv[j + 1] - fv[0]);
+      put(k * 3 + l, g);
+    }
+  }
+}
+
+// A thread per element. Bound by the write of the gradients (24 nc bytes an
+// element) once they are written a block at a time through shared memory:
+// a thread writing its own element's values put 32 lanes 24 nc bytes apart
+// in every store, and the running sums were kept in the output array, read
+// and written again for each edge (1.57M tets: nc = 1 and 3 took 418 us
+// together, now 79 us, 33 us of it the bytes at copy rate).
+constexpr u32 GRAD_BLOCK = 128;
+
+template <u32 DIM, u32 NC>
+__global__ void __launch_bounds__(GRAD_BLOCK) k_element_gradients(u32 ne,
+    u32 const* __restrict__ voe, double const* __restrict__ x, double const* __restrict__ f,
+    double* __restrict__ out)
+{
+  pdl_wait();
+  __shared__ double s_out[GRAD_BLOCK * NC * 3];
+  u32 const first = blockIdx.x * GRAD_BLOCK, i = first + threadIdx.x;
+  if (i < ne) {
+    u32 ve[DIM + 1];
+#pragma unroll
+    for (u32 j = 0; j <= DIM; ++j) ve[j] = voe[(size_t)i * (DIM + 1) + j];
+    double* mine = s_out + threadIdx.x * (NC * 3);  // (an odd stride: no bank conflicts)
+    element_gradient<NC>(DIM, ve, x, NC, f, [&](u32 k, double g) { mine[k] = g; });
+  }
+  __syncthreads();
+  u32 const n = (ne - first < GRAD_BLOCK ? ne - first : GRAD_BLOCK) * NC * 3;
+  double* o = out + (size_t)first * (NC * 3);
+  for (u32 k = threadIdx.x; k < n; k += GRAD_BLOCK) o[k] = s_out[k];
+}
+
+// any number of components and dimensions 1 to 3
+__global__ void k_element_gradients_any(u32 dim, u32 ne, u32 const* __restrict__ voe,
     double const* __restrict__ x, u32 nc, double const* __restrict__ f,
     double* __restrict__ out)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ne) return;
-  u32 vpe = dim + 1;
-  u32 const* ve = voe + (size_t)i * vpe;
-  double ex[4][3];
-  for (u32 j = 0; j < vpe; ++j) load3(x, ve[j], ex[j]);
-  // element_jacobian: column j is x[j+1] - x[0]
-  double jac[3][3];
-  for (u32 a = 0; a < 3; ++a)
-    for (u32 b = 0; b < 3; ++b) jac[a][b] = 0;
-  for (u32 a = 0; a < dim; ++a)
-    for (u32 b = 0; b < 3; ++b) jac[b][a] = ex[a + 1][b] - ex[0][b];
-  double jaci[3][3];
-  invert_jacobian(dim, jac, jaci);
   double* g = out + (size_t)i * nc * 3;
-  for (u32 k = 0; k < nc * 3; ++k) g[k] = 0;
-  for (u32 j = 0; j < dim; ++j)
-    for (u32 k = 0; k < nc; ++k)
-      for (u32 l = 0; l < 3; ++l)
-        g[k * 3 + l] += jaci[j][l] * (f[(size_t)ve[j + 1] * nc + k] - f[(size_t)ve[0] * nc + k]);
+  element_gradient<0>(dim, voe + (size_t)i * (dim + 1), x, nc, f,
+      [&](u32 k, double v) { g[k] = v; });
 }
 
-__global__ void k_recover_by_volume(u32 nv, u32 const* __restrict__ offs,
+// A thread per vertex and component: the nc lanes of a vertex read an
+// element's nc values side by side (and its size and id from one address),
+// and each component is summed over the row in its order, as the reference
+// sums it. RECOVER_BATCH elements' loads are issued before any is used:
+// the gathers' latency bounds the kernel, the sums are short. (A thread per
+// vertex kept its nc sums in the output array, with 32 rows' gathers in
+// every load: 1.57M tets, nc = 3 and 9 took 771 us together, now
+// 119 us, 38 us of it the bytes at copy rate.)
+constexpr u32 RECOVER_BATCH = 4;
+
+__global__ void __launch_bounds__(BLOCK) k_recover_by_volume(u32 nv, u32 const* __restrict__ offs,
     u32 const* __restrict__ adj, double const* __restrict__ sizes, u32 nc,
     double const* __restrict__ f, double* __restrict__ out)
 {
   pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+  u64 const t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  u32 const i = (u32)(t / nc), c = (u32)(t - (u64)i * nc);
   if (i >= nv) return;
-  double* o = out + (size_t)i * nc;
-  for (u32 k = 0; k < nc; ++k) o[k] = 0;
-  double size_sum = 0;
-  for (u32 j = offs[i]; j < offs[i + 1]; ++j) {
-    u32 e = adj[j];
-    double es = sizes[e];
-    size_sum += es;
-    for (u32 k = 0; k < nc; ++k) o[k] += es * f[(size_t)e * nc + k];
+  double sum = 0, size_sum = 0;
+  u32 const e1 = offs[i + 1];
+  u32 j = offs[i];
+  for (; j + RECOVER_BATCH <= e1; j += RECOVER_BATCH) {
+    u32 e[RECOVER_BATCH];
+    double es[RECOVER_BATCH], fe[RECOVER_BATCH];
+#pragma unroll
+    for (u32 k = 0; k < RECOVER_BATCH; ++k) e[k] = adj[j + k];
+#pragma unroll
+    for (u32 k = 0; k < RECOVER_BATCH; ++k) {
+      es[k] = sizes[e[k]];
+      fe[k] = f[(size_t)e[k] * nc + c];
+    }
+#pragma unroll
+    for (u32 k = 0; k < RECOVER_BATCH; ++k) {
+      size_sum += es[k];
+      sum += es[k] * fe[k];
+    }
   }
-  for (u32 k = 0; k < nc; ++k) o[k] /= size_sum;
+  for (; j < e1; ++j) {
+    u32 const e = adj[j];
+    double const es = sizes[e];
+    size_sum += es;
+    sum += es * f[(size_t)e * nc + c];
+  }
+  out[t] = sum / size_sum;
 }
 
 __global__ void k_size_from_hessian(u32 nv, u32 nhc, double const* __restrict__ hess,
@@ -172,8 +251,19 @@ void element_gradients(Mesh& m, char const* name)
   u32 dim = m.dim, ne = m.count(dim), nc = t->ncomps;
   double* out = dalloc<double>((size_t)ne * nc * 3, s);
   if (ne) {
-    CK(launch_kernel(k_element_gradients, dim3(grid_for(ne)), dim3(BLOCK), 0, s, dim, ne, m.ask_down(dim, 0), m.coords(),
-        nc, static_cast<double const*>(t->data), out));
+    u32 const* voe = m.ask_down(dim, 0);
+    double const* f = static_cast<double const*>(t->data);
+    // the components of a scalar and of its gradient, in 2D and 3D (the
+    // size-field chain's); any other count goes a thread per element
+    auto k = dim == 3 ? (nc == 1 ? k_element_gradients<3, 1> : nc == 3 ? k_element_gradients<3, 3> : nullptr)
+           : dim == 2 ? (nc == 1 ? k_element_gradients<2, 1> : nc == 3 ? k_element_gradients<2, 3> : nullptr)
+                      : nullptr;
+    if (k)
+      CK(launch_kernel(k, dim3(grid_for(ne, GRAD_BLOCK)), dim3(GRAD_BLOCK), 0, s, ne, voe,
+          m.coords(), f, out));
+    else
+      CK(launch_kernel(k_element_gradients_any, dim3(grid_for(ne)), dim3(BLOCK), 0, s, dim, ne,
+          voe, m.coords(), nc, f, out));
     CK_LAUNCH();
   }
   m.add_tag(dim, T_F64, (std::string("grad_") + name).c_str(), nc * 3, X_NOT, out);
@@ -189,9 +279,9 @@ void recover_by_volume(Mesh& m, char const* name)
   UpAdj const& ve = m.ask_up(0, dim, true);
   double* sizes = m.element_sizes();
   double* out = dalloc<double>((size_t)nv * nc, s);
-  if (nv) {
-    CK(launch_kernel(k_recover_by_volume, dim3(grid_for(nv)), dim3(BLOCK), 0, s, nv, ve.offs, ve.adj, sizes, nc,
-        static_cast<double const*>(m.find_tag(dim, name)->data), out));
+  if (nv && nc) {
+    CK(launch_kernel(k_recover_by_volume, dim3(grid_for((u64)nv * nc)), dim3(BLOCK), 0, s, nv, ve.offs,
+        ve.adj, sizes, nc, static_cast<double const*>(m.find_tag(dim, name)->data), out));
     CK_LAUNCH();
   }
   dev_free(sizes, s);
