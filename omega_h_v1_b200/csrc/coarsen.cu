@@ -10,39 +10,54 @@ namespace osh {
 
 __device__ inline u32 collapses(u32 code, u32 dir) { return (code >> dir) & 1u; }
 
-// coarsen_size_code (coarsen.cpp:13-21) fused with measure_edge
-__global__ void k_coarsen_size_codes(u32 ne, u32 const* __restrict__ voe,
-    double const* __restrict__ x, double const* __restrict__ h, double size_floor,
-    SegView sv, Fp32Stats* fs, u32* __restrict__ codes, u32* any)
+// coarsen_size_code (coarsen.cpp:13-21) fused with measure_edge; a block
+// takes CODE_TILE edges, CODE_UNROLL to a thread with their loads issued
+// together (as the refinement's candidate kernel)
+constexpr u32 CODE_UNROLL = 4, CODE_TILE = CODE_UNROLL * BLOCK;
+
+__global__ void __launch_bounds__(BLOCK) k_coarsen_size_codes(u32 ne,
+    u32 const* __restrict__ voe, double const* __restrict__ x, double const* __restrict__ h,
+    double size_floor, SegView sv, Fp32Stats* fs, u32* __restrict__ codes, u32* any)
 {
   pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  u32 c = 0;
-  bool decided = false, rechecked = false, flipped = false;
-  if (i < ne) {
-    u32 a = voe[i * 2], b = voe[i * 2 + 1];
+  u32 const i0 = blockIdx.x * CODE_TILE + threadIdx.x;
+  uint2 v[CODE_UNROLL];
+#pragma unroll
+  for (u32 k = 0; k < CODE_UNROLL; ++k) {
+    u32 const i = i0 + k * BLOCK;
+    v[k] = i < ne ? reinterpret_cast<uint2 const*>(voe)[i] : make_uint2(0u, 0u);
+  }
+  u32 some = 0, ndecided = 0, nrechecked = 0, naudited = 0, nflipped = 0;
+#pragma unroll
+  for (u32 k = 0; k < CODE_UNROLL; ++k) {
+    u32 const i = i0 + k * BLOCK;
+    if (i >= ne) continue;
+    u32 const a = v[k].x, b = v[k].y;
     double xa[3], xb[3];
     load3(x, a, xa);
     load3(x, b, xb);
-    int r32 = fs ? edge_ratio_side_f32(xa, xb, h[a], h[b], size_floor) : 0;
+    double const ha = h[a], hb = h[b];
+    int r32 = fs ? edge_ratio_side_f32(xa, xb, ha, hb, size_floor) : 0;
     bool shorter = false;
     if (r32) {
-      decided = true;
+      ++ndecided;
+      if (fs->audit) ++naudited;
       shorter = r32 < 0;
     }
     if (!r32 || fs->audit) {
-      rechecked = !r32;
+      nrechecked += !r32;
       double len = sqrt(sqdist3(xb, xa));
-      double want = (h[a] + h[b]) / 2;
+      double want = (ha + hb) / 2;
       bool s64 = (len / want) < size_floor;
-      flipped = r32 && s64 != shorter;
+      nflipped += r32 && s64 != shorter;
       shorter = s64;
     }
-    c = (shorter && seg_acts(sv, a)) ? (u32)COLLAPSE_BOTH : (u32)DONT_COLLAPSE;
+    u32 const c = (shorter && seg_acts(sv, a)) ? (u32)COLLAPSE_BOTH : (u32)DONT_COLLAPSE;
     codes[i] = c;
+    some |= c;
   }
-  if (fs) fp32_count_warp(fs, decided, rechecked, decided && fs->audit, flipped);
-  if (__any_sync(0xffffffffu, c) && (threadIdx.x & 31) == 0) atomicOr(any, 1u);
+  if (fs) fp32_count_block(fs, ndecided, nrechecked, naudited, nflipped);
+  if (__syncthreads_or((int)some) && threadIdx.x == 0) raise_flag(any);
 }
 
 // coarsen_sliver_code (coarsen.cpp:38-49)
@@ -57,7 +72,7 @@ __global__ void k_coarsen_sliver_codes(u32 ne, u32 const* __restrict__ voe,
     if (marked[voe[i * 2 + 1]]) c |= 2u;
     codes[i] = c;
   }
-  if (__any_sync(0xffffffffu, c) && (threadIdx.x & 31) == 0) atomicOr(any, 1u);
+  if (__any_sync(0xffffffffu, c) && (threadIdx.x & 31) == 0) raise_flag(any);
 }
 
 // check_basic_edge_class (check_collapse_class.cpp:12-37)
@@ -179,7 +194,9 @@ __device__ inline float warp_minf(float v)
   return v;
 }
 
-template <u32 DIM>
+// F32: with the single-precision filter (fs); without it, its estimates and
+// counters cost the double path no registers.
+template <u32 DIM, bool F32>
 __global__ void k_coarsen_quality(u32 const* __restrict__ list,
     u32 const* __restrict__ nlist, u32 const* __restrict__ voe1, u32 const* __restrict__ voe,
     u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev,
@@ -193,8 +210,11 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
   u32 n = *nlist;
   constexpr u32 vpe = deg(dim, 0);
   double const perfect = dim == 3 ? perfect_tet_quality() : perfect_tri_quality();
-  bool const use32 = fs && dim == 3;
+  constexpr bool use32 = F32 && dim == 3;
   float const k6 = tet_k6_f32();
+  // the filter's and the audit's counts of this warp, added once at the end
+  u32 ndecided = 0, nrechecked = 0, naudited = 0, nflipped = 0;
+  bool kept = false;
   for (u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n;
        w += (gridDim.x * blockDim.x) >> 5) {
     u32 i = list[w];
@@ -236,12 +256,10 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
         upper = warp_minf(upper);
         filtered = true;
         rejected32 = (double)upper < fq || (eq && (double)upper <= old_minq);
-        if (lane == 0) {
-          if (rejected32)
-            atomicAdd(&fs->decided, 1ull);
-          else
-            atomicAdd(&fs->rechecked, 1ull);
-        }
+        if (rejected32)
+          ++ndecided;
+        else
+          ++nrechecked;
       }
       double minq = 1.0;
       if (!rejected32) {
@@ -256,13 +274,13 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
           u32 base = opp(dim, 0, ev_dirs[k]);
           for (u32 l = 0; l + 1 < vpe; ++l) load3(x, ve[canon(dim, dim - 1, 0, base, l)], ex[l]);
           double q = dim == 3 ? tet_quality(ex, perfect) : tri_quality(ex, 1, perfect);
-          if (filtered && fs->audit) fp32_note_error(fs, tet_quality_f32(ex, k6), q);
+          if (use32 && filtered && fs->audit) fp32_note_error(fs, tet_quality_f32(ex, k6), q);
           first_min_add(mm, q, k - f + 1);
         }
         minq = warp_first_min(mm);
       }
       bool drop = rejected32 || minq < fq || (eq && minq <= old_minq);
-      if (filtered && fs->audit) {
+      if (use32 && filtered && fs->audit) {
         // the double path's result over the whole cavity, and every
         // estimate against its double value
         FirstMin m64{1.0, 0};
@@ -280,21 +298,24 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
         double q64 = warp_first_min(m64);
         bool drop64 = q64 < fq || (eq && q64 <= old_minq);
         bool flip = drop64 != drop || (!drop && q64 != minq);
-        if (lane == 0) {
-          atomicAdd(&fs->audited, 1ull);
-          if (flip) atomicAdd(&fs->flips, 1ull);
-        }
+        ++naudited;
+        if (flip) ++nflipped;
       }
       if (drop)
         code &= ~(1u << j);
       else if (lane == 0)
         out[i * 2 + j] = minq;
     }
-    if (lane == 0) {
-      codes[i] = code;
-      if (code != DONT_COLLAPSE) atomicOr(any, 1u);
-    }
+    if (lane == 0) codes[i] = code;
+    kept = kept || code != DONT_COLLAPSE;
   }
+  if (lane) return;
+  if (kept) raise_flag(any);
+  if (!use32) return;
+  if (ndecided) atomicAdd(&fs->decided, (unsigned long long)ndecided);
+  if (nrechecked) atomicAdd(&fs->rechecked, (unsigned long long)nrechecked);
+  if (naudited) atomicAdd(&fs->audited, (unsigned long long)naudited);
+  if (nflipped) atomicAdd(&fs->flips, (unsigned long long)nflipped);
 }
 
 // the candidate edges listed (a warp's candidates take consecutive slots,
@@ -785,7 +806,9 @@ static bool coarsen_select(Mesh& m, u32* codes, double qual_floor, bool require_
     // a warp per listed edge; the list's length is read on the device
     u32 const qb = tuned(TK_QUALITY_BLOCK);
     u32 blocks = (u32)std::min<u64>(ceil_div((u64)ne * 32, qb), 148u * 16u * 256u / qb);
-    CK(launch_kernel(dim == 3 ? k_coarsen_quality<3> : k_coarsen_quality<2>, dim3(blocks),
+    auto kq = dim == 2 ? k_coarsen_quality<2, false>
+            : m.fp32_filter ? k_coarsen_quality<3, true> : k_coarsen_quality<3, false>;
+    CK(launch_kernel(kq, dim3(blocks),
         dim3(qb), 0, s, clist, ncand, voe1, m.ask_down(dim, 0),
         ev.offs, ev.adj, ev.dirs, m.coords(), eq, qual_floor, m.segview(),
         m.fp32_filter ? fp32_stats_dev() : nullptr, codes, sel.q2, any));
@@ -1064,7 +1087,7 @@ u32 coarsen_by_size(Mesh& m, double qual_floor, double size_floor)
   // read-back
   u32* any = m.mb->dev + 5;
   if (ne) {
-    CK(launch_kernel(k_coarsen_size_codes, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, m.ask_down(1, 0), m.coords(),
+    CK(launch_kernel(k_coarsen_size_codes, dim3(grid_for(ne, CODE_TILE)), dim3(BLOCK), 0, s, ne, m.ask_down(1, 0), m.coords(),
         static_cast<double const*>(h->data), size_floor, m.segview(),
         m.fp32_filter ? fp32_stats_dev() : nullptr, codes, any));
     CK_LAUNCH();
@@ -1130,7 +1153,7 @@ u32 coarsen_sets(Mesh& m, double qual_floor, double size_floor, u32* codes_size,
   CK(cudaMemsetAsync(indset, 0, sizeof(u32) * nv, s));
   CK(cudaMemsetAsync(gen_vert, 0xff, sizeof(u32) * nv, s));
   if (ne) {
-    CK(launch_kernel(k_coarsen_size_codes, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, m.ask_down(1, 0), m.coords(),
+    CK(launch_kernel(k_coarsen_size_codes, dim3(grid_for(ne, CODE_TILE)), dim3(BLOCK), 0, s, ne, m.ask_down(1, 0), m.coords(),
         static_cast<double const*>(h->data), size_floor, m.segview(),
         m.fp32_filter ? fp32_stats_dev() : nullptr, codes_size, any));
     CK_LAUNCH();

@@ -461,6 +461,99 @@ __device__ inline void fp32_count_warp(Fp32Stats* st, bool decided, bool recheck
   }
 }
 
+// The same for a thread's counts of the flags, summed over the block: one
+// update of a counter per block (a million edges in warps of their own
+// updated the same two words 62,500 times, which took longer than the
+// edges' lengths). Every thread of the block must call it, once.
+__device__ inline void fp32_count_block(Fp32Stats* st, u32 decided, u32 rechecked,
+    u32 audited, u32 flipped)
+{
+  __shared__ u32 s_n[4];
+  if (threadIdx.x < 4) s_n[threadIdx.x] = 0;
+  __syncthreads();
+  u32 const n[4] = {__reduce_add_sync(0xffffffffu, decided),
+      __reduce_add_sync(0xffffffffu, rechecked), __reduce_add_sync(0xffffffffu, audited),
+      __reduce_add_sync(0xffffffffu, flipped)};
+  if ((threadIdx.x & 31) == 0)
+    for (u32 k = 0; k < 4; ++k)
+      if (n[k]) atomicAdd(&s_n[k], n[k]);
+  __syncthreads();
+  unsigned long long* const to[4] = {&st->decided, &st->rechecked, &st->audited, &st->flips};
+  if (threadIdx.x < 4 && s_n[threadIdx.x])
+    atomicAdd(to[threadIdx.x], (unsigned long long)s_n[threadIdx.x]);
+}
+
+// The marked items of a block's tile appended to a list of *count items, in
+// order within the tile, with one update of the count per block: item k of
+// a thread (k < K, bit k of `on`) is first + k * BLOCK, first being the
+// tile's base + threadIdx.x. Every thread of a block of BLOCK threads must
+// call it, once; returns the number the block appended.
+template <u32 K>
+__device__ inline u32 block_append(u32 on, u32 first, u32* __restrict__ list, u32* count)
+{
+  constexpr u32 WARPS = 8, N = K * WARPS;  // (warp, k) runs of 32 consecutive items
+  static_assert(N <= 32, "one warp scans the runs");
+  __shared__ u32 s_at[N];
+  __shared__ u32 s_total;
+  u32 const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  u32 mask[K];
+#pragma unroll
+  for (u32 k = 0; k < K; ++k) {
+    mask[k] = __ballot_sync(0xffffffffu, (on >> k) & 1u);
+    if (lane == 0) s_at[k * WARPS + warp] = __popc(mask[k]);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    u32 const c = lane < N ? s_at[lane] : 0u;
+    u32 x = c;
+#pragma unroll
+    for (u32 o = 1; o < 32; o <<= 1) {
+      u32 y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    u32 const total = __shfl_sync(0xffffffffu, x, 31);
+    u32 base = 0;
+    if (lane == 0 && total) base = atomicAdd(count, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (lane < N) s_at[lane] = base + x - c;
+    if (lane == 0) s_total = total;
+  }
+  __syncthreads();
+#pragma unroll
+  for (u32 k = 0; k < K; ++k)
+    if ((on >> k) & 1u)
+      list[s_at[k * WARPS + warp] + __popc(mask[k] & ((1u << lane) - 1u))] = first + k * 256u;
+  return s_total;
+}
+
+// sets a flag that several threads may set, without an atomic update once
+// it is set
+__device__ inline void raise_flag(u32* flag)
+{
+  if (*(u32 volatile*)flag == 0) *(u32 volatile*)flag = 1u;
+}
+
+// the least key of a block into *minkey: one update per block, none when it
+// would not change it. Every thread of a block of at most 1024 must call it.
+__device__ inline void block_min_key(unsigned long long key, unsigned long long* minkey)
+{
+  __shared__ unsigned long long s_min[32];
+  u32 const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+  for (int o = 16; o; o >>= 1) {
+    unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
+    key = other < key ? other : key;
+  }
+  if (lane == 0) s_min[warp] = key;
+  __syncthreads();
+  if (warp) return;
+  key = lane < nwarps ? s_min[lane] : ~0ull;
+  for (int o = 16; o; o >>= 1) {
+    unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
+    key = other < key ? other : key;
+  }
+  if (lane == 0 && key < *(unsigned long long volatile*)minkey) atomicMin(minkey, key);
+}
+
 // tet_quality (quality.hpp:68-89): Shewchuk's V / A_rms^(3/2), normalised
 __host__ __device__ inline double tet_quality(double const (*x)[3], double perfect)
 {
@@ -508,6 +601,24 @@ __device__ inline void load3(double const* __restrict__ c, u32 v, double* o)
   o[0] = c[v * 3 + 0];
   o[1] = c[v * 3 + 1];
   o[2] = c[v * 3 + 2];
+}
+
+// the corners of element i (a tet's vertices in one 16-byte load: entity
+// arrays start on a pool allocation)
+template <u32 DIM>
+__device__ inline void load_corners(u32 const* __restrict__ voe, double const* __restrict__ x,
+    u32 i, double (*ex)[3])
+{
+  u32 v[4] = {0, 0, 0, 0};
+  if (DIM == 3) {
+    uint4 const t = reinterpret_cast<uint4 const*>(voe)[i];
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+  } else {
+#pragma unroll
+    for (u32 j = 0; j <= DIM; ++j) v[j] = voe[(size_t)i * (DIM + 1) + j];
+  }
+#pragma unroll
+  for (u32 j = 0; j <= DIM; ++j) load3(x, v[j], ex[j]);
 }
 
 // ---------------------------------------------------------------------------

@@ -221,24 +221,19 @@ __global__ void k_axpy(u32 n, double a, double const* __restrict__ x,
   if (i < n) out[i] = a * x[i] + y[i];
 }
 
-__global__ void k_min_quality(u32 dim, u32 ne, u32 const* __restrict__ voe,
+template <u32 DIM>
+__global__ void k_min_quality(u32 ne, u32 const* __restrict__ voe,
     double const* __restrict__ x, unsigned long long* minkey)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long key = ~0ull;
   if (i < ne) {
-    u32 vpe = dim + 1;
     double ex[4][3];
-    for (u32 j = 0; j < vpe; ++j) load3(x, voe[(size_t)i * vpe + j], ex[j]);
-    double q = elem_quality(dim, ex, 1);
-    key = order_key(q);
+    load_corners<DIM>(voe, x, i, ex);
+    key = order_key(elem_quality(DIM, ex, 1));
   }
-  for (int o = 16; o; o >>= 1) {
-    unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
-    key = other < key ? other : key;
-  }
-  if ((threadIdx.x & 31) == 0 && key != ~0ull) atomicMin(minkey, key);
+  block_min_key(key, minkey);
 }
 
 }  // namespace
@@ -322,7 +317,8 @@ static double min_quality_of(Mesh& m, double const* x)
   unsigned long long* mk = reinterpret_cast<unsigned long long*>(m.mb->dev + 30);
   CK(cudaMemsetAsync(mk, 0xff, sizeof(unsigned long long), s));
   if (ne) {
-    CK(launch_kernel(k_min_quality, dim3(grid_for(ne)), dim3(BLOCK), 0, s, m.dim, ne, m.ask_down(m.dim, 0), x, mk));
+    auto k = m.dim == 3 ? k_min_quality<3> : m.dim == 2 ? k_min_quality<2> : k_min_quality<1>;
+    CK(launch_kernel(k, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, m.ask_down(m.dim, 0), x, mk));
     CK_LAUNCH();
   }
   m.mb->fetch(s, 32);

@@ -1941,27 +1941,24 @@ u32 const* Mesh::ask_dual()
 // geometry: qualities, sizes, edge lengths (quality.cpp, size.cpp)
 
 
-__global__ void k_elem_quality(u32 dim, u32 ne, u32 const* __restrict__ voe,
-    double const* __restrict__ x, double* __restrict__ q,
-    unsigned long long* minkey)
+// (DIM at compile time: the corners stay in registers; the minimum takes
+// one update per block, where a warp's of its own queued every warp on one
+// word)
+template <u32 DIM>
+__global__ void k_elem_quality(u32 ne, u32 const* __restrict__ voe,
+    double const* __restrict__ x, double* __restrict__ q, unsigned long long* minkey)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   double qi = DBL_MAX;
   if (i < ne) {
-    u32 vpe = deg(dim, 0);
     double ex[4][3];
-    for (u32 j = 0; j < vpe; ++j) load3(x, voe[(size_t)i * vpe + j], ex[j]);
-    qi = dim >= 2 ? elem_quality(dim, ex, 1) : 1.0;
+    load_corners<DIM>(voe, x, i, ex);
+    qi = DIM >= 2 ? elem_quality(DIM, ex, 1) : 1.0;
     q[i] = qi;
   }
   // min over elements below DBL_MAX, as doubles_min's `a[i] < min` keeps
-  unsigned long long key = (qi < DBL_MAX) ? order_key(qi) : ~0ull;
-  for (int o = 16; o; o >>= 1) {
-    unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
-    key = other < key ? other : key;
-  }
-  if ((threadIdx.x & 31) == 0 && key != ~0ull) atomicMin(minkey, key);
+  block_min_key((qi < DBL_MAX) ? order_key(qi) : ~0ull, minkey);
 }
 
 // The cache holds ne qualities followed by one 8-byte slot with the
@@ -1976,8 +1973,9 @@ double const* Mesh::qualities()
   if (ne) {
     PROBE(P_ELEM_QUALITY, s, 4.0 * deg(dim, 0) * ne + 24.0 * counts[0] + 8.0 * ne);
     u32 const qb = tuned(TK_QUALITY_BLOCK);
-    CK(launch_kernel(k_elem_quality, dim3(grid_for(ne, qb)), dim3(qb), 0, s, dim, ne,
-        ask_down(dim, 0), coords(), qual_cache, mk));
+    auto k = dim == 3 ? k_elem_quality<3> : dim == 2 ? k_elem_quality<2> : k_elem_quality<1>;
+    CK(launch_kernel(k, dim3(grid_for(ne, qb)), dim3(qb), 0, s, ne, ask_down(dim, 0), coords(),
+        qual_cache, mk));
     CK_LAUNCH();
   }
   return qual_cache;
@@ -1994,19 +1992,19 @@ double Mesh::min_quality()
   return from_order_key(k);
 }
 
-__global__ void k_elem_size(u32 dim, u32 ne, u32 const* __restrict__ voe,
+template <u32 DIM>
+__global__ void k_elem_size(u32 ne, u32 const* __restrict__ voe,
     double const* __restrict__ x, double* __restrict__ out)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ne) return;
-  u32 vpe = deg(dim, 0);
   double ex[4][3];
-  for (u32 j = 0; j < vpe; ++j) load3(x, voe[(size_t)i * vpe + j], ex[j]);
+  load_corners<DIM>(voe, x, i, ex);
   double v;
-  if (dim == 3)
+  if (DIM == 3)
     v = tet_volume(ex);
-  else if (dim == 2)
+  else if (DIM == 2)
     v = tri_area(ex[0], ex[1], ex[2]);
   else
     v = sqrt(sqdist3(ex[1], ex[0]));
@@ -2018,7 +2016,9 @@ double* Mesh::element_sizes()
   u32 ne = count(dim);
   double* out = dalloc<double>(ne, s);
   if (ne) {
-    CK(launch_kernel(k_elem_size, dim3(grid_for(ne)), dim3(BLOCK), 0, s, dim, ne, ask_down(dim, 0), coords(), out));
+    auto k = dim == 3 ? k_elem_size<3> : dim == 2 ? k_elem_size<2> : k_elem_size<1>;
+    CK(launch_kernel(k, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, ask_down(dim, 0), coords(),
+        out));
     CK_LAUNCH();
   }
   return out;
