@@ -447,6 +447,17 @@ __device__ inline void expand_same_rows(ExpandJob const& jb, u32 warp, u32 nwarp
     for (u32 ch = 0; ch < EXPAND_CHUNKS; ++ch) {
       u32 const cb = base + ch * 32;
       u32 const nw = (cb < jb.n ? min(32u, jb.n - cb) : 0u) * W;
+      // 32 rows that all survive (most runs of a pass that changes little)
+      // are one run of the output: no row to find for a word
+      if (__all_sync(0xffffffffu, o1[ch] == o0[ch] + 1)) {
+        size_t const at = (size_t)__shfl_sync(0xffffffffu, o0[ch], 0) * W + lane;
+#pragma unroll
+        for (u32 it = 0; it < W; ++it) {
+          out[at + it * 32] = a[ch][it];
+          if (two) out2[at + it * 32] = b[ch][it];
+        }
+        continue;
+      }
 #pragma unroll
       for (u32 it = 0; it < W; ++it) {
         u32 const q = it * 32 + lane;
