@@ -709,27 +709,20 @@ double wall_s()
   return duration<double>(steady_clock::now().time_since_epoch()).count();
 }
 
-// consecutive runs of `idx` whose current elements sum to at most `max`
-// (0 = no limit); each run holds at least one mesh
-std::vector<std::vector<u32>> chunks_of(std::vector<Mesh*>& ms, std::vector<u32> const& idx,
-    unsigned long long max)
-{
-  std::vector<std::vector<u32>> out;
-  std::vector<u32> cur;
-  unsigned long long sum = 0;
-  for (u32 k : idx) {
-    unsigned long long ne = ms[k]->count(ms[k]->dim);
-    if (!cur.empty() && max && sum + ne > max) {
-      out.push_back(cur);
-      cur.clear();
-      sum = 0;
-    }
-    cur.push_back(k);
-    sum += ne;
-  }
-  if (!cur.empty()) out.push_back(cur);
-  return out;
-}
+// unions past this many elements are not kept between passes (their passes
+// are bound by their bytes, and their use counts must stay below 2^32)
+constexpr u64 KEEP_UNION_ELEMS = 1u << 26;
+// A union is regathered when over 7/8 of its elements, and over a million,
+// wait. A pass over a million waiting elements costs about 0.25 ms (they are
+// renumbered with the rest); splitting, gathering anew and deriving the
+// adjacency that was carried cost 1 to 2 ms for meshes of a few thousand
+// tets. (48 boxes of n = 4..12: 30 ms splitting at one half, 26 at a
+// quarter, 23 at an eighth, 22 never; 37 split after every pass.)
+constexpr u64 IDLE_ELEMS = 1000000;
+
+// the point of mesh_adapt's loop a pass acts on: refine (the quality floor
+// is read before the first), coarsen, shape
+u32 phase_of(u32 state) { return state == ST_INIT ? (u32)ST_REFINE : state; }
 
 }  // namespace
 
@@ -737,17 +730,14 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
     std::vector<char>& owned)
 {
   BatchStats& bs = last_batch_stats();
-  u32 n = (u32)ms.size();
-  bool live = false;
-  for (u32 k = 0; k < n; ++k) live = live || st[k].state < ST_DONE;
-  if (!live) return false;
-  bs.steps += 1;
-  auto group = [&](u32 state) {
-    std::vector<u32> g;
+  u32 const n = (u32)ms.size();
+  auto any_live = [&] {
     for (u32 k = 0; k < n; ++k)
-      if (st[k].state == state) g.push_back(k);
-    return g;
+      if (st[k].state < ST_DONE) return true;
+    return false;
   };
+  if (!any_live()) return false;
+  bs.steps += 1;
   // incr_op_count (adapt.cpp:36-45) for mesh k after a pass that changed it
   auto counted = [&](u32 k, u32 op, u32 elems) {
     BatchMeshResult& r = st[k].res;
@@ -764,167 +754,238 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
     }
     ++st[k].ops;
   };
-  auto replace = [&](u32 k, Mesh* m) {
-    if (owned[k]) delete ms[k];
-    ms[k] = m;
-    owned[k] = 1;
-  };
-  // a union of the meshes c; a lone mesh is its own union of one segment,
-  // changed in place by the pass with nothing to copy in or out
-  auto gather = [&](std::vector<u32> const& c) {
-    if (c.size() == 1) {
-      Mesh* m = ms[c[0]];
-      if (!m->seg) {
-        u32 nv = m->count(0);
-        m->seg = dalloc<u32>(nv ? nv : 1, m->s);
-        CK(cudaMemsetAsync(m->seg, 0, sizeof(u32) * (nv ? nv : 1), m->s));
-        m->nseg = 1;
+  // the kept unions and their meshes, in mesh order
+  std::vector<std::shared_ptr<Resident>> rs;
+  std::vector<std::vector<u32>> members;
+  auto list_residents = [&] {
+    rs.clear();
+    members.clear();
+    for (u32 k = 0; k < n; ++k) {
+      if (!st[k].in) continue;
+      size_t q = 0;
+      while (q < rs.size() && rs[q] != st[k].in) ++q;
+      if (q == rs.size()) {
+        rs.push_back(st[k].in);
+        members.emplace_back();
       }
-      return m;
+      members[q].push_back(k);
     }
-    std::vector<Mesh*> parts;
-    for (u32 k : c) parts.push_back(ms[k]);
-    bs.unions += 1;
-    double t = wall_s();
-    Mesh* u = concat_meshes(parts, s);
-    stream_sync(s);
-    bs.secs_concat += wall_s() - t;
-    return u;
   };
-  auto release = [&](Mesh* u, std::vector<u32> const& c) {
-    if (c.size() != 1) delete u;
+  // the point a union's next pass acts on: the earliest of its live meshes'
+  auto phase_of_members = [&](std::vector<u32> const& mk) {
+    u32 p = ST_DONE;
+    for (u32 k : mk) p = std::min(p, phase_of(st[k].state));
+    return p;
   };
-  auto split = [&](Mesh& u, std::vector<char> const& want) {
+  // meshes out of the union that holds them
+  auto take_out = [&](Resident& r, std::vector<u32> const& mk) {
     double t = wall_s();
-    std::vector<Mesh*> o = split_union(u, s, &want);
+    std::vector<char> want(r.u->nseg, 0);
+    bool any = false;
+    for (u32 k : mk)
+      if (r.dirty[st[k].seg]) want[st[k].seg] = any = true;
+    std::vector<Mesh*> o;
+    if (any) o = split_union(*r.u, s, &want);
+    std::shared_ptr<Resident> hold = st[mk[0]].in;
+    for (u32 k : mk) {
+      if (want[st[k].seg]) {
+        if (owned[k]) delete ms[k];
+        ms[k] = o[st[k].seg];
+        owned[k] = 1;
+      }
+      st[k].in.reset();
+    }
     bs.secs_split += wall_s() - t;
-    return o;
   };
-  // satisfy_size's floor (adapt.cpp:47-52), once per mesh
-  for (auto const& c : chunks_of(ms, group(ST_INIT), max_union_elems)) {
-    Mesh* u = gather(c);
-    std::vector<double> mq;
-    try {
-      UnionCtl ctl(*u);
-      mq = ctl.min_quality();
-    } catch (...) {
-      release(u, c);
-      throw;
-    }
-    release(u, c);
-    for (u32 j = 0; j < c.size(); ++j) {
-      SegState& x = st[c[j]];
-      x.qf = mq[j];
-      if (ap.good_qual < x.qf) x.qf = ap.good_qual;
-      x.state = ST_REFINE;
-    }
+  // unions that are done, too large to keep, or mostly waiting: split
+  list_residents();
+  for (size_t q = 0; q < rs.size(); ++q) {
+    Resident& r = *rs[q];
+    u32 const p = phase_of_members(members[q]);
+    u64 const total = r.u->count(r.u->dim);
+    u64 counted_elems = 0, acting = 0;
+    for (u32 e : r.elems) counted_elems += e;
+    for (u32 k : members[q])
+      if (phase_of(st[k].state) == p) acting += r.elems[st[k].seg];
+    if (p >= ST_DONE || total > KEEP_UNION_ELEMS ||
+        (max_union_elems && total > max_union_elems && members[q].size() > 1) ||
+        (8 * acting < counted_elems && counted_elems - acting > IDLE_ELEMS))
+      take_out(r, members[q]);
   }
-  // satisfy_size: refine while it changes a mesh, then coarsen
-  for (u32 op : {OP_REFINE, OP_COARSEN}) {
-    u32 here = op == OP_REFINE ? ST_REFINE : ST_COARSEN;
-    u32 next = op == OP_REFINE ? ST_COARSEN : ST_SHAPE;
-    for (auto const& c : chunks_of(ms, group(here), max_union_elems)) {
-      Mesh* u = gather(c);
-      u32 m = (u32)c.size();
-      std::vector<u32> sel(m), elems(m), all(m);
-      std::vector<double> qf(m);
-      for (u32 j = 0; j < m; ++j) {
-        all[j] = j;
-        qf[j] = st[c[j]].qf;
+  // Meshes held apart are gathered by the point they are at, with the kept
+  // unions at that point (a union of unions): consecutive items of at most
+  // max_union_elems elements. Kept unions alone stay as they are.
+  list_residents();
+  std::vector<std::pair<u32, u32>> alone;  // (phase, mesh): gathered with nothing
+  for (u32 p : {ST_REFINE, ST_COARSEN, ST_SHAPE}) {
+    struct Item {
+      Mesh* m;
+      int r;  // a kept union's index, or -1: mesh k
+      u32 k;
+      u64 elems;
+    };
+    std::vector<Item> items;
+    bool apart = false;
+    for (u32 k = 0; k < n; ++k)
+      if (!st[k].in && st[k].state < ST_DONE && phase_of(st[k].state) == p) {
+        items.push_back({ms[k], -1, k, ms[k]->count(ms[k]->dim)});
+        apart = true;
       }
-      std::vector<Mesh*> outs;
-      try {
-        {
-          double t = wall_s();
-          UnionCtl ctl(*u);
-          ctl.run(op, all, qf, ap.size_floor, ap.good_qual, ap.nlayers);
-          bs.secs_passes += wall_s() - t;
-          for (u32 j = 0; j < m; ++j) {
-            sel[j] = ctl.h_u32[j];
-            elems[j] = ctl.h_u32[m + j];
-          }
-        }
-        if (m > 1) {
-          std::vector<char> want(m);
-          for (u32 j = 0; j < m; ++j) want[j] = sel[j] ? 1 : 0;
-          outs = split(*u, want);
-        }
-      } catch (...) {
-        release(u, c);
-        throw;
+    if (!apart) continue;
+    for (size_t q = 0; q < rs.size(); ++q)
+      if (phase_of_members(members[q]) == p)
+        items.push_back({rs[q]->u, (int)q, 0, rs[q]->u->count(rs[q]->u->dim)});
+    for (size_t at = 0; at < items.size();) {
+      size_t end = at;
+      u64 sum = 0;
+      bool some = false;
+      while (end < items.size() &&
+             (end == at || !max_union_elems || sum + items[end].elems <= max_union_elems) &&
+             (end == at || sum + items[end].elems <= KEEP_UNION_ELEMS)) {
+        sum += items[end].elems;
+        some = some || items[end].r < 0;
+        ++end;
       }
-      release(u, c);
-      for (u32 j = 0; j < m; ++j) {
-        u32 k = c[j];
-        if (sel[j]) {
-          counted(k, op, elems[j]);
-          if (m > 1) replace(k, outs[j]);
-        } else {
-          st[k].state = next;
-        }
+      if (end - at == 1 || !some) {
+        for (size_t i = at; i < end; ++i)
+          if (items[i].r < 0) alone.push_back({p, items[i].k});
+        at = end;
+        continue;
       }
-    }
-  }
-  // satisfy_shape (adapt.cpp:58-80): swap, else collapse slivers
-  for (auto const& c : chunks_of(ms, group(ST_SHAPE), max_union_elems)) {
-    Mesh* u = gather(c);
-    u32 m = (u32)c.size();
-    std::vector<char> changed(m, 0);
-    std::vector<Mesh*> outs;
-    try {
       double t = wall_s();
-      UnionCtl ctl(*u);
-      std::vector<double> mq = ctl.min_quality(), qf(m, 0.0);
-      std::vector<u32> g2, g3;
-      for (u32 j = 0; j < m; ++j)
-        if (mq[j] >= ap.good_qual)
-          st[c[j]].state = ST_DONE;
+      std::vector<Mesh*> parts;
+      for (size_t i = at; i < end; ++i) parts.push_back(items[i].m);
+      auto r = std::make_shared<Resident>();
+      r->u = concat_meshes(parts, s);
+      stream_sync(s);
+      bs.unions += 1;
+      r->dirty.assign(r->u->nseg, 0);
+      r->elems.assign(r->u->nseg, 0);
+      u32 seg = 0;
+      for (size_t i = at; i < end; ++i) {
+        if (items[i].r < 0) {
+          u32 const k = items[i].k;
+          r->elems[seg] = (u32)items[i].elems;
+          if (owned[k]) {  // the union holds it now
+            r->dirty[seg] = 1;
+            delete ms[k];
+            ms[k] = nullptr;
+            owned[k] = 0;
+          }
+          st[k].in = r;
+          st[k].seg = seg++;
+          continue;
+        }
+        Resident& o = *rs[items[i].r];
+        for (size_t j = 0; j < o.elems.size(); ++j) {
+          r->elems[seg + j] = o.elems[j];
+          r->dirty[seg + j] = o.dirty[j];
+        }
+        for (u32 k : members[items[i].r]) {
+          st[k].in = r;
+          st[k].seg += seg;
+        }
+        seg += o.u->nseg;
+      }
+      r->ctl.reset(new UnionCtl(*r->u));
+      bs.secs_concat += wall_s() - t;
+      at = end;
+    }
+  }
+  // one pass (a shape step: a swap, then collapses of slivers) over a union
+  // whose segment j is mesh mk[j] of segs[j]
+  auto pass = [&](UnionCtl& ctl, u32 p, std::vector<u32> const& mk, std::vector<u32> const& segs,
+                  Resident* r) {
+    double t = wall_s();
+    u32 const m = ctl.nm;
+    std::vector<double> qf(m, 0.0);
+    auto ran = [&](u32 j, u32 op) {  // whether the pass changed member j
+      u32 const sg = segs[j];
+      if (r) r->elems[sg] = ctl.h_u32[m + sg];
+      if (!ctl.h_u32[sg]) return false;
+      counted(mk[j], op, ctl.h_u32[m + sg]);
+      if (r) r->dirty[sg] = 1;
+      return true;
+    };
+    if (p == ST_SHAPE) {
+      // satisfy_shape (adapt.cpp:58-80): swap, else collapse slivers
+      std::vector<double> mq = ctl.min_quality();
+      std::vector<u32> g2, g3, gs;
+      for (u32 j = 0; j < mk.size(); ++j) {
+        if (phase_of(st[mk[j]].state) != p) continue;
+        if (mq[segs[j]] >= ap.good_qual)
+          st[mk[j]].state = ST_DONE;
         else
           g2.push_back(j);
-      if (u->dim == 3 && !g2.empty()) {
-        ctl.run(OP_SWAP, g2, qf, ap.size_floor, ap.good_qual, ap.nlayers);
+      }
+      if (ctl.u.dim == 3 && !g2.empty()) {
+        for (u32 j : g2) gs.push_back(segs[j]);
+        ctl.run(OP_SWAP, gs, qf, ap.size_floor, ap.good_qual, ap.nlayers);
         for (u32 j : g2)
-          if (ctl.h_u32[j]) {
-            counted(c[j], OP_SWAP, ctl.h_u32[m + j]);
-            changed[j] = 1;
-          } else {
-            g3.push_back(j);
-          }
+          if (!ran(j, OP_SWAP)) g3.push_back(j);
       } else {
         g3 = g2;
       }
       if (!g3.empty()) {
-        ctl.run(OP_CSLIVERS, g3, qf, ap.size_floor, ap.good_qual, ap.nlayers);
+        gs.clear();
+        for (u32 j : g3) gs.push_back(segs[j]);
+        ctl.run(OP_CSLIVERS, gs, qf, ap.size_floor, ap.good_qual, ap.nlayers);
         for (u32 j : g3)
-          if (ctl.h_u32[j]) {
-            counted(c[j], OP_CSLIVERS, ctl.h_u32[m + j]);
-            changed[j] = 1;
-          } else {
-            st[c[j]].state = ST_DONE;  // shape quality could not be satisfied
-          }
+          if (!ran(j, OP_CSLIVERS)) st[mk[j]].state = ST_DONE;  // could not be satisfied
       }
       bs.secs_passes += wall_s() - t;
-    } catch (...) {
-      release(u, c);
-      throw;
+      return;
     }
-    bool any = false;
-    for (char x : changed) any = any || x;
-    if (any && m > 1) {
-      try {
-        outs = split(*u, changed);
-      } catch (...) {
-        release(u, c);
-        throw;
+    // satisfy_size's floor (adapt.cpp:47-52), once per mesh
+    bool first = false;
+    for (u32 k : mk) first = first || st[k].state == ST_INIT;
+    if (first) {
+      std::vector<double> mq = ctl.min_quality();
+      for (u32 j = 0; j < mk.size(); ++j) {
+        SegState& x = st[mk[j]];
+        if (x.state != ST_INIT) continue;
+        x.qf = std::min(mq[segs[j]], ap.good_qual);
+        x.state = ST_REFINE;
       }
-      for (u32 j = 0; j < m; ++j)
-        if (changed[j]) replace(c[j], outs[j]);
     }
-    release(u, c);
+    // satisfy_size: refine while it changes a mesh, then coarsen
+    u32 const op = p == ST_REFINE ? OP_REFINE : OP_COARSEN;
+    std::vector<u32> g, gs;
+    for (u32 j = 0; j < mk.size(); ++j) {
+      if (st[mk[j]].state != p) continue;
+      g.push_back(j);
+      gs.push_back(segs[j]);
+      qf[segs[j]] = st[mk[j]].qf;
+    }
+    ctl.run(op, gs, qf, ap.size_floor, ap.good_qual, ap.nlayers);
+    for (u32 j : g)
+      if (!ran(j, op)) st[mk[j]].state = p == ST_REFINE ? ST_COARSEN : ST_SHAPE;
+    bs.secs_passes += wall_s() - t;
+  };
+  // a lone mesh is its own union of one segment, changed in place by the
+  // pass with nothing to copy in or out
+  for (auto const& a : alone) {
+    Mesh* m = ms[a.second];
+    if (!m->seg) {
+      u32 nv = m->count(0);
+      m->seg = dalloc<u32>(nv ? nv : 1, m->s);
+      CK(cudaMemsetAsync(m->seg, 0, sizeof(u32) * (nv ? nv : 1), m->s));
+      m->nseg = 1;
+    }
+    UnionCtl ctl(*m);
+    pass(ctl, a.first, {a.second}, {0u}, nullptr);
   }
-  live = false;
-  for (u32 k = 0; k < n; ++k) live = live || st[k].state < ST_DONE;
-  return live;
+  list_residents();
+  for (size_t q = 0; q < rs.size(); ++q) {
+    std::vector<u32> segs, done;
+    for (u32 k : members[q]) segs.push_back(st[k].seg);
+    pass(*rs[q]->ctl, phase_of_members(members[q]), members[q], segs, rs[q].get());
+    for (u32 k : members[q])
+      if (st[k].state >= ST_DONE) done.push_back(k);
+    if (!done.empty() && (hand_back || done.size() == members[q].size()))
+      take_out(*rs[q], done);
+  }
+  return any_live();
 }
 
 // ---------------------------------------------------------------------------
@@ -1145,6 +1206,7 @@ void adapt_batch(std::vector<Mesh*> const& ms, double size_floor, double good_qu
   auto cleanup = [&]() {
     for (u32 k = 0; k < n; ++k)
       if (owned[k]) delete cur[k];
+    st.clear();  // and with it any union still kept
     release_stream_scratch(run.s);
     cudaStreamSynchronize(run.s);
     cudaStreamDestroy(run.s);

@@ -8,6 +8,7 @@
 // so each mesh comes out exactly as mesh_adapt would leave it.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "passes.hpp"
@@ -67,11 +68,17 @@ struct AdaptParams {
   u32 max_ops;
 };
 
+struct Resident;
+
 struct SegState {
   u32 state = ST_INIT;
   u32 ops = 0;
   double qf = 0;          // satisfy_size's quality floor
   BatchMeshResult res;
+  // the union this mesh is held in between passes, and its segment there
+  // (none: the mesh is held apart)
+  std::shared_ptr<Resident> in;
+  u32 seg = 0;
 };
 
 // per-segment control arrays of a union and the host copies of their results
@@ -99,18 +106,41 @@ struct UnionCtl {
       double size_floor, double good_qual, u32 nlayers);
 };
 
-// Runs mesh_adapt's loop for many meshes held apart between passes: every
-// step gathers the meshes that are at the same point of their loop into
-// unions of at most max_union_elems current elements (0 = no limit), runs
-// that pass over each union (one launch per stage), and splits out the
-// meshes it changed. A union thus only holds meshes its pass acts on.
+// A union kept between passes with the adjacency its passes carry. A
+// segment is dirty once a pass changed it (or when the mesh it was made from
+// is gone): it has to be split out to be read.
+struct Resident {
+  Mesh* u = nullptr;
+  std::unique_ptr<UnionCtl> ctl;
+  std::vector<char> dirty;
+  std::vector<u32> elems;  // each segment's elements when last counted
+  Resident() = default;
+  Resident(Resident const&) = delete;
+  Resident& operator=(Resident const&) = delete;
+  ~Resident()
+  {
+    ctl.reset();
+    delete u;
+  }
+};
+
+// Runs mesh_adapt's loop for many meshes: every step gathers the meshes that
+// are at the same point of their loop into unions of at most max_union_elems
+// current elements (0 = no limit) and runs that pass over each union, one
+// launch per stage. A union is kept between passes, with the adjacency they
+// carry; its meshes that got further wait for the others. Once most of its
+// elements wait (IDLE_ELEMS) its meshes are split out and gathered anew.
 struct GroupRunner {
   AdaptParams ap{1.0 / 3.0, 0.3, 4, 50};
   unsigned long long max_union_elems = 0;
   cudaStream_t s = nullptr;  // unions and the meshes split out of them
+  // split a mesh out at the end of the step its loop ends in (a server's
+  // jobs leave then); otherwise when the last mesh of its union is done
+  bool hand_back = false;
   // one step for every live mesh; ms[k] is replaced (and owned[k] set) when
-  // a pass changes it, the previous ms[k] deleted if it was owned. Returns
-  // whether any mesh is still live.
+  // it is split out of a union, the previous ms[k] deleted if it was owned
+  // (null, not owned, while st[k].in holds the mesh). Returns whether any
+  // mesh is still live; every mesh is held apart again when none is.
   bool step(std::vector<Mesh*>& ms, std::vector<SegState>& st, std::vector<char>& owned);
 };
 

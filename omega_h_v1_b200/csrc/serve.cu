@@ -111,6 +111,7 @@ struct Server {
     stop();
     for (size_t k = 0; k < ms.size(); ++k)
       if (owned[k]) delete ms[k];
+    st.clear();  // and with it any union still kept
     jobs.clear();
     if (run.s) {
       release_stream_scratch(run.s);
@@ -285,6 +286,7 @@ Server* server_new(AdaptParams const& ap, unsigned long long budget)
   // unions of a few million elements: enough work per launch, and a working
   // set that keeps most gathers in L2
   sv->run.max_union_elems = 4000000ull;
+  sv->run.hand_back = true;
   sv->budget = budget;
   sv->t0 = now_s();
   CK(cudaStreamCreateWithFlags(&sv->run.s, cudaStreamNonBlocking));
