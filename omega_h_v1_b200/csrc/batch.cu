@@ -86,54 +86,94 @@ __global__ void k_ent_seg(u32 n, u32 const* __restrict__ voe, u32 vpe,
 }
 
 // per tile of SPLIT_TILE entities (one warp), the count of each segment,
-// stored segment-major: hist[seg * ntiles + tile]
+// stored segment-major: hist[seg * ntiles + tile]. A union's entities come
+// in runs of one segment (each pass keeps the survivors' order and appends
+// its products by domain), so a warp mostly meets the segment it met last:
+// that segment's count stays in a register and reaches memory when another
+// segment comes. (Every step's count read and written in memory was a chain
+// of 64 round trips: 48 us a launch at any size.) TILE_AHEAD steps'
+// segments are loaded together.
+constexpr u32 TILE_AHEAD = 8;
+
 __global__ void k_tile_hist(u32 n, u32 const* __restrict__ es, u32 ntiles, u32* __restrict__ hist)
 {
   pdl_wait();
   u32 tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (tile >= ntiles) return;
-  u32 base = tile * SPLIT_TILE;
-  for (u32 c = 0; c < SPLIT_TILE; c += 32) {
-    u32 i = base + c + lane;
-    bool on = i < n;
-    u32 mask = __ballot_sync(FULL_MASK, on);
-    if (!mask) break;
-    if (on) {
-      u32 sg = es[i];
-      u32 peers = __match_any_sync(mask, sg);
-      if (lane == (u32)(__ffs(peers) - 1)) hist[(size_t)sg * ntiles + tile] += __popc(peers);
+  u32 const base = tile * SPLIT_TILE, end = min(n, base + SPLIT_TILE);
+  u32 cur = INV, cnt = 0;  // the segment in hand (the same in every lane) and its count
+  for (u32 c = base; c < end; c += 32 * TILE_AHEAD) {
+    u32 sgs[TILE_AHEAD];
+#pragma unroll
+    for (u32 k = 0; k < TILE_AHEAD; ++k) {
+      u32 const i = c + k * 32 + lane;
+      sgs[k] = i < end ? es[i] : INV;
     }
-    __syncwarp();
+#pragma unroll
+    for (u32 k = 0; k < TILE_AHEAD; ++k) {
+      u32 const sg = sgs[k], mask = __ballot_sync(FULL_MASK, sg != INV);
+      if (!mask) break;
+      if (__all_sync(FULL_MASK, sg == cur || sg == INV)) {
+        cnt += __popc(mask);
+        continue;
+      }
+      if (cnt && lane == 0) hist[(size_t)cur * ntiles + tile] += cnt;
+      __syncwarp();
+      cur = __shfl_sync(FULL_MASK, sg, 0);
+      cnt = 0;
+      u32 const peers = __match_any_sync(FULL_MASK, sg);
+      if (sg == cur) cnt = __popc(peers);
+      cnt = __shfl_sync(FULL_MASK, cnt, 0);
+      if (sg != INV && sg != cur && lane == (u32)(__ffs(peers) - 1))
+        hist[(size_t)sg * ntiles + tile] += __popc(peers);
+      __syncwarp();
+    }
   }
+  if (cnt && lane == 0) hist[(size_t)cur * ntiles + tile] += cnt;
 }
 
 // stable positions: run[seg * ntiles + tile] starts at the scanned histogram
-// and advances as the warp walks its tile in order
-__global__ void k_tile_scatter(u32 n, u32 const* __restrict__ es, u32 ntiles, u32* __restrict__ run,
+// and advances as the warp walks its tile in order (the position of the
+// segment in hand in a register, as in k_tile_hist)
+__global__ void k_tile_scatter(u32 n, u32 const* __restrict__ es, u32 ntiles, u32* run,
     u32* __restrict__ perm)
 {
   pdl_wait();
   u32 tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (tile >= ntiles) return;
-  u32 base = tile * SPLIT_TILE;
-  u32 lt = (1u << lane) - 1u;
-  for (u32 c = 0; c < SPLIT_TILE; c += 32) {
-    u32 i = base + c + lane;
-    bool on = i < n;
-    u32 mask = __ballot_sync(FULL_MASK, on);
-    if (!mask) break;
-    if (on) {
-      u32 sg = es[i];
-      u32 peers = __match_any_sync(mask, sg);
-      u32 leader = (u32)(__ffs(peers) - 1);
-      size_t slot = (size_t)sg * ntiles + tile;
-      u32 b = 0;
-      if (lane == leader) b = run[slot];
-      b = __shfl_sync(peers, b, leader);
-      perm[i] = b + __popc(peers & lt);
-      if (lane == leader) run[slot] = b + __popc(peers);
+  u32 const base = tile * SPLIT_TILE, end = min(n, base + SPLIT_TILE);
+  u32 const lt = (1u << lane) - 1u;
+  u32 cur = INV, at = 0;  // the segment in hand and its next position
+  for (u32 c = base; c < end; c += 32 * TILE_AHEAD) {
+    u32 sgs[TILE_AHEAD];
+#pragma unroll
+    for (u32 k = 0; k < TILE_AHEAD; ++k) {
+      u32 const i = c + k * 32 + lane;
+      sgs[k] = i < end ? es[i] : INV;
     }
-    __syncwarp();
+#pragma unroll
+    for (u32 k = 0; k < TILE_AHEAD; ++k) {
+      u32 const sg = sgs[k], i = c + k * 32 + lane, mask = __ballot_sync(FULL_MASK, sg != INV);
+      if (!mask) break;
+      if (__all_sync(FULL_MASK, sg == cur || sg == INV)) {
+        if (sg != INV) perm[i] = at + __popc(mask & lt);
+        at += __popc(mask);
+        continue;
+      }
+      if (cur != INV && lane == 0) run[(size_t)cur * ntiles + tile] = at;
+      __syncwarp();
+      u32 const peers = __match_any_sync(FULL_MASK, sg);
+      u32 const leader = (u32)(__ffs(peers) - 1);
+      size_t const slot = (size_t)sg * ntiles + tile;
+      u32 b = 0;
+      if (sg != INV && lane == leader) b = run[slot];
+      b = __shfl_sync(FULL_MASK, b, leader);
+      if (sg != INV) perm[i] = b + __popc(peers & lt);
+      cur = __shfl_sync(FULL_MASK, sg, 0);  // (lane 0's entity is always there)
+      at = __shfl_sync(FULL_MASK, b, 0) + __popc(__shfl_sync(FULL_MASK, peers, 0));
+      if (sg != INV && sg != cur && lane == leader) run[slot] = b + __popc(peers);
+      __syncwarp();
+    }
   }
 }
 
