@@ -67,52 +67,43 @@ Mesh* Mesh::spawn() const
 
 Mesh* Mesh::clone()
 {
+  // the copies run on this mesh's stream, after its work so far
   Mesh* c = new Mesh(dim, full, parallel, nullptr);
-  stream_sync(s);
   try {
+    std::vector<CopyJob> jobs;
+    auto copied = [&](void const* src, size_t bytes) {
+      void* p = dev_alloc(bytes, s);
+      jobs.push_back(CopyJob{src, p, bytes});
+      return p;
+    };
     for (u32 d = 0; d <= dim; ++d) {
       if (!has_dim(d)) continue;
       u32 n = counts[d];
       u32* v = nullptr;
-      if (d) {
-        size_t bytes = sizeof(u32) * (size_t)n * deg(d, 0);
-        v = static_cast<u32*>(dev_alloc(bytes, c->s));
-        CK(cudaMemcpyAsync(v, down[d][0], bytes, cudaMemcpyDeviceToDevice, c->s));
-      }
+      if (d) v = static_cast<u32*>(copied(down[d][0], sizeof(u32) * (size_t)n * deg(d, 0)));
       c->set_ents(d, n, v);
-      for (auto const& t : tags[d]) {
-        size_t bytes = (size_t)n * t.ncomps * tag_esz(t.type);
-        void* p = dev_alloc(bytes, c->s);
-        CK(cudaMemcpyAsync(p, t.data, bytes, cudaMemcpyDeviceToDevice, c->s));
-        c->add_tag(d, t.type, t.name.c_str(), t.ncomps, t.transfer, p);
-      }
-      if (globals[d]) {
-        u64* g = dalloc<u64>(n, c->s);
-        CK(cudaMemcpyAsync(g, globals[d], sizeof(u64) * n, cudaMemcpyDeviceToDevice, c->s));
-        c->globals[d] = g;
-      }
+      for (auto const& t : tags[d])
+        c->add_tag(d, t.type, t.name.c_str(), t.ncomps, t.transfer,
+            copied(t.data, (size_t)n * t.ncomps * tag_esz(t.type)));
+      if (globals[d]) c->globals[d] = static_cast<u64*>(copied(globals[d], sizeof(u64) * (size_t)n));
       c->globals_iota[d] = globals_iota[d];
       c->ranks_zero[d] = ranks_zero[d];
       c->ids_iota[d] = ids_iota[d];
       u32* const* own[2] = {&own_ranks[d], &own_ids[d]};
       u32** cown[2] = {&c->own_ranks[d], &c->own_ids[d]};
       for (u32 k = 0; k < 2; ++k)
-        if (*own[k]) {
-          *cown[k] = dalloc<u32>(n ? n : 1, c->s);
-          CK(cudaMemcpyAsync(*cown[k], *own[k], sizeof(u32) * n, cudaMemcpyDeviceToDevice,
-              c->s));
-        }
+        if (*own[k]) *cown[k] = static_cast<u32*>(copied(*own[k], sizeof(u32) * (size_t)n));
     }
     c->ghost_layers = ghost_layers;
     c->fp32_filter = fp32_filter;
     if (seg) {
       c->nseg = nseg;
-      c->seg = dalloc<u32>(counts[0], c->s);
-      CK(cudaMemcpyAsync(c->seg, seg, sizeof(u32) * counts[0], cudaMemcpyDeviceToDevice,
-          c->s));
+      c->seg = static_cast<u32*>(copied(seg, sizeof(u32) * (size_t)counts[0]));
     }
-    stream_sync(c->s);
+    copy_many(jobs.data(), jobs.size(), s);
+    stream_sync(s);
   } catch (...) {
+    cudaStreamSynchronize(s);  // c frees its arrays on its own stream
     delete c;
     throw;
   }

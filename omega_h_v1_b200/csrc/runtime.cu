@@ -1065,6 +1065,56 @@ void fill_u32(u32* a, u32 n, u32 v, cudaStream_t s)
   CK_LAUNCH();
 }
 
+struct CopyJobs {
+  CopyJob j[MAX_COPY_JOBS];
+};
+
+// blockIdx.y: the job. 16-byte words, COPY_UNROLL to a thread with their
+// loads issued together (bound by DRAM); the bytes past the last word, and
+// arrays that do not start on 16 bytes, one at a time.
+constexpr u32 COPY_UNROLL = 4;
+
+__global__ void __launch_bounds__(BLOCK) k_copy_many(const __grid_constant__ CopyJobs jobs)
+{
+  pdl_wait();
+  CopyJob const jb = jobs.j[blockIdx.y];
+  size_t const t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  size_t const stride = (size_t)gridDim.x * blockDim.x;
+  bool const wide = ((reinterpret_cast<uintptr_t>(jb.src) | reinterpret_cast<uintptr_t>(jb.dst)) & 15) == 0;
+  size_t const nw = wide ? jb.bytes / 16 : 0;
+  uint4 const* __restrict__ src = static_cast<uint4 const*>(jb.src);
+  uint4* __restrict__ dst = static_cast<uint4*>(jb.dst);
+  for (size_t t = t0; t < nw; t += stride * COPY_UNROLL) {
+    uint4 v[COPY_UNROLL];
+#pragma unroll
+    for (u32 k = 0; k < COPY_UNROLL; ++k)
+      if (t + k * stride < nw) v[k] = src[t + k * stride];
+#pragma unroll
+    for (u32 k = 0; k < COPY_UNROLL; ++k)
+      if (t + k * stride < nw) dst[t + k * stride] = v[k];
+  }
+  for (size_t b = nw * 16 + t0; b < jb.bytes; b += stride)
+    static_cast<unsigned char*>(jb.dst)[b] = static_cast<unsigned char const*>(jb.src)[b];
+}
+
+void copy_many(CopyJob const* jobs, size_t njobs, cudaStream_t s)
+{
+  for (size_t at = 0; at < njobs;) {
+    CopyJobs pack;
+    u32 cnt = 0;
+    size_t most = 0;
+    for (; at < njobs && cnt < MAX_COPY_JOBS; ++at) {
+      if (!jobs[at].bytes) continue;
+      pack.j[cnt++] = jobs[at];
+      most = std::max(most, jobs[at].bytes);
+    }
+    if (!cnt) return;
+    u32 const gx = (u32)std::min<size_t>(ceil_div(most, 16 * COPY_UNROLL * BLOCK), 148 * 8);
+    CK(launch_kernel(k_copy_many, dim3(gx, cnt), dim3(BLOCK), 0, s, pack));
+    CK_LAUNCH();
+  }
+}
+
 __global__ void k_iota(u32* a, u32 n, u32 stride)
 {
   pdl_wait();

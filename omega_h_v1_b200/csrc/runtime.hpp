@@ -132,6 +132,17 @@ u32* negate_offsets(u32 const* offs, u32 n, cudaStream_t s, u32* total_to = null
 
 void fill_u32(u32* a, u32 n, u32 v, cudaStream_t s);
 
+// device arrays copied to others that they do not overlap, MAX_COPY_JOBS to
+// a launch (a mesh's connectivity and tags are a dozen arrays, and a driver
+// copy costs the host 8 us whatever its size)
+constexpr u32 MAX_COPY_JOBS = 16;
+struct CopyJob {
+  void const* src;
+  void* dst;
+  size_t bytes;
+};
+void copy_many(CopyJob const* jobs, size_t njobs, cudaStream_t s);
+
 // grow the device's memory pool to at least `bytes` now (the pool keeps what
 // it holds), so that later passes do not pay for growing it
 void pool_reserve(unsigned long long bytes);

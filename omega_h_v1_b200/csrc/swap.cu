@@ -519,23 +519,25 @@ static bool swap_build(Mesh& m, SwapSel const& sel, bool deferred)
   u32 ne = m.count(1), nv = m.count(0), dim = m.dim;
   Mesh* out = m.spawn();
   out->set_ents(0, nv, nullptr);
+  std::vector<CopyJob> vcopies;  // the vertices' arrays, in one launch
   for (auto const& t : m.tags[0]) {
     size_t bytes = (size_t)nv * t.ncomps * tag_esz(t.type);
     void* d = dev_alloc(bytes, s);
-    CK(cudaMemcpyAsync(d, t.data, bytes, cudaMemcpyDeviceToDevice, s));
+    vcopies.push_back(CopyJob{t.data, d, bytes});
     out->add_tag(0, t.type, t.name.c_str(), t.ncomps, t.transfer, d);
   }
   if (m.seg) {
     out->seg = dalloc<u32>(nv, s);
-    CK(cudaMemcpyAsync(out->seg, m.seg, sizeof(u32) * nv, cudaMemcpyDeviceToDevice, s));
+    vcopies.push_back(CopyJob{m.seg, out->seg, sizeof(u32) * (size_t)nv});
   }
   if (m.parallel && m.globals[0]) {
     u64* g = dalloc<u64>(nv, s);
-    CK(cudaMemcpyAsync(g, m.globals[0], sizeof(u64) * nv, cudaMemcpyDeviceToDevice, s));
+    vcopies.push_back(CopyJob{m.globals[0], g, sizeof(u64) * (size_t)nv});
     out->set_globals(0, g);
   } else if (m.parallel && m.globals_iota[0]) {
     out->set_iota_globals(0);
   }
+  copy_many(vcopies.data(), vcopies.size(), s);
   UpAdj const& te = m.ask_up(1, 3);
   u32 const* voe1 = m.ask_down(1, 0);
   u32 const* vot = m.ask_down(3, 0);
