@@ -608,169 +608,204 @@ constexpr u32 SCAN_SPIN_LIMIT = 1u << 24;
 // claimed through one ticket, so a look-back, which stops at its job's
 // first tile, only waits on tiles claimed before it. Independent scans of a
 // pass share a launch, and their look-back chains overlap.
+//
+// A warp takes CH chunks of 128 consecutive items, a lane 4 consecutive ones
+// of each, as one 16-byte word where every array of the job starts on 16
+// bytes: loads and stores are coalesced as they stand, the chunks' scans are
+// independent shuffles, and nothing is transposed through shared memory
+// (which took four shared-memory accesses an item and half the issue slots:
+// 15.6 us a launch over a 48^3 adapt, now 13). A launch of one tile needs no ticket, status or clean-up.
+__device__ inline void scan_store4(u32* __restrict__ a, size_t gi, u32 n, bool wide, u32 x0,
+    u32 x1, u32 x2, u32 x3)
+{
+  if (wide && gi + 4 <= n) {
+    *reinterpret_cast<uint4*>(a + gi) = make_uint4(x0, x1, x2, x3);
+    return;
+  }
+  if (gi < n) a[gi] = x0;
+  if (gi + 1 < n) a[gi + 1] = x1;
+  if (gi + 2 < n) a[gi + 2] = x2;
+  if (gi + 3 < n) a[gi + 3] = x3;
+}
+
 template <int SCAN_T, int SCAN_ITEMS>
 __global__ void __launch_bounds__(SCAN_T)
-k_exscan(ScanJobs jobs, unsigned long long* status, u32* ticket_and_err, u32 spin_limit)
+k_exscan(const __grid_constant__ ScanJobs jobs, unsigned long long* status,
+    u32* ticket_and_err, u32 spin_limit)
 {
   pdl_wait();
-  constexpr int SCAN_THREADS = SCAN_T, SCAN_WARPS = SCAN_T / 32;
+  constexpr u32 WARPS = SCAN_T / 32, CH = SCAN_ITEMS / 4;
+  constexpr u32 SCAN_TILE = SCAN_T * SCAN_ITEMS;
   __shared__ u32 s_tile;
-  __shared__ u32 s_warp[SCAN_WARPS];
+  __shared__ u32 s_warp[WARPS];
   __shared__ u32 s_prefix;
-  constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-  __shared__ u32 s_buf[SCAN_TILE + SCAN_TILE / 32];
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket_and_err, 1u);
-  __syncthreads();
-  u32 const tile = s_tile;
   u32 const ntiles = jobs.tile0[jobs.njobs];
-  if (tile >= ntiles) return;
+  bool const single = ntiles == 1;
+  u32 tile = 0;
+  if (!single) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket_and_err, 1u);
+    __syncthreads();
+    tile = s_tile;
+    if (tile >= ntiles) return;
+  }
   u32 jn = 0;
   while (jn + 1 < jobs.njobs && tile >= jobs.tile0[jn + 1]) ++jn;
   ScanJob const job = jobs.j[jn];
   u32 const first = jobs.tile0[jn], last = jobs.tile0[jn + 1] - 1;
   u32 const* __restrict__ in = job.in;
-  u32 const n = job.n;
-  bool const mode1 = job.mode == 1, mode2 = job.mode == 2;
-  u32 const stamp = job.stamp;
-  size_t const base = (size_t)(tile - first) * SCAN_TILE;
-  // coalesced load into shared memory (padded to avoid bank conflicts)
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    u32 li = k * SCAN_THREADS + threadIdx.x;
-    size_t gi = base + li;
-    u32 v = 0;
-    if (gi < n)
-      v = mode2 ? (in[gi] == stamp ? 1u : 0u)
-                : !mode1 ? in[gi] : (in[gi + 1] == in[gi] ? 1u : 0u);
-    s_buf[li + (li >> 5)] = v;
-  }
-  __syncthreads();
-  u32 v[SCAN_ITEMS];
-  u32 sum = 0;
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    u32 li = threadIdx.x * SCAN_ITEMS + k;
-    v[k] = s_buf[li + (li >> 5)];
-    sum += v[k];
-  }
-  u32 const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  u32 x = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    u32 y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= (u32)o) x += y;
-  }
-  if (lane == 31) s_warp[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    u32 w = lane < SCAN_WARPS ? s_warp[lane] : 0u;
-#pragma unroll
-    for (int o = 1; o < SCAN_WARPS; o <<= 1) {
-      u32 y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= (u32)o) w += y;
-    }
-    if (lane < SCAN_WARPS) s_warp[lane] = w;
-  }
-  __syncthreads();
-  u32 const thread_excl = (warp ? s_warp[warp - 1] : 0u) + x - sum;
-  u32 const total = s_warp[SCAN_WARPS - 1];
-  if (warp == 0) {
-    // warp-cooperative look-back: lane l inspects tile (p - l)
-    u32 prefix = 0;
-    if (tile == first) {
-      if (lane == 0) atomicExch(&status[tile], FLAG_PRE | (unsigned long long)total);
-    } else {
-      if (lane == 0) atomicExch(&status[tile], FLAG_AGG | (unsigned long long)total);
-      int p = (int)tile - 1;
-      u32 spins = 0;
-      bool gave_up = false;
-      for (;;) {
-        int idx = p - (int)lane;
-        unsigned long long st = FLAG_PRE;  // before the job's first tile: empty
-        if (idx >= (int)first) st = *((volatile unsigned long long*)&status[idx]);
-        while (__any_sync(0xffffffffu, (st >> 62) == 0)) {
-          if (++spins > spin_limit) {
-            gave_up = true;
-            break;
-          }
-          if (idx >= (int)first && (st >> 62) == 0)
-            st = *((volatile unsigned long long*)&status[idx]);
-        }
-        if (gave_up) {
-          if (lane == 0) atomicOr(&ticket_and_err[1], 1u);
-          break;
-        }
-        u32 pre = __ballot_sync(0xffffffffu, (st & (3ull << 62)) == FLAG_PRE);
-        u32 stop = pre ? (u32)(__ffs(pre) - 1) : 31u;
-        u32 val = (lane <= stop) ? (u32)st : 0u;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
-        prefix += val;
-        if (pre) break;
-        p -= 32;
-      }
-      if (lane == 0) atomicExch(&status[tile], FLAG_PRE | (unsigned long long)(prefix + total));
-    }
-    if (lane == 0) s_prefix = prefix;
-  }
-  __syncthreads();
   u32* __restrict__ out = job.out;
   u32* __restrict__ newid = job.newid;
   u32* __restrict__ list = job.list;
   u32* __restrict__ comp = job.comp;
   u32* __restrict__ comp_newid = job.comp_newid;
-  // jobs that need each item's mark keep it in bit 31 of its staged prefix
-  // (their prefixes count marked entities: below 2^31), so the store phase
-  // does not read the items again
-  bool const need_on = newid || list || comp_newid;
-  constexpr u32 ON_BIT = 0x80000000u;
-  u32 run = s_prefix + thread_excl;
+  u32 const n = job.n;
+  u32 const mode = job.mode, stamp = job.stamp;
+  bool const wide = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) |
+      reinterpret_cast<uintptr_t>(newid) | reinterpret_cast<uintptr_t>(comp) |
+      reinterpret_cast<uintptr_t>(comp_newid)) & 15) == 0;
+  u32 const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  size_t const base = (size_t)(tile - first) * SCAN_TILE + warp * (CH * 128) + lane * 4;
+  u32 v[CH][4];
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    u32 li = threadIdx.x * SCAN_ITEMS + k;
-    s_buf[li + (li >> 5)] = run | (need_on && v[k] ? ON_BIT : 0u);
-    run += v[k];
+  for (u32 c = 0; c < CH; ++c) {
+    size_t const gi = base + c * 128;
+    if (wide && gi + 4 <= n) {
+      uint4 const x = *reinterpret_cast<uint4 const*>(in + gi);
+      v[c][0] = x.x, v[c][1] = x.y, v[c][2] = x.z, v[c][3] = x.w;
+    } else {
+#pragma unroll
+      for (u32 k = 0; k < 4; ++k) v[c][k] = gi + k < n ? in[gi + k] : 0u;
+    }
+  }
+  if (mode == 1) {
+    // (in has n + 1 entries; an item's right neighbour is the next lane's
+    // first, or the entry after the chunk)
+#pragma unroll
+    for (u32 c = 0; c < CH; ++c) {
+      size_t const gi = base + c * 128;
+      u32 next = __shfl_down_sync(0xffffffffu, v[c][0], 1);
+      if (gi + 4 >= n || lane == 31) next = gi + 4 <= n ? in[gi + 4] : 0u;
+      u32 const tail = gi < n ? in[n] : 0u;  // the last item's neighbour
+#pragma unroll
+      for (u32 k = 0; k < 4; ++k) {
+        u32 const r = gi + k + 1 == n ? tail : k < 3 ? v[c][k < 3 ? k + 1 : 3] : next;
+        v[c][k] = gi + k < n && r == v[c][k] ? 1u : 0u;
+      }
+    }
+  } else if (mode == 2) {
+#pragma unroll
+    for (u32 c = 0; c < CH; ++c)
+#pragma unroll
+      for (u32 k = 0; k < 4; ++k) v[c][k] = base + c * 128 + k < n && v[c][k] == stamp ? 1u : 0u;
+  }
+  u32 excl[CH];  // the lane's first item's prefix within the warp
+  {
+    u32 x[CH], sum[CH];
+#pragma unroll
+    for (u32 c = 0; c < CH; ++c) x[c] = sum[c] = v[c][0] + v[c][1] + v[c][2] + v[c][3];
+#pragma unroll
+    for (u32 o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (u32 c = 0; c < CH; ++c) {
+        u32 const y = __shfl_up_sync(0xffffffffu, x[c], o);
+        if (lane >= o) x[c] += y;
+      }
+    u32 run = 0;
+#pragma unroll
+    for (u32 c = 0; c < CH; ++c) {
+      excl[c] = run + x[c] - sum[c];
+      run += __shfl_sync(0xffffffffu, x[c], 31);
+    }
+    if (lane == 0) s_warp[warp] = run;
   }
   __syncthreads();
+  u32 before = 0, total = 0;  // the warps before this one; the tile
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    u32 li = k * SCAN_THREADS + threadIdx.x;
-    size_t gi = base + li;
-    if (gi < n) {
-      u32 const w = s_buf[li + (li >> 5)];
-      u32 const o = need_on ? w & ~ON_BIT : w;
-      out[gi] = o;
-      if (comp) comp[gi] = (u32)gi - o;
-      if (need_on) {
-        bool const on = (w & ON_BIT) != 0;
-        if (newid) newid[gi] = on ? o : INV;
-        if (list && on) list[o] = (u32)gi;
-        if (comp_newid) comp_newid[gi] = on ? INV : (u32)gi - o;
+  for (u32 w = 0; w < WARPS; ++w) {
+    u32 const t = s_warp[w];
+    if (w < warp) before += t;
+    total += t;
+  }
+  u32 prefix = 0;
+  if (tile != first || !single) {
+    if (warp == 0) {
+      // warp-cooperative look-back: lane l inspects tile (p - l)
+      if (tile == first) {
+        if (lane == 0) atomicExch(&status[tile], FLAG_PRE | (unsigned long long)total);
+      } else {
+        if (lane == 0) atomicExch(&status[tile], FLAG_AGG | (unsigned long long)total);
+        int p = (int)tile - 1;
+        u32 spins = 0;
+        bool gave_up = false;
+        for (;;) {
+          int idx = p - (int)lane;
+          unsigned long long st = FLAG_PRE;  // before the job's first tile: empty
+          if (idx >= (int)first) st = *((volatile unsigned long long*)&status[idx]);
+          while (__any_sync(0xffffffffu, (st >> 62) == 0)) {
+            if (++spins > spin_limit) {
+              gave_up = true;
+              break;
+            }
+            if (idx >= (int)first && (st >> 62) == 0)
+              st = *((volatile unsigned long long*)&status[idx]);
+          }
+          if (gave_up) {
+            if (lane == 0) atomicOr(&ticket_and_err[1], 1u);
+            break;
+          }
+          u32 pre = __ballot_sync(0xffffffffu, (st & (3ull << 62)) == FLAG_PRE);
+          u32 stop = pre ? (u32)(__ffs(pre) - 1) : 31u;
+          prefix += __reduce_add_sync(0xffffffffu, lane <= stop ? (u32)st : 0u);
+          if (pre) break;
+          p -= 32;
+        }
+        if (lane == 0) atomicExch(&status[tile], FLAG_PRE | (unsigned long long)(prefix + total));
       }
+      if (lane == 0) s_prefix = prefix;
+    }
+    __syncthreads();
+    prefix = s_prefix;
+  }
+  // counted once the look-back is over; the count is looked at after the
+  // stores, so its round trip is not waited for
+  u32 done = 0;
+  if (!single && threadIdx.x == 0) done = atomicAdd(&ticket_and_err[2], 1u);
+  bool const marks = newid || list || comp_newid;
+#pragma unroll
+  for (u32 c = 0; c < CH; ++c) {
+    size_t const gi = base + c * 128;
+    if (gi >= n) break;
+    u32 const g = (u32)gi;
+    u32 const o0 = prefix + before + excl[c], o1 = o0 + v[c][0], o2 = o1 + v[c][1], o3 = o2 + v[c][2];
+    scan_store4(out, gi, n, wide, o0, o1, o2, o3);
+    if (comp) scan_store4(comp, gi, n, wide, g - o0, g + 1 - o1, g + 2 - o2, g + 3 - o3);
+    if (!marks) continue;
+    // (0/1 items)
+    if (newid)
+      scan_store4(newid, gi, n, wide, v[c][0] ? o0 : INV, v[c][1] ? o1 : INV,
+          v[c][2] ? o2 : INV, v[c][3] ? o3 : INV);
+    if (comp_newid)
+      scan_store4(comp_newid, gi, n, wide, v[c][0] ? INV : g - o0, v[c][1] ? INV : g + 1 - o1,
+          v[c][2] ? INV : g + 2 - o2, v[c][3] ? INV : g + 3 - o3);
+    if (list) {
+      if (v[c][0]) list[o0] = g;
+      if (v[c][1]) list[o1] = g + 1;
+      if (v[c][2]) list[o2] = g + 2;
+      if (v[c][3]) list[o3] = g + 3;
     }
   }
   if (tile == last && threadIdx.x == 0) {
-    out[n] = s_prefix + total;
-    if (comp) comp[n] = n - (s_prefix + total);
-    if (job.total_to) *job.total_to = s_prefix + total;
+    out[n] = prefix + total;
+    if (comp) comp[n] = n - (prefix + total);
+    if (job.total_to) *job.total_to = prefix + total;
   }
-  // The last tile to finish returns the scratch to zero for the next scan
-  // on the stream: every other tile has counted itself done, so no look-back
-  // reads a status word any more.
-  __shared__ u32 s_last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(&ticket_and_err[2], 1u) == ntiles - 1 ? 1u : 0u;
-  }
-  __syncthreads();
-  if (s_last) {
-    for (u32 t = threadIdx.x; t < ntiles; t += blockDim.x) status[t] = 0ull;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  // The last tile past its look-back returns the scratch to zero for the
+  // next scan on the stream: no look-back reads a status word any more.
+  if (!single && warp == 0 && __shfl_sync(0xffffffffu, done, 0) == ntiles - 1) {
+    for (u32 t = lane; t < ntiles; t += 32) status[t] = 0ull;
+    if (lane == 0) {
       ticket_and_err[0] = 0;
       ticket_and_err[2] = 0;
-      __threadfence();
     }
   }
 }
@@ -919,12 +954,23 @@ struct ScanShape {
   u32 tile() const { return threads * items; }
 };
 ScanShape tuned_scan_shape() { return {tuned(TK_SCAN_THREADS), tuned(TK_SCAN_ITEMS)}; }
+// A large scan is bound by the tiles' look-backs rather than by its bytes,
+// so it takes the widest tile that keeps three blocks on an SM (28M items:
+// 59 us with 16 items a thread, 51 with 32; 6M: 14 and 12); below LONG_SCAN
+// items the two are level and the smaller tile starts sooner.
+constexpr u64 LONG_SCAN = 4u << 20;
+ScanShape scan_shape_for(u64 items)
+{
+  ScanShape const sh = tuned_scan_shape();
+  return items >= LONG_SCAN && sh.items == 16 ? ScanShape{256, 32} : sh;
+}
 
 void launch_scan_jobs(ScanJobs const& jobs, ScanShape sh, u32* scratch, u32 spin_limit,
     cudaStream_t s)
 {
   u32 const ntiles = jobs.tile0[jobs.njobs];
-  auto k = sh.threads == 256 ? (sh.items == 8 ? k_exscan<256, 8> : k_exscan<256, 16>)
+  auto k = sh.items == 32   ? k_exscan<256, 32>
+           : sh.threads == 256 ? (sh.items == 8 ? k_exscan<256, 8> : k_exscan<256, 16>)
                              : (sh.items == 8 ? k_exscan<512, 8> : k_exscan<512, 16>);
   CK(launch_kernel(k, dim3(ntiles), dim3(sh.threads), 0, s, jobs,
       reinterpret_cast<unsigned long long*>(scratch + 4), scratch, spin_limit));
@@ -934,11 +980,13 @@ void launch_scan_jobs(ScanJobs const& jobs, ScanShape sh, u32* scratch, u32 spin
 
 void exscan_jobs(ScanJob const* jobs, u32 njobs, cudaStream_t s)
 {
-  ScanShape const sh = tuned_scan_shape();
-  u32 const tile = sh.tile();
   for (u32 at = 0; at < njobs; at += MAX_SCAN_JOBS) {
     ScanJobs pack;
     pack.njobs = std::min<u32>(MAX_SCAN_JOBS, njobs - at);
+    u64 total = 0;
+    for (u32 q = 0; q < pack.njobs; ++q) total += jobs[at + q].n;
+    ScanShape const sh = scan_shape_for(total);
+    u32 const tile = sh.tile();
     pack.tile0[0] = 0;
     double bytes = 0;
     for (u32 q = 0; q < pack.njobs; ++q) {
