@@ -1237,7 +1237,7 @@ void adapt_batch(std::vector<Mesh*> const& ms, double size_floor, double good_qu
   GroupRunner run;
   run.ap = AdaptParams{size_floor, good_qual, nlayers, max_ops};
   run.max_union_elems = max_union_elems;
-  CK(cudaStreamCreateWithFlags(&run.s, cudaStreamNonBlocking));
+  run.s = take_stream();
   std::vector<Mesh*> cur(ms.begin(), ms.end());
   std::vector<char> owned(n, 0);
   std::vector<SegState> st(n);
@@ -1247,9 +1247,8 @@ void adapt_batch(std::vector<Mesh*> const& ms, double size_floor, double good_qu
     for (u32 k = 0; k < n; ++k)
       if (owned[k]) delete cur[k];
     st.clear();  // and with it any union still kept
-    release_stream_scratch(run.s);
     cudaStreamSynchronize(run.s);
-    cudaStreamDestroy(run.s);
+    give_back_stream(run.s);
   };
   try {
     while (run.step(cur, st, owned)) {

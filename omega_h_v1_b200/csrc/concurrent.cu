@@ -186,7 +186,7 @@ void adapt_concurrent(std::vector<Mesh*> const& ms, AdaptParams const& ap, u32 n
     cudaStream_t st = nullptr;
     try {
       CK(cudaSetDevice(dev));
-      CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      st = take_stream();
     } catch (Failure const& f) {
       std::lock_guard<std::mutex> g(mu);
       if (!first_error) {
@@ -280,9 +280,8 @@ void adapt_concurrent(std::vector<Mesh*> const& ms, AdaptParams const& ap, u32 n
       }
       cv.notify_all();
     }
-    release_stream_scratch(st);
     cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
+    give_back_stream(st);
   };
   std::vector<std::thread> th;
   for (u32 t = 0; t < nthreads; ++t) th.emplace_back(worker);

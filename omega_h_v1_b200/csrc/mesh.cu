@@ -32,7 +32,7 @@ Mesh::Mesh(u32 d, bool f, bool p, cudaStream_t stream,
     : dim(d), full(f), parallel(p), s(stream), mb(mailbox)
 {
   if (!s && !exact_stream) {
-    CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    s = take_stream();
     own_stream = true;
   }
   if (!mb) {
@@ -47,12 +47,10 @@ Mesh::~Mesh()
     clear_contents();
   } catch (...) {
   }
-  if (own_stream) {
-    mb.reset();
-    release_stream_scratch(s);
-    cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-  }
+  // (a mailbox goes back with no kernel pending that writes it)
+  if (own_stream || mb.use_count() == 1) cudaStreamSynchronize(s);
+  mb.reset();
+  if (own_stream) give_back_stream(s);
 }
 
 Mesh* Mesh::spawn() const
@@ -114,7 +112,7 @@ void Mesh::own_new_stream()
 {
   stream_sync(s);
   if (own_stream) return;
-  CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  s = take_stream();
   own_stream = true;
   mb = std::shared_ptr<Mailbox>(new Mailbox(), release_mailbox);
   mb->init(s);
@@ -123,10 +121,7 @@ void Mesh::own_new_stream()
 void Mesh::use_stream(cudaStream_t stream)
 {
   stream_sync(s);
-  if (own_stream) {
-    release_stream_scratch(s);
-    CK(cudaStreamDestroy(s));
-  }
+  if (own_stream) give_back_stream(s);
   own_stream = false;
   s = stream;
 }

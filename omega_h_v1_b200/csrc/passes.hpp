@@ -121,7 +121,7 @@ struct Counter {
     d = dalloc<u32>(1, s);
     CK(cudaMemsetAsync(d, 0, sizeof(u32), s));
   }
-  ~Counter() { cudaFreeAsync(d, s); }
+  ~Counter() { dev_free(d, s); }
   void zero() { CK(cudaMemsetAsync(d, 0, sizeof(u32), s)); }
   u32 get() { return read_u32(d, s); }
 };

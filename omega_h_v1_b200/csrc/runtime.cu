@@ -11,6 +11,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <unordered_map>
 #include <vector>
 
 #include "runtime.hpp"
@@ -381,19 +382,177 @@ static void setup_pool()
   });
 }
 
+// Blocks of up to BLOCK_MAX bytes that dev_free gets back are kept for the
+// next dev_alloc on the same stream, by size class (four to an octave), up
+// to KEEP_MAX bytes a stream: a pass on a small mesh makes and drops some
+// forty arrays, and a call into the driver's pool for each took longer than
+// its kernels (0.6 to 1.9 us a call, 735 calls in a 6^3 adapt of 188
+// launches). Order is the stream's, as the driver's pool keeps it. The
+// blocks go back to that pool when the stream's scratch is released
+// (release_stream_scratch), when an allocation fails, and past KEEP_MAX. A
+// stream under capture goes to the driver's pool, whose calls are captured.
+namespace {
+constexpr size_t BLOCK_MAX = 4u << 20, KEEP_MAX = 256u << 20;
+constexpr u32 BLOCK_CLASSES = 1 + 13 * 4;  // 512 bytes; then 2^9 .. 2^22 in quarters
+
+u32 block_class(size_t bytes, size_t* rounded)
+{
+  if (bytes <= 512) {
+    *rounded = 512;
+    return 0;
+  }
+  u32 const l = 63 - (u32)__builtin_clzll((unsigned long long)(bytes - 1));  // >= 9
+  size_t const base = (size_t)1 << l, step = base / 4;
+  u32 const k = (u32)((bytes - 1 - base) / step);
+  *rounded = base + (k + 1) * step;
+  return 1 + (l - 9) * 4 + k;
+}
+
+size_t class_bytes(u32 c)
+{
+  if (!c) return 512;
+  size_t const base = (size_t)1 << (9 + (c - 1) / 4);
+  return base + ((c - 1) % 4 + 1) * (base / 4);
+}
+
+struct KeptBlocks {
+  std::vector<void*> free_of[BLOCK_CLASSES];
+  size_t bytes = 0;
+};
+
+struct BlockTable {
+  std::mutex mu;
+  std::map<std::pair<int, cudaStream_t>, KeptBlocks> kept;
+  std::unordered_map<void*, std::pair<int, u32>> made;  // (device, class) of each block
+  size_t kept_bytes[64] = {};
+};
+BlockTable& blocks()
+{
+  static auto* t = new BlockTable();  // lives to exit
+  return *t;
+}
+
+// (the table's lock held) every kept block of a stream back to the pool
+void drop_kept_blocks(BlockTable& t, std::map<std::pair<int, cudaStream_t>, KeptBlocks>::iterator it)
+{
+  for (auto& list : it->second.free_of)
+    for (void* p : list) {
+      t.made.erase(p);
+      cudaFreeAsync(p, it->first.second);
+    }
+  t.kept_bytes[it->first.first & 63] -= it->second.bytes;
+  t.kept.erase(it);
+}
+
+bool capturing(cudaStream_t s)
+{
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // (the legacy stream while another captures)
+  return true;
+}
+
+// streams and mailboxes that meshes gave back, for the next mesh: a stream
+// takes the driver about 70 us to make and 80 to destroy
+constexpr size_t SPARE_MAX = 64;
+struct Spares {
+  std::mutex mu;
+  std::map<cudaStream_t, int> made_on;  // the device of each stream made here
+  std::map<int, std::vector<cudaStream_t>> streams;
+  std::map<int, std::vector<Mailbox>> boxes;
+};
+Spares& spares()
+{
+  static auto* t = new Spares();
+  return *t;
+}
+}  // namespace
+
+cudaStream_t take_stream()
+{
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  Spares& sp = spares();
+  {
+    std::lock_guard<std::mutex> g(sp.mu);
+    auto& v = sp.streams[dev];
+    if (!v.empty()) {
+      cudaStream_t s = v.back();
+      v.pop_back();
+      return s;
+    }
+  }
+  cudaStream_t s = nullptr;
+  CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  std::lock_guard<std::mutex> g(sp.mu);
+  sp.made_on[s] = dev;
+  return s;
+}
+
+void give_back_stream(cudaStream_t s)
+{
+  release_stream_scratch(s);
+  Spares& sp = spares();
+  {
+    std::lock_guard<std::mutex> g(sp.mu);
+    auto it = sp.made_on.find(s);
+    if (it != sp.made_on.end()) {
+      auto& v = sp.streams[it->second];
+      if (v.size() < SPARE_MAX && cudaStreamQuery(s) != cudaErrorInvalidResourceHandle) {
+        v.push_back(s);
+        return;
+      }
+      sp.made_on.erase(it);
+    }
+  }
+  cudaStreamDestroy(s);
+}
+
 void* dev_alloc(size_t bytes, cudaStream_t s)
 {
   setup_pool();
   void* p = nullptr;
   if (bytes < 16) bytes = 16;
   g_allocs.fetch_add(1, std::memory_order_relaxed);
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  BlockTable& t = blocks();
+  bool const small = bytes <= BLOCK_MAX && !capturing(s);
+  u32 cls = 0;
+  if (small) {
+    cls = block_class(bytes, &bytes);
+    std::lock_guard<std::mutex> g(t.mu);
+    auto it = t.kept.find({dev, s});
+    if (it != t.kept.end() && !it->second.free_of[cls].empty()) {
+      p = it->second.free_of[cls].back();
+      it->second.free_of[cls].pop_back();
+      it->second.bytes -= bytes;
+      t.kept_bytes[dev & 63] -= bytes;
+      return p;
+    }
+  }
   cudaError_t e = cudaMallocAsync(&p, bytes, s);
+  if (e == cudaErrorMemoryAllocation) {
+    // once more with what this stream keeps
+    cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> g(t.mu);
+      auto it = t.kept.find({dev, s});
+      if (it != t.kept.end()) drop_kept_blocks(t, it);
+    }
+    e = cudaMallocAsync(&p, bytes, s);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     char buf[128];
     snprintf(buf, sizeof(buf), "device allocation of %zu bytes failed", bytes);
     throw Failure(E_NOMEM, buf);
   }
+  std::lock_guard<std::mutex> g(t.mu);
+  if (small)
+    t.made[p] = {dev, cls};
+  else
+    t.made.erase(p);
   return p;
 }
 
@@ -424,6 +583,12 @@ void pool_stats(unsigned long long* reserved, unsigned long long* used,
   CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &u));
   CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &h));
   if (reserved) *reserved = r;
+  // the blocks kept for the next allocations are not in use
+  {
+    BlockTable& t = blocks();
+    std::lock_guard<std::mutex> g(t.mu);
+    u -= std::min<unsigned long long>(u, t.kept_bytes[dev & 63]);
+  }
   if (used) *used = u;
   if (used_high) *used_high = h;
   if (reset_high) {
@@ -434,7 +599,27 @@ void pool_stats(unsigned long long* reserved, unsigned long long* used,
 
 void dev_free(void* p, cudaStream_t s)
 {
-  if (p) CK(cudaFreeAsync(p, s));
+  if (!p) return;
+  BlockTable& t = blocks();
+  bool const keep = !capturing(s);
+  {
+    std::lock_guard<std::mutex> g(t.mu);
+    auto it = t.made.find(p);
+    if (it != t.made.end()) {
+      int const dev = it->second.first;
+      u32 const cls = it->second.second;
+      size_t const bytes = class_bytes(cls);
+      KeptBlocks& k = t.kept[{dev, s}];
+      if (keep && k.bytes + bytes <= KEEP_MAX) {
+        k.free_of[cls].push_back(p);
+        k.bytes += bytes;
+        t.kept_bytes[dev & 63] += bytes;
+        return;
+      }
+      t.made.erase(it);
+    }
+  }
+  CK(cudaFreeAsync(p, s));
 }
 
 namespace {
@@ -496,6 +681,22 @@ double read_f64(double const* d, cudaStream_t s)
 void Mailbox::init(cudaStream_t s)
 {
   if (host) return;
+  int d = 0;
+  CK(cudaGetDevice(&d));
+  {
+    Spares& sp = spares();
+    std::lock_guard<std::mutex> g(sp.mu);
+    auto& v = sp.boxes[d];
+    if (!v.empty()) {
+      *this = v.back();
+      v.pop_back();
+    }
+  }
+  if (host) {  // (its sequence goes on: the host word holds the last number)
+    clear(s);
+    return;
+  }
+  device = d;
   // the sequence word on a line of its own
   CK(cudaMallocHost(&host, (SEQ_SLOT + 32) * sizeof(u32)));
   std::memset(host, 0, (SEQ_SLOT + 32) * sizeof(u32));
@@ -503,12 +704,27 @@ void Mailbox::init(cudaStream_t s)
   CK(cudaHostGetDevicePointer(&hd, host, 0));
   hdev = static_cast<u32*>(hd);
   seq = 0;
-  dev = dalloc<u32>(64, s);
+  // (not one of the kept blocks: it outlives any stream)
+  void* p = nullptr;
+  CK(cudaMalloc(&p, 64 * sizeof(u32)));
+  dev = static_cast<u32*>(p);
   clear(s);
 }
 
 void Mailbox::release()
 {
+  if (host && dev) {
+    Spares& sp = spares();
+    std::lock_guard<std::mutex> g(sp.mu);
+    auto& v = sp.boxes[device];
+    if (v.size() < SPARE_MAX) {
+      v.push_back(*this);
+      host = nullptr;
+      hdev = nullptr;
+      dev = nullptr;
+      return;
+    }
+  }
   if (host) cudaFreeHost(host);
   if (dev) cudaFree(dev);
   host = nullptr;
@@ -908,6 +1124,12 @@ void release_stream_scratch(cudaStream_t s)
 {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
+  {
+    BlockTable& t = blocks();
+    std::lock_guard<std::mutex> g(t.mu);
+    auto it = t.kept.find({dev, s});
+    if (it != t.kept.end()) drop_kept_blocks(t, it);
+  }
   {
     std::lock_guard<std::mutex> g(g_scan_mu);
     auto& all = scan_scratches();

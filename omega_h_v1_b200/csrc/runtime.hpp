@@ -112,6 +112,11 @@ inline u32 resident_blocks(K kernel, u32 block, size_t smem = 0)
 // current device; called before a stream is destroyed, so that scratch does
 // not outlive its stream (no kernel may use it afterwards)
 void release_stream_scratch(cudaStream_t s);
+
+// a non-blocking stream of the current device, and one back (its scratch
+// released; its work may still run: the next user's comes after it)
+cudaStream_t take_stream();
+void give_back_stream(cudaStream_t s);
 u32* stream_marks(u32 key, size_t words, cudaStream_t s, u32* gen);
 
 // The same scan with caller-provided scratch of at least
@@ -254,6 +259,9 @@ struct Mailbox {
   u32* hdev = nullptr;   // host's device address
   u32* dev = nullptr;    // device, 64 slots
   u32 seq = 0;
+  int device = 0;
+  // init takes a mailbox another mesh gave back where there is one; release
+  // gives it back, so no kernel that writes its slots may be pending then
   void init(cudaStream_t s);
   void release();
   void clear(cudaStream_t s);                 // zero the device slots

@@ -114,9 +114,8 @@ struct Server {
     st.clear();  // and with it any union still kept
     jobs.clear();
     if (run.s) {
-      release_stream_scratch(run.s);
       cudaStreamSynchronize(run.s);
-      cudaStreamDestroy(run.s);
+      give_back_stream(run.s);
     }
   }
 
@@ -289,7 +288,7 @@ Server* server_new(AdaptParams const& ap, unsigned long long budget)
   sv->run.hand_back = true;
   sv->budget = budget;
   sv->t0 = now_s();
-  CK(cudaStreamCreateWithFlags(&sv->run.s, cudaStreamNonBlocking));
+  sv->run.s = take_stream();
   return sv;
 }
 

@@ -286,8 +286,8 @@ struct Reader {
   {
     if (dtext) {
       cudaStreamSynchronize(s);
-      cudaFreeAsync(dtext, s);
-      cudaFreeAsync(dbad, s);
+      dev_free(dtext, s);
+      dev_free(dbad, s);
     }
     if (text) cudaFreeHost(text);
   }
@@ -599,7 +599,7 @@ struct Writer {
   {
     if (f) fclose(f);
     cudaStreamSynchronize(s);
-    if (dtext) cudaFreeAsync(dtext, s);
+    dev_free(dtext, s);
     if (htext) cudaFreeHost(htext);
   }
   void close()
