@@ -55,7 +55,8 @@ double osh_b200_min_quality(osh_t m) OSH_PUBLIC;
 
 /* statistics of the last pass run on this thread: op (1 refine, 2 coarsen,
    3 swap, 4 coarsen slivers), elements in / out, selected entities and
-   independent-set rounds */
+   independent-set rounds (the set is decided without rounds: a bound on
+   those the reference would take, which may differ between runs) */
 void osh_b200_last_pass(unsigned* op, unsigned* elems_in, unsigned* elems_out,
     unsigned* nselected, unsigned* rounds) OSH_PUBLIC;
 

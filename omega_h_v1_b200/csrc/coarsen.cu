@@ -318,64 +318,9 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
   if (nflipped) atomicAdd(&fs->flips, (unsigned long long)nflipped);
 }
 
-// the candidate edges listed (a warp's candidates take consecutive slots,
-// warps in any order) and every edge's two collapse qualities zeroed (the
-// quality kernel writes the kept ones)
-// collapse_to_vert (collapses_to_verts.cpp:13-42)
-__global__ void k_collapses_to_verts(u32 nv, u32 const* __restrict__ ue_offs,
-    u32 const* __restrict__ ue, u32 const* __restrict__ ue_dirs,
-    u32 const* __restrict__ codes, double const* __restrict__ q2, u32* __restrict__ cand,
-    double* __restrict__ colq)
-{
-  pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  double maxq = 0;
-  u32 c = 0;
-  for (u32 j = ue_offs[i]; j < ue_offs[i + 1]; ++j) {
-    u32 e = ue[j], d = ue_dirs[j];
-    if (!collapses(codes[e], d)) continue;
-    double q = q2[e * 2 + d];
-    if (!c) {
-      c = 1;
-      maxq = q;
-    } else if (q > maxq) {
-      maxq = q;
-    }
-  }
-  cand[i] = c;
-  colq[i] = c ? maxq : 0.0;
-}
-
-// vertex_dest (collapses_to_verts.cpp:72-105): first edge in upward order
-// whose collapse quality equals the vertex's best
-__global__ void k_vertex_dest(u32 nv, u32 const* __restrict__ ue_offs,
-    u32 const* __restrict__ ue, u32 const* __restrict__ ue_dirs,
-    u32 const* __restrict__ voe1, u32 const* __restrict__ ind,
-    double const* __restrict__ colq, u32 const* __restrict__ codes,
-    double const* __restrict__ q2, u32* __restrict__ gen_vert)
-{
-  pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  u32 g = INV;
-  if (ind[i]) {
-    double maxq = colq[i];
-    if (maxq == 1e10) maxq = -1e10;
-    for (u32 j = ue_offs[i]; j < ue_offs[i + 1]; ++j) {
-      u32 e = ue[j], d = ue_dirs[j];
-      if (!collapses(codes[e], d)) continue;
-      double q = q2[e * 2 + d];
-      if (q == 1e10) q = -1e10;
-      if (q == maxq) {
-        g = voe1[e * 2 + (1 - d)];
-        break;
-      }
-    }
-  }
-  gen_vert[i] = g;
-}
-
+// collapse_to_vert (collapses_to_verts.cpp:13-42) and vertex_dest (:72-105:
+// the first edge in upward order whose collapse quality equals the vertex's
+// best).
 // The two vertex kernels with a group of VG lanes per vertex row (rows of
 // about 13.5 edges; VG is the tuning table's vert_group): lane l takes the
 // row's entries l, l + VG, ..., and shuffles within the group combine the
@@ -388,17 +333,18 @@ template <u32 VG>
 __global__ void k_collapses_to_verts_grouped(u32 nv, u32 const* __restrict__ ue_offs,
     u32 const* __restrict__ ue, u32 const* __restrict__ ue_dirs,
     u32 const* __restrict__ codes, double const* __restrict__ q2, u32* __restrict__ cand,
-    double* __restrict__ colq)
+    unsigned long long* __restrict__ keys, double* __restrict__ colq, u32* __restrict__ list,
+    u32* nlist, u32* __restrict__ ind)
 {
   pdl_wait();
   u32 const t = blockIdx.x * blockDim.x + threadIdx.x;
   u32 const i = t / VG, lg = t % VG;
-  if (i >= nv) return;  // a group shares i: it leaves together
   u32 const gbase = (threadIdx.x & 31) & ~(VG - 1);
   u32 const gmask = ((1u << VG) - 1u) << gbase;
   double maxq = 0;
   u32 pos = INV;  // position of the lane's best entry; INV: no collapse seen
-  for (u32 j = ue_offs[i] + lg; j < ue_offs[i + 1]; j += VG) {
+  u32 const rb = i < nv ? ue_offs[i] : 0u, re = i < nv ? ue_offs[i + 1] : 0u;
+  for (u32 j = rb + lg; j < re; j += VG) {
     u32 e = ue[j], d = ue_dirs[j];
     if (!collapses(codes[e], d)) continue;
     double q = q2[e * 2 + d];
@@ -415,10 +361,20 @@ __global__ void k_collapses_to_verts_grouped(u32 nv, u32 const* __restrict__ ue_
       pos = op;
     }
   }
-  if (lg == 0) {
-    cand[i] = pos != INV;
+  if (lg == 0 && i < nv) {
+    if (cand) cand[i] = pos != INV;
+    keys[i] = pos != INV ? indset_key(maxq) : 0ull;
     colq[i] = pos != INV ? maxq : 0.0;
+    ind[i] = 0;
   }
+  // the candidates listed for the independent set, a warp's in one update
+  u32 const lane = threadIdx.x & 31;
+  u32 const m = __ballot_sync(0xffffffffu, lg == 0 && i < nv && pos != INV);
+  if (!m) return;
+  u32 base = 0;
+  if (lane == 0) base = atomicAdd(nlist, (u32)__popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if ((m >> lane) & 1u) list[base + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
 template <u32 VG>
@@ -827,17 +783,28 @@ static bool coarsen_select(Mesh& m, u32* codes, double qual_floor, bool require_
     if (!m.mb->host[4]) return false;
   }
   UpAdj const& ue = m.ask_up(0, 1);
-  sel.cand = dalloc<u32>(nv, s);
+  if (!deferred) sel.cand = dalloc<u32>(nv, s);  // (for the caller)
+  IndsetIn in;
+  in.alloc(nv, s);
+  // (mailbox slot 5, zeroed with 4 to 7 above: the candidates listed)
+  u32* nlist = m.mb->dev + 5;
+  in.nlist = nlist;
   sel.colq = dalloc<double>(nv, s);
   if (nv) {
     u32 const vg = tuned(TK_VERT_GROUP);
     auto k = vg == 4 ? k_collapses_to_verts_grouped<4>
            : vg == 16 ? k_collapses_to_verts_grouped<16> : k_collapses_to_verts_grouped<8>;
     CK(launch_kernel(k, dim3(grid_for((u64)nv * vg)), dim3(BLOCK), 0, s, nv, ue.offs, ue.adj,
-        ue.dirs, codes, sel.q2, sel.cand, sel.colq));
+        ue.dirs, codes, sel.q2, sel.cand, in.keys, sel.colq, in.own_list, nlist,
+        in.out));
     CK_LAUNCH();
   }
-  sel.ind = find_indset(m, 0, sel.cand, sel.colq, !deferred);
+  try {
+    sel.ind = find_indset(m, 0, in, sel.colq, !deferred);
+  } catch (...) {
+    in.free(s);
+    throw;
+  }
   sel.gen_vert = dalloc<u32>(nv, s);
   if (nv) {
     u32 const vg = tuned(TK_VERT_GROUP);

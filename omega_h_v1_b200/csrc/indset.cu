@@ -42,188 +42,451 @@ struct Nbrs {
 // indset_at_vert (indset.cpp:55-84) for entity i: out of the set if a
 // neighbour is in it; in the set if no undecided neighbour beats it (higher
 // goodness, or equal goodness and a lower global id); undecided otherwise.
-// The rounds here update one state array in place and keep a list of the
-// entities still undecided, so a round's work is the undecided entities,
-// not all of them. The set is the same as the reference's synchronous
-// rounds give: states only ever change from undecided to decided, so a
-// state read during a round is either the one of the round before or the
-// final one, and an entity that joins sees every better neighbour decided
-// out -- the lexicographically first independent set in goodness order,
-// whatever the timing. (A state read from the round before only delays a
-// decision to a later round.)
+// Goodness and id order the candidates strictly, so the set is the same
+// whatever the order in which they are decided, as long as each is decided
+// on decided neighbours: the lexicographically first independent set, which
+// the reference's rounds find. So there are no rounds here, and no barrier:
+// a warp keeps the candidates it could not decide, each with its best
+// undecided neighbour (its blocker), and looks at their states until they
+// are decided; an entity that joins the set puts its undecided neighbours
+// out of it. The best undecided candidate can always be decided. (Rounds
+// over lists of the undecided, a grid barrier after each, spent 40 to 60 us
+// a set on a small mesh, most of it in the barriers and in walking every
+// row again: 632 us over a 48^3 adapt and 776 over a 39^3 coarsening, now 290 and 200.)
 //
-// A group of G lanes (G divides 32, so a group never straddles a warp)
-// walks the entity's upward entries l, l + G, ...; each lane folds its
-// neighbours into two flags, and two ballots over the group combine them.
-// (One thread per long row issues loads whose lanes are a row apart and
-// fills the load/store queue.)
+// Words (keys, one per entity): 0 no candidate; an undecided candidate's
+// order_key, by which goodness compares as an integer; or decided, below
+// KEY_MIN (1 + depth: out of the set) or from KEY_IN on (+ depth: in it).
+// One gather tells all of a neighbour, and nothing is written before the
+// walks: the kernels that choose the candidates write their keys. The depth
+// bounds the reference's round for the entity from above: one more than the
+// largest of the better neighbours it joined after (of all its neighbours
+// below DEPTH_EXACT, where the bound is far from the cap), or than that of a
+// neighbour in the set. Where it passes 100 for some entity, the
+// reference's cap of 100 rounds (indset.cpp:33) may have been met, and the
+// last block to finish runs rounds as the reference does, alone.
 //
-// All rounds run in one launch: a cooperative grid (every block resident)
-// sets the states and lists the candidates, then runs round 0 over them and
-// later rounds over the list the round before left, separated by a grid
-// barrier (by a block barrier when block 0 alone takes few candidates),
-// until a round leaves no entity undecided or 100 rounds have run.
-// Control words (zero on entry but [1]: see the prologue): [0] barrier
-// arrivals, [1] barrier generation (only its changes count), [2..4]
-// length of the list round r builds for round r + 1, r + 1 = 0, 1, 2 mod 3
-// (round r zeroes the counter of round r + 2, last read after the barrier
-// of round r - 2 that every block has passed), [5] rounds run, [6] a barrier
-// wait gave up. States and list entries are read past L1 (L1 may keep a
-// line another block has since rewritten; a stale undecided state would
-// only delay the decision, but a line kept stale for good would never let
-// it end, and a stale list entry would name the wrong entity). The
-// barrier's wait is bounded: after COOP_SPIN_LIMIT polls it sets [6] and
-// every block leaves.
-constexpr u32 COOP_SPIN_LIMIT = 1u << 24;
+// A group of G lanes walks a candidate's upward entries l, l + G, ..., and
+// every lane issues the loads of all neighbours of an entry together. (One
+// thread per long row issues loads whose lanes are a row apart and fills
+// the load/store queue; one neighbour at a time waits for three dependent
+// loads each.) Every block must be resident, as warps wait on one another:
+// one thread-block cluster or a cooperative launch. The waits are bounded: a
+// warp that meets no decided state in ASYNC_SPIN_LIMIT sweeps of its
+// candidates sets control word 6 and leaves, and the others leave when they
+// see it.
+constexpr u32 ASYNC_SPIN_LIMIT = 1u << 22;
+constexpr u32 DEPTH_MAX = 127, DEPTH_EXACT = 48;
+typedef unsigned long long Key;
 
-__device__ inline bool coop_barrier(u32* ctl)
+__device__ inline bool key_undecided(Key k) { return k - KEY_MIN < KEY_IN - KEY_MIN; }
+__device__ inline bool key_in(Key k) { return k >= KEY_IN; }
+// (of a decided word)
+__device__ inline u32 key_depth(Key k) { return key_in(k) ? (u32)(k - KEY_IN) : (u32)k - 1u; }
+__device__ inline Key key_decided(u32 depth, bool in)
 {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    u32 const g0 = *(volatile u32*)&ctl[1];
-    __threadfence();
-    if (atomicAdd(&ctl[0], 1u) + 1u == gridDim.x) {
-      *(volatile u32*)&ctl[0] = 0;
-      __threadfence();
-      atomicAdd(&ctl[1], 1u);
-    } else {
-      u32 spins = 0;
-      while (*(volatile u32*)&ctl[1] == g0) {
-        if (++spins > COOP_SPIN_LIMIT) {
-          atomicOr(&ctl[6], 1u);
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return *(volatile u32*)&ctl[6] == 0;
+  return (in ? KEY_IN : (Key)1) + min(depth, DEPTH_MAX);
 }
 
-// (at least 4 blocks per SM: without a minimum the compiler held the
-// kernel to 32 registers and spilled)
-template <int G>
-__global__ void __launch_bounds__(BLOCK, 4) k_indset_coop(u32 n, Nbrs g,
-    u32 const* __restrict__ filter, u32* st, u32* wl0, u32* wl1,
-    double const* __restrict__ good, u64 const* __restrict__ glob, u32* ctl)
+// neighbours of an upward entry: 1 (a vertex's edge), 3 or 6 (an edge's
+// triangle or tet, the edge itself among them); NB: those a lane takes at once
+template <u32 PER>
+struct NbrBatch {
+  static constexpr u32 USES = PER == 1 ? 2 : 1, NB = PER * USES;
+};
+
+// up to NB neighbours of entity i from its entries j, j + G, ... (INV: none)
+template <int G, u32 PER>
+__device__ inline void load_neighbors(Nbrs const& g, u32 i, u32 j, u32 re, u32* o)
 {
-  pdl_wait();
-  u32 const lg = threadIdx.x % G;
-  u32 const gbase = (threadIdx.x & 31) & ~(u32)(G - 1);
-  u32 const gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << gbase;
-  u32 const lane = threadIdx.x & 31;
-  u32 const stride = gridDim.x * blockDim.x;
-  // The states (the filter's candidates undecided, the rest out of the set)
-  // and round 0's list, the candidates, appended a warp at a time to the
-  // list whose length is control word 2 (zero on entry: this kernel zeroes
-  // the list lengths when it settles, the host when a set fails); then the
-  // grid barrier, so round 0 sees every state and the whole list
-  for (u64 b = (u64)blockIdx.x * blockDim.x; b < n; b += stride) {
-    u32 const i = (u32)b + threadIdx.x;
-    bool const c = i < n && (!filter || filter[i]);
-    if (i < n) __stcg(&st[i], c ? (u32)UNKNOWN : (u32)NOT_IN_SET);
-    unsigned const want = __ballot_sync(0xffffffffu, c);
-    if (want) {
-      u32 const leader = __ffs(want) - 1;
-      u32 base = 0;
-      if (lane == leader) base = atomicAdd(&ctl[2], (u32)__popc(want));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (c) wl1[base + __popc(want & ((1u << lane) - 1u))] = i;
+  if (PER == 1) {
+    u32 e[2], d[2];
+#pragma unroll
+    for (u32 k = 0; k < 2; ++k) {
+      bool const on = j + k * G < re;
+      e[k] = on ? g.adj[j + k * G] : INV;
+      d[k] = on ? g.dirs[j + k * G] : 0u;
+    }
+#pragma unroll
+    for (u32 k = 0; k < 2; ++k) o[k] = e[k] != INV ? g.down[(size_t)e[k] * 2 + (1 - d[k])] : INV;
+  } else {
+    u32 const* ds = g.down + (size_t)g.adj[j] * PER;
+#pragma unroll
+    for (u32 k = 0; k < PER; ++k) o[k] = ds[k];
+#pragma unroll
+    for (u32 k = 0; k < PER; ++k)
+      if (o[k] == i) o[k] = INV;
+  }
+}
+
+struct Walk {
+  bool in;       // a neighbour is in the set
+  bool worse;    // some undecided neighbour is worse
+  u32 depth;     // of a neighbour in the set, else the largest of those out of it
+  u32 blocker;   // the best undecided better neighbour, or INV
+};
+
+// The first walk of an entity (FRESH false) reads the words through L1, which
+// neighbouring entities' walks share: a word that has been decided since
+// reads as undecided, which only makes the entity wait. Later ones read past
+// L1, or a stale word would block it for good.
+template <int G, u32 PER, bool FRESH>
+__device__ inline Walk walk_neighbors(Nbrs const& g, u32 i, Key mykey, u32 lg, u32 gmask,
+    u32 gbase, Key const* keys, double const* __restrict__ good, u64 const* __restrict__ glob)
+{
+  constexpr u32 NB = NbrBatch<PER>::NB, STEP = G * NbrBatch<PER>::USES;
+  u32 const rb = g.offs[i], re = g.offs[i + 1];
+  u32 in_depth = 0, out_depth = 0, blocker = INV;
+  Key bk = 0;
+  bool in = false, worse = false;
+  auto id_of = [&](u32 o) { return glob ? glob[o] : (u64)o; };
+  for (u32 j = rb + lg; j < re; j += STEP) {
+    u32 o[NB];
+    Key ko[NB];
+    load_neighbors<G, PER>(g, i, j, re, o);
+#pragma unroll
+    for (u32 k = 0; k < NB; ++k)
+      ko[k] = o[k] == INV ? 0ull : FRESH ? __ldcg(&keys[o[k]]) : __ldca(&keys[o[k]]);
+#pragma unroll
+    for (u32 k = 0; k < NB; ++k) {
+      if (!ko[k]) continue;
+      if (key_undecided(ko[k])) {
+        if (ko[k] < mykey || (ko[k] == mykey && id_of(o[k]) > id_of(i)))
+          worse = true;
+        else if (blocker == INV || ko[k] > bk || (ko[k] == bk && id_of(o[k]) < id_of(blocker))) {
+          blocker = o[k];
+          bk = ko[k];
+        }
+        continue;
+      }
+      u32 const d = key_depth(ko[k]);
+      if (key_in(ko[k])) {
+        in = true;
+        in_depth = d;
+      } else if (d > out_depth) {
+        bool counts = d < DEPTH_EXACT;
+        if (!counts) {
+          double const myg = good[i], og = good[o[k]];
+          counts = (myg == og && id_of(o[k]) < id_of(i)) || myg < og;
+        }
+        if (counts) out_depth = d;
+      }
     }
   }
+  Walk w;
+  u32 const ins = (__ballot_sync(gmask, in) & gmask) >> gbase;
+  w.in = ins != 0;
+  w.worse = (__ballot_sync(gmask, worse) & gmask) != 0;
+#pragma unroll
+  for (int o = G / 2; o; o >>= 1) {
+    out_depth = max(out_depth, __shfl_xor_sync(gmask, out_depth, o));
+    u32 const b2 = __shfl_xor_sync(gmask, blocker, o);
+    Key const k2 = __shfl_xor_sync(gmask, bk, o);
+    if (b2 != INV && b2 != blocker &&
+        (blocker == INV || k2 > bk || (k2 == bk && id_of(b2) < id_of(blocker)))) {
+      blocker = b2;
+      bk = k2;
+    }
+  }
+  u32 const d = __shfl_sync(gmask, in_depth, gbase + (ins ? __ffs(ins) - 1 : 0));
+  w.depth = w.in ? d : out_depth;
+  w.blocker = blocker;
+  return w;
+}
+
+// The reference's rounds, by one block, over lists of the undecided, in
+// place (a state read during a round is the round before's or the final
+// one: states only change from undecided to decided). was: the words of
+// the kernel above (0: no candidate). wl: two lists of n.
+template <int G>
+__device__ void indset_rounds(u32 n, Nbrs const& g, Key const* was, u32* st, u32* wl, double const* __restrict__ good, u64 const* __restrict__ glob, u32* ctl)
+{
+  u32* const wl0 = wl;
+  u32* const wl1 = wl + n;
+  u32 const lg = threadIdx.x % G, lane = threadIdx.x & 31;
+  u32 const gbase = lane & ~(u32)(G - 1);
+  u32 const gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << gbase;
+  for (u64 b = 0; b < n; b += blockDim.x) {
+    u64 const i = b + threadIdx.x;
+    bool const c = i < n && __ldcg(&was[i]) != 0;
+    if (i < n) __stcg(&st[i], c ? (u32)UNKNOWN : (u32)NOT_IN_SET);
+    if (c) __stcg(&wl1[atomicAdd(&ctl[2], 1u)], (u32)i);
+  }
   __threadfence();
-  if (!coop_barrier(ctl)) return;
-  // A short candidate list (two sweeps of one block at most) is left to
-  // block 0, whose rounds are separated by block barriers instead of grid
-  // barriers. Every block decides the same: one reading the length after
-  // block 0 has gone on reads a later list's length or zero, never more.
-  bool const solo = (u64)(*(volatile u32*)&ctl[2]) * G <= 2u * blockDim.x;
-  if (solo && blockIdx.x != 0) return;
-  u32 const rstride = solo ? blockDim.x : stride;
+  __syncthreads();
   for (u32 r = 0; r < MAX_INDSET_ROUNDS; ++r) {
     // round 0 walks the candidates, round r > 0 the list round r - 1 left
     u32 const len = *(volatile u32*)&ctl[2 + r % 3];
     u32 const* list = (r % 2 == 1) ? wl0 : wl1;
     u32* next = (r % 2 == 0) ? wl0 : wl1;
     u32* next_len = &ctl[2 + (r + 1) % 3];
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[2 + (r + 2) % 3] = 0;
-    for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < (u64)len * G; t += rstride) {
-      // past L1, like the states: the lists alternate between two
-      // buffers, so this block may hold lines of this one from two rounds
-      // ago that other blocks have since rewritten
+    if (threadIdx.x == 0) ctl[2 + (r + 2) % 3] = 0;
+    for (u64 t = threadIdx.x; t < (u64)len * G; t += blockDim.x) {
       u32 const i = __ldcg(&list[t / G]);
-      u32 const s0 = __ldcg(&st[i]);
-      bool undecided = false;
-      if (s0 == UNKNOWN) {
-        u32 const rb = g.offs[i], re = g.offs[i + 1];
-        double const myg = good[i];
-        u64 const myid = glob ? glob[i] : (u64)i;
-        bool in_set = false, beaten = false;
-        auto visit = [&](u32 o) {
-          u32 so = __ldcg(&st[o]);
-          if (so == IN_SET) in_set = true;
-          if (so == NOT_IN_SET) return;
-          double og = good[o];
-          u64 oid = glob ? glob[o] : (u64)o;
-          if ((myg == og && oid < myid) || myg < og) beaten = true;
-        };
-        for (u32 j = rb + lg; j < re; j += G) {
-          if (g.mode == 0) {
-            visit(g.down[g.adj[j] * 2 + (1 - g.dirs[j])]);
-          } else {
-            u32 const* ds = g.down + (size_t)g.adj[j] * g.per;
-            for (u32 k = 0; k < g.per; ++k)
-              if (ds[k] != i) visit(ds[k]);
-          }
-        }
-        bool const any_in = (__ballot_sync(gmask, in_set) & gmask) != 0;
-        bool const lost = (__ballot_sync(gmask, beaten) & gmask) != 0;
-        if (lg == 0) {
-          if (any_in)
-            __stcg(&st[i], (u32)NOT_IN_SET);
-          else if (!lost)
-            __stcg(&st[i], (u32)IN_SET);
-          else
-            undecided = true;
+      u32 const rb = g.offs[i], re = g.offs[i + 1];
+      double const myg = good[i];
+      u64 const myid = glob ? glob[i] : (u64)i;
+      bool in_set = false, beaten = false;
+      auto visit = [&](u32 o) {
+        u32 so = __ldcg(&st[o]);
+        if (so == IN_SET) in_set = true;
+        if (so == NOT_IN_SET) return;
+        double og = good[o];
+        u64 oid = glob ? glob[o] : (u64)o;
+        if ((myg == og && oid < myid) || myg < og) beaten = true;
+      };
+      for (u32 j = rb + lg; j < re; j += G) {
+        if (g.mode == 0) {
+          visit(g.down[g.adj[j] * 2 + (1 - g.dirs[j])]);
+        } else {
+          u32 const* ds = g.down + (size_t)g.adj[j] * g.per;
+          for (u32 k = 0; k < g.per; ++k)
+            if (ds[k] != i) visit(ds[k]);
         }
       }
-      // the undecided entities of this pass of the loop, appended to the
-      // next list: one counter update per warp
-      unsigned const act = __activemask();
-      unsigned const want = __ballot_sync(act, undecided);
-      if (want) {
-        u32 const leader = __ffs(want) - 1;
-        u32 base = 0;
-        if (lane == leader) base = atomicAdd(next_len, (u32)__popc(want));
-        base = __shfl_sync(act, base, leader);
-        if (undecided) next[base + __popc(want & ((1u << lane) - 1u))] = i;
-      }
+      bool const any_in = (__ballot_sync(gmask, in_set) & gmask) != 0;
+      bool const lost = (__ballot_sync(gmask, beaten) & gmask) != 0;
+      if (lg) continue;
+      if (any_in)
+        __stcg(&st[i], (u32)NOT_IN_SET);
+      else if (!lost)
+        __stcg(&st[i], (u32)IN_SET);
+      else
+        __stcg(&next[atomicAdd(next_len, 1u)], i);
     }
     __threadfence();
-    if (solo)
-      __syncthreads();
-    else if (!coop_barrier(ctl))
-      return;
+    __syncthreads();
     if (*(volatile u32*)next_len == 0) {
-      // settled: every block still running has passed the last barrier and
-      // reads only next_len (zero) from here, so the list lengths go back to
-      // zero for the next set's prologue
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
+      // settled: the list lengths go back to zero for the next set
+      if (threadIdx.x == 0) {
         ctl[5] = r + 1;
         ctl[2] = ctl[3] = ctl[4] = 0;
       }
       return;
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl[5] = MAX_INDSET_ROUNDS;
+  // not settled: the caller reports it, but its next kernels are queued
+  // already and count on 0 and 1
+  for (u64 i = threadIdx.x; i < n; i += blockDim.x)
+    if (__ldcg(&st[i]) == UNKNOWN) __stcg(&st[i], (u32)NOT_IN_SET);
+  if (threadIdx.x == 0) ctl[5] = MAX_INDSET_ROUNDS;
+}
+
+// Control words, zero on entry but [5]: [0] blocks done, [1] the largest
+// depth, [2..4] list lengths of the rounds, [5] rounds (or the largest
+// depth), [6] a wait gave up. The listed entities (those whose key is not 0
+// are the candidates) are dealt to the lane groups in turn: entry t to group
+// t % all groups, so that candidates that lie together are spread evenly.
+// (Tiles of the entities dealt to warps left most warps idle where the
+// candidates lay together, and every pass read every key.) queue: an entry
+// {entity, blocker} per listed entity, 2 n words at least: the last block's
+// rounds use it as their lists.
+constexpr u32 ITEMS_AHEAD = 4;
+
+// every listed candidate of this warp decided; returns their largest depth
+// (item: 32 words of shared memory of the warp's own)
+template <int G, u32 PER>
+__device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list, u32 nitems,
+    Key* keys, uint2* queue, double const* __restrict__ good, u64 const* __restrict__ glob,
+    u32* __restrict__ out, u32* ctl, u32* item)
+{
+  constexpr u32 FULL = 0xffffffffu, NG = 32 / G;  // groups of a warp
+  u32 const lane = threadIdx.x & 31, lg = lane % G, gi = lane / G;
+  u32 const gbase = lane & ~(u32)(G - 1);
+  u32 const gmask = (G == 32 ? FULL : ((1u << G) - 1u)) << gbase;
+  u32 const below = (1u << lane) - 1u;
+  u32 const nwarps = (gridDim.x * blockDim.x) >> 5;
+  u32 const w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  u32 len = 0, deepest = 0;
+  // entry q of this warp's queue (the places of its list entries, in order)
+  auto slot = [&](u32 q) { return queue + ((size_t)(q / NG) * nwarps + w) * NG + q % NG; };
+  // an entity found decided, or decided, by this thread
+  auto settled = [&](u32 i, Key k) {
+    out[i] = key_in(k) ? 1u : 0u;
+    deepest = max(deepest, key_depth(k));
+  };
+  // entity i walked by a group (key: its key as read by the group): decided,
+  // or its blocker returned
+  auto walk = [&](u32 i, Key mine, bool fresh) -> u32 {
+    if (!key_undecided(mine)) {  // put out of the set meanwhile
+      if (lg == 0) settled(i, mine);
+      return INV;
+    }
+    Walk const r =
+        fresh ? walk_neighbors<G, PER, true>(g, i, mine, lg, gmask, gbase, keys, good, glob)
+              : walk_neighbors<G, PER, false>(g, i, mine, lg, gmask, gbase, keys, good, glob);
+    if (!r.in && r.blocker != INV) return r.blocker;
+    if (lg == 0) {
+      Key const k = key_decided(r.depth + 1, !r.in);
+      __stcg(&keys[i], k);
+      settled(i, k);
+    }
+    if (!r.in && r.worse) {
+      // its neighbours are out of the set
+      Key const no = key_decided(r.depth + 2, false);
+      bool const exact = r.depth + 2 >= DEPTH_EXACT;
+      constexpr u32 NB = NbrBatch<PER>::NB, STEP = G * NbrBatch<PER>::USES;
+      for (u32 j = g.offs[i] + lg, re = g.offs[i + 1]; j < re; j += STEP) {
+        u32 o[NB];
+        load_neighbors<G, PER>(g, i, j, re, o);
+        Key ko[NB];
+#pragma unroll
+        for (u32 k = 0; k < NB; ++k) ko[k] = o[k] != INV ? __ldcg(&keys[o[k]]) : 0ull;
+#pragma unroll
+        for (u32 k = 0; k < NB; ++k) {
+          if (exact && ko[k])  // (the smaller depth stays)
+            atomicMin(&keys[o[k]], no);
+          else if (key_undecided(ko[k]))
+            __stcg(&keys[o[k]], no);
+        }
+      }
+    }
+    return INV;
+  };
+  // entities with blockers (one per group, lane 0 of it) onto the queue
+  auto append = [&](u32 i, u32 blocker) {
+    bool const keep = lg == 0 && blocker != INV;
+    u32 const m = __ballot_sync(FULL, keep);
+    if (keep) *slot(len + __popc(m & below)) = make_uint2(i, blocker);
+    len += __popc(m);
+  };
+  // every candidate once (ITEMS_AHEAD entries' words loaded together)
+  for (u32 q0 = w * NG; q0 < nitems; q0 += nwarps * NG * ITEMS_AHEAD) {
+    u32 it[ITEMS_AHEAD];
+    Key key[ITEMS_AHEAD];
+#pragma unroll
+    for (u32 k = 0; k < ITEMS_AHEAD; ++k) {
+      size_t const t = (size_t)q0 + (size_t)k * nwarps * NG + gi;
+      it[k] = t < nitems ? list[t] : INV;
+    }
+    // (one lane's reading for the group: a word may change between two)
+#pragma unroll
+    for (u32 k = 0; k < ITEMS_AHEAD; ++k)
+      key[k] = lg == 0 && it[k] != INV ? __ldcg(&keys[it[k]]) : 0ull;
+#pragma unroll
+    for (u32 k = 0; k < ITEMS_AHEAD; ++k) {
+      Key const mine = __shfl_sync(FULL, key[k], gbase);
+      if (!__any_sync(FULL, mine != 0)) continue;
+      append(it[k], mine ? walk(it[k], mine, false) : INV);
+    }
+  }
+  // then the undecided, until none is left
+  u32 spins = 0;
+  while (len) {
+    u32 const todo = len;
+    bool moved = false;
+    __syncwarp();  // the entries written by other lanes
+    len = 0;       // entries kept are written at or before the ones being read
+    for (u32 q = 0; q < todo; q += 32) {
+      uint2 e = make_uint2(0u, INV);
+      Key mine = 0, ko = 0;
+      if (q + lane < todo) {
+        e = *slot(q + lane);
+        mine = __ldcg(&keys[e.x]);
+        ko = __ldcg(&keys[e.y]);
+      }
+      bool const have = e.y != INV;
+      bool const put_out = have && !key_undecided(mine);
+      // a decided blocker: in the set, it puts its entity out of it (its own
+      // writes may be on their way); out, the entity is walked again
+      bool const ready = have && !put_out && !key_undecided(ko);
+      bool const again = ready && !key_in(ko);
+      __syncwarp();
+      if (put_out || (ready && !again)) {
+        if (!put_out) {
+          mine = key_decided(key_depth(ko) + 1, false);
+          __stcg(&keys[e.x], mine);
+        }
+        settled(e.x, mine);
+      }
+      bool const wait = have && !put_out && !ready;
+      u32 const kept = __ballot_sync(FULL, wait);
+      if (wait) *slot(len + __popc(kept & below)) = e;
+      len += __popc(kept);
+      moved = moved || __any_sync(FULL, have && !wait);
+      u32 const m = __ballot_sync(FULL, again);
+      if (!m) continue;
+      if (again) item[__popc(m & below)] = e.x;
+      __syncwarp();
+      u32 const cnt = __popc(m);
+      for (u32 b = 0; b < cnt; b += NG) {
+        u32 i = 0, blocker = INV;
+        if (b + gi < cnt) {
+          i = item[b + gi];
+          Key const k = __shfl_sync(gmask, lg == 0 ? __ldcg(&keys[i]) : 0ull, gbase);
+          blocker = walk(i, k, true);
+        }
+        append(i, blocker);
+      }
+      __syncwarp();
+    }
+    if (moved) {
+      spins = 0;
+      continue;
+    }
+    if (++spins > ASYNC_SPIN_LIMIT) {
+      if (lane == 0) atomicOr(&ctl[6], 1u);
+      break;
+    }
+    if ((spins & 255u) == 0 && *(volatile u32*)&ctl[6]) break;
+    __nanosleep(spins < 16 ? 20 : 200);
+  }
+  return __reduce_max_sync(FULL, deepest);
+}
+
+// G: lanes per entity of a long list, where the walks' instructions and
+// loads in flight bound the set; a list with a group of WIDE lanes to every
+// entity is bound by the chain of one walk, which more lanes shorten (edges'
+// rows: 2 lanes 67 us and 8 lanes 222 us on the first list of a 48^3 adapt,
+// 17 and 9 us on a late one).
+constexpr int WIDE = 8;
+
+template <int G, u32 PER>
+__global__ void __launch_bounds__(1024, 1) k_indset(u32 n, Nbrs g,
+    u32 const* __restrict__ list, u32 const* nlist, Key* keys, uint2* queue,
+    double const* __restrict__ good, u64 const* __restrict__ glob, u32* __restrict__ out,
+    u32* ctl)
+{
+  pdl_wait();
+  __shared__ u32 s_item[32][32];
+  __shared__ u32 s_depth;
+  __shared__ u32 s_last;
+  if (threadIdx.x == 0) s_depth = 0;
+  __syncthreads();
+  u32 const nitems = *(u32 const volatile*)nlist;
+  u32* const item = s_item[threadIdx.x >> 5];
+  u32 deepest;
+  if (G < WIDE && (u64)nitems * WIDE <= (u64)gridDim.x * blockDim.x)
+    deepest = decide_listed<(G < WIDE ? WIDE : G), PER>(g, list, nitems, keys, queue, good,
+        glob, out, ctl, item);
+  else
+    deepest = decide_listed<G, PER>(g, list, nitems, keys, queue, good, glob, out, ctl, item);
+  if ((threadIdx.x & 31) == 0 && deepest) atomicMax(&s_depth, deepest);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_depth) atomicMax(&ctl[1], s_depth);
+    __threadfence();
+    s_last = atomicAdd(&ctl[0], 1u) + 1u == gridDim.x ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  u32 const depth = atomicMax(&ctl[1], 0u);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ctl[0] = 0;
+    ctl[1] = 0;
+    ctl[5] = depth;
+  }
+  if (depth <= MAX_INDSET_ROUNDS || *(volatile u32*)&ctl[6]) return;
+  __threadfence();
+  __syncthreads();
+  indset_rounds<G>(n, g, keys, out, reinterpret_cast<u32*>(queue), good, glob, ctl);
 }
 
 namespace {
 // blocks of BLOCK threads a cooperative launch uses on this device: the
 // tuning table's indset_blocks per SM, at most as many as are resident
-template <int G>
+template <int G, u32 PER>
 u32 coop_blocks()
 {
   static std::atomic<u32> per_sm_of[64];
@@ -233,7 +496,7 @@ u32 coop_blocks()
   if (dev < 0 || dev >= 64) return 0;
   if (!sms_of[dev].load()) {
     int per_sm = 0, sms = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_indset_coop<G>, BLOCK, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_indset<G, PER>, BLOCK, 0));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     per_sm_of[dev].store((u32)per_sm);
     sms_of[dev].store((u32)sms);
@@ -243,24 +506,59 @@ u32 coop_blocks()
   return per_sm * sms_of[dev].load();
 }
 
-template <int G>
-void launch_coop(u32 n, Nbrs const& g, u32 const* filter, u32* st, u32* wl,
-    double const* good, u64 const* glob, u32* ctl, cudaStream_t s)
+// A set of at most CLUSTER_ENTS entities goes to one cluster of eight blocks
+// of 1024 threads: an ordinary launch, which need not wait for the whole
+// device to drain as a cooperative one does.
+constexpr u32 CLUSTER_BLOCKS = 8, CLUSTER_ENTS = 8192;
+
+template <int G, u32 PER>
+void launch_indset_as(u32 n, Nbrs const& g, IndsetIn const& in, double const* good,
+    u64 const* glob, u32* ctl, cudaStream_t s)
 {
-  u32 blocks = std::min<u32>(grid_for((u64)n * G), coop_blocks<G>());
-  if (!blocks) throw Failure(E_CUDA, "independent set: no resident blocks");
+  bool const one_cluster = n <= CLUSTER_ENTS;
+  u32 const threads = one_cluster ? 1024 : BLOCK;
+  u32 const most = one_cluster ? CLUSTER_BLOCKS : coop_blocks<G, PER>();
+  if (!most) throw Failure(E_CUDA, "independent set: no resident blocks");
+  // (the list's length is read on the device; n bounds it)
+  u32 const wide = std::max(G, WIDE);
+  u32 const blocks =
+      one_cluster ? CLUSTER_BLOCKS : std::min<u32>(ceil_div((u64)n * wide, threads), most);
+  // a place per listed entity of each group (at either width)
+  u64 const all = (u64)blocks * threads;
+  auto places = [&](u32 lanes) { return (size_t)ceil_div(n, all / lanes) * (all / lanes); };
+  uint2* queue = dalloc<uint2>(std::max(places(G), places(wide)), s);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(BLOCK);
+  cfg.blockDim = dim3(threads);
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CK(cudaLaunchKernelEx(&cfg, k_indset_coop<G>, n, g, filter, st, wl, wl + n, good, glob,
-      ctl));
+  if (one_cluster) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CLUSTER_BLOCKS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
+  CK(cudaLaunchKernelEx(&cfg, k_indset<G, PER>, n, g, in.list, in.nlist, in.keys, queue, good, glob,
+      in.out, ctl));
   CK_LAUNCH();
+  dev_free(queue, s);
+}
+
+template <int G>
+void launch_indset(u32 n, Nbrs const& g, IndsetIn const& in, double const* good,
+    u64 const* glob, u32* ctl, cudaStream_t s)
+{
+  if (g.mode == 0) launch_indset_as<G, 1>(n, g, in, good, glob, ctl, s);
+  else if (g.per == 3) launch_indset_as<G, 3>(n, g, in, good, glob, ctl, s);
+  else launch_indset_as<G, 6>(n, g, in, good, glob, ctl, s);
 }
 }  // namespace
 
@@ -271,7 +569,53 @@ static u32 read_cached_uses(Mesh& m, u32 ent_dim)
   return ent_dim == 0 ? 2u * m.counts[1] : deg(m.dim, 1) * m.counts[m.dim];
 }
 
-u32* find_indset(Mesh& m, u32 ent_dim, u32 const* filter, double const* good, bool check)
+__global__ void __launch_bounds__(BLOCK) k_indset_in(u32 n, u32 const* __restrict__ filter,
+    double const* __restrict__ good, Key* __restrict__ keys, u32* __restrict__ list, u32* nlist,
+    u32* __restrict__ out)
+{
+  pdl_wait();
+  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool const c = i < n && filter[i];
+  if (i < n) {
+    keys[i] = c ? indset_key(good[i]) : 0ull;
+    out[i] = 0;
+  }
+  block_append<1>(c ? 1u : 0u, i, list, nlist);
+}
+
+void IndsetIn::alloc(u32 n, cudaStream_t s)
+{
+  keys = dalloc<Key>(n ? n : 1, s);
+  own_list = dalloc<u32>(n ? n : 1, s);
+  list = own_list;
+  out = dalloc<u32>(n ? n : 1, s);
+}
+
+void IndsetIn::free(cudaStream_t s)
+{
+  dev_free(keys, s);
+  dev_free(own_list, s);
+  dev_free(out, s);
+  keys = nullptr;
+  list = own_list = out = nullptr;
+}
+
+IndsetIn indset_in(Mesh& m, u32 n, u32 const* filter, double const* good)
+{
+  IndsetIn in;
+  in.alloc(n, m.s);
+  u32* nlist = m.mb->dev + COOP_CTL_SLOT + COOP_CTL_WORDS;
+  in.nlist = nlist;
+  CK(cudaMemsetAsync(nlist, 0, sizeof(u32), m.s));
+  if (n) {
+    CK(launch_kernel(k_indset_in, dim3(grid_for(n)), dim3(BLOCK), 0, m.s, n, filter, good,
+        in.keys, in.own_list, nlist, in.out));
+    CK_LAUNCH();
+  }
+  return in;
+}
+
+u32* find_indset(Mesh& m, u32 ent_dim, IndsetIn& in, double const* good, bool check)
 {
   u32 n = m.count(ent_dim);
   Nbrs g{};
@@ -297,10 +641,7 @@ u32* find_indset(Mesh& m, u32 ent_dim, u32 const* filter, double const* good, bo
   // global numbers held as the identity flag are the local index, which is
   // what the kernel compares when it has no array
   u64 const* glob = m.parallel ? m.globals[ent_dim] : nullptr;
-  u32* a = dalloc<u32>(n, m.s);
-  u32* b = dalloc<u32>(2 * (size_t)n, m.s);  // the two lists of undecided entities
-  // One cooperative launch sets the states, lists the candidates and runs
-  // every round, updating a in place; its control words (mailbox slots
+  // One launch decides every candidate; its control words (mailbox slots
   // COOP_CTL_SLOT..) come back with slots 1-3, which a caller that left
   // flags there reads after this call without a read-back of its own. With
   // no entity, only the rounds count is zeroed.
@@ -310,24 +651,21 @@ u32* find_indset(Mesh& m, u32 ent_dim, u32 const* filter, double const* good, bo
     double avg_row = nuse / n;
     u32 lanes = avg_row >= 8.0 ? tuned(TK_INDSET_VERT_GROUP)
               : avg_row >= 3.0 ? tuned(TK_INDSET_EDGE_GROUP) : 1u;
-    if (lanes == 16) launch_coop<16>(n, g, filter, a, b, good, glob, ctl, m.s);
-    else if (lanes == 8) launch_coop<8>(n, g, filter, a, b, good, glob, ctl, m.s);
-    else if (lanes == 4) launch_coop<4>(n, g, filter, a, b, good, glob, ctl, m.s);
-    else if (lanes == 2) launch_coop<2>(n, g, filter, a, b, good, glob, ctl, m.s);
-    else launch_coop<1>(n, g, filter, a, b, good, glob, ctl, m.s);
+    if (lanes == 16) launch_indset<16>(n, g, in, good, glob, ctl, m.s);
+    else if (lanes == 8) launch_indset<8>(n, g, in, good, glob, ctl, m.s);
+    else if (lanes == 4) launch_indset<4>(n, g, in, good, glob, ctl, m.s);
+    else if (lanes == 2) launch_indset<2>(n, g, in, good, glob, ctl, m.s);
+    else launch_indset<1>(n, g, in, good, glob, ctl, m.s);
   } else {
     CK(cudaMemsetAsync(ctl + 5, 0, sizeof(u32), m.s));
   }
-  dev_free(b, m.s);
   if (check) {
     m.mb->fetch(m.s, INDSET_FETCH_SLOTS);
-    try {
-      indset_check(m);
-    } catch (...) {
-      dev_free(a, m.s);
-      throw;
-    }
+    indset_check(m);
   }
+  u32* a = in.out;
+  in.out = nullptr;
+  in.free(m.s);
   return a;
 }
 
@@ -335,18 +673,18 @@ void indset_check(Mesh& m)
 {
   u32 const* hc = m.mb->host + COOP_CTL_SLOT;
   // a set that failed leaves its control words standing: zeroed here for
-  // the next set's prologue, which appends to list length 0
+  // the next set
   auto reset = [&] {
     CK(cudaMemsetAsync(m.mb->dev + COOP_CTL_SLOT, 0, COOP_CTL_WORDS * sizeof(u32), m.s));
   };
   if (hc[6]) {
     reset();
-    throw Failure(E_TIMEOUT, "independent set: a grid barrier wait gave up");
+    throw Failure(E_TIMEOUT, "independent set: a wait for a neighbour gave up");
   }
   u32 rounds = hc[5];
   last_pass_stats().indset_rounds = rounds;
-  // settled: no entity, or the last round left none undecided (the rounds
-  // kernel zeroed the list lengths then)
+  // settled, unless the last block ran rounds and the last of them left some
+  // undecided (the list lengths are zero otherwise)
   bool done = rounds == 0 || hc[2 + rounds % 3] == 0;
   if (!done) {
     reset();

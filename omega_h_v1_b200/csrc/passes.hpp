@@ -24,13 +24,35 @@ __device__ inline double seg_floor(SegView const& v, u32 vert, double f)
 void seg_tally(Mesh& m, u32 ent_dim, u32 const* flags);
 
 // Luby independent set over the star graph of `ent_dim` entities
-// (mesh_find_indset, indset.cpp:119-139). filter and goodness are device
-// arrays; returns a device state array (1 = in set) or throws E_NOCONVERGE.
+// (mesh_find_indset, indset.cpp:119-139). The candidates are listed
+// (*nlist of them, on the device; entities that are none may be listed too);
+// a candidate's key is indset_key of its goodness, any other entity's 0 (only
+// the candidates' goodness is read), and out is zero. Returns out, a device
+// array (1 = in set), and frees the rest of `in`, or throws E_NOCONVERGE.
 // With check = false the outcome is not read back here: the caller fetches
 // at least INDSET_FETCH_SLOTS mailbox slots later (with its own read-back)
 // and calls indset_check, which throws as find_indset would have.
+struct IndsetIn {
+  unsigned long long* keys = nullptr;
+  u32 const* list = nullptr;
+  u32* own_list = nullptr;  // the list, where it is freed with the rest
+  u32 const* nlist = nullptr;
+  u32* out = nullptr;
+  // keys, a list of its own and out for n entities (nlist is the caller's)
+  void alloc(u32 n, cudaStream_t s);
+  void free(cudaStream_t s);
+};
+constexpr unsigned long long KEY_MIN = 256, KEY_IN = ~0ull - 255;
+__device__ inline unsigned long long indset_key(double goodness)
+{
+  // (adding 0.0 makes the two zeros one)
+  unsigned long long const k = order_key(goodness + 0.0);
+  return k < KEY_MIN ? KEY_MIN : k >= KEY_IN ? KEY_IN - 1 : k;
+}
+// the input for the entities a 0 / 1 filter marks (one launch)
+IndsetIn indset_in(Mesh& m, u32 n, u32 const* filter, double const* goodness);
 constexpr u32 INDSET_FETCH_SLOTS = 51;
-u32* find_indset(Mesh& m, u32 ent_dim, u32 const* filter, double const* goodness,
+u32* find_indset(Mesh& m, u32 ent_dim, IndsetIn& in, double const* goodness,
     bool check = true);
 void indset_check(Mesh& m);
 

@@ -13,8 +13,9 @@ namespace osh {
 
 // refine_candidate (refine.cpp:11-15) fused with measure_edge (size.cpp:57)
 // (optional) list, nlist: the candidates appended, a block's in one counter
-// update (nlist zero on entry); zero_q: every edge's goodness zeroed for
-// the quality kernel, which then writes only the listed edges'
+// update (nlist zero on entry); keys, ind: every edge's independent-set key
+// and place in the set zeroed (the quality kernel then writes the kept
+// edges' keys; cand may be null)
 // A block takes EDGE_TILE edges, EDGE_UNROLL to a thread with their loads
 // issued together: the end points' coordinates and sizes are gathers, and
 // the counters (the list's length, the filter's) are words that every block
@@ -26,7 +27,8 @@ constexpr u32 EDGE_UNROLL = 4, EDGE_TILE = EDGE_UNROLL * BLOCK;
 __global__ void __launch_bounds__(BLOCK) k_refine_candidates(u32 ne,
     u32 const* __restrict__ voe, double const* __restrict__ x, double const* __restrict__ h,
     SegView sv, Fp32Stats* fs, u32* __restrict__ cand, u32* any, u32* zero2,
-    u32* __restrict__ list, u32* nlist, double* __restrict__ zero_q)
+    u32* __restrict__ list, u32* nlist, unsigned long long* __restrict__ keys,
+    u32* __restrict__ ind)
 {
   pdl_wait();
   // (optional) two flags the quality kernel that follows sets, zeroed here
@@ -65,8 +67,11 @@ __global__ void __launch_bounds__(BLOCK) k_refine_candidates(u32 ne,
       c = c64;
     }
     c = c && seg_acts(sv, a);
-    cand[i] = c;
-    if (zero_q) zero_q[i] = 0.0;
+    if (cand) cand[i] = c;
+    if (keys) {
+      keys[i] = 0ull;
+      ind[i] = 0;
+    }
     on |= c << k;
   }
   if (fs) fp32_count_block(fs, ndecided, nrechecked, naudited, nflipped);
@@ -102,9 +107,10 @@ __device__ inline void refine_child(u32 dim, u32 const* __restrict__ ve, u32 dir
 //
 // With a list (the candidate kernel's, nlist of them): a grid of the blocks
 // that fit at once strides over the listed edges in block-wide steps (the
-// candidates in order, so each thread draws as many as any other), and the
-// goodness of the other edges was zeroed before. Without one: a thread per
-// edge, its candidacy read from cand.
+// candidates in order, so each thread draws as many as any other), the
+// kept edges' goodness and keys are written, and every other edge's key was
+// zeroed before. Without one: a thread per edge, its candidacy read from
+// cand and taken back there, and every edge's goodness written.
 // F32: with the single-precision filter (fs); without it, its estimates
 // cost the double path no registers.
 template <u32 DIM, bool F32>
@@ -113,7 +119,8 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
     u32 const* __restrict__ voe, u32 const* __restrict__ eo_offs,
     u32 const* __restrict__ eo, u32 const* __restrict__ eo_dirs,
     double const* __restrict__ x, double qual_floor, SegView sv, Fp32Stats* fs,
-    u32* __restrict__ cand, double* __restrict__ out, u32* any, u32* inverted)
+    u32* __restrict__ cand, double* __restrict__ out, unsigned long long* __restrict__ keys,
+    u32* any, u32* inverted)
 {
   pdl_wait();
   constexpr u32 dim = DIM;  // the element dimension (2 or 3): loops over
@@ -211,14 +218,14 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
         }
       }
       if (filtered == 1 || minq < fl) {
-        cand[i] = 0;
+        if (!list) cand[i] = 0;
       } else {
         out[i] = minq;
+        if (list) keys[i] = indset_key(minq);
         keep = 1;
       }
     }
-    // every edge's goodness is written here (with a list: the listed ones)
-    if (t < n && !keep) out[i] = 0.0;
+    if (!list && t < n && !keep) out[i] = 0.0;
     if (F32 && dim == 3) fp32_count_warp(fs, decided, rechecked, audited, flipped);
     if (__any_sync(0xffffffffu, keep) && (threadIdx.x & 31) == 0) raise_flag(any);
   }
@@ -733,15 +740,16 @@ static u32 refine_build(Mesh& m, EdgeSplits const& es, bool deferred, bool unifo
 // deferred (see refine_deferred): the set is returned unchecked, and the
 // build's read-back brings its outcome and the flags
 // zeroed: the candidate kernel already zeroed mailbox slots 1-2
-// list, nlist (optional): the candidates listed by the candidate kernel,
-// which also zeroed q_in (the goodness array this call then owns)
+// in (optional): the candidates listed by the candidate kernel, with zeroed
+// keys and set (this call then owns them, and cand is not looked at)
 static u32* choose_refinement(Mesh& m, u32* cand, double qual_floor, double** quals_out,
-    bool uniform, bool deferred = false, bool zeroed = false, u32 const* list = nullptr,
-    u32 const* nlist = nullptr, double* q_in = nullptr)
+    bool uniform, bool deferred = false, bool zeroed = false, IndsetIn* listed = nullptr)
 {
   cudaStream_t s = m.s;
   u32 ne = m.count(1), dim = m.dim;
-  double* q = q_in ? q_in : dalloc<double>(ne, s);
+  u32 const* list = listed ? listed->list : nullptr;
+  u32 const* nlist = listed ? listed->nlist : nullptr;
+  double* q = dalloc<double>(ne, s);
   if (dim < 2) CK(cudaMemsetAsync(q, 0, sizeof(double) * ne, s));
   u32* any = m.mb->dev + 1;
   u32* inverted = m.mb->dev + 2;
@@ -757,14 +765,11 @@ static u32* choose_refinement(Mesh& m, u32* cand, double qual_floor, double** qu
       auto kq = dim == 2 ? k_refine_quality<2, false>
               : m.fp32_filter ? k_refine_quality<3, true> : k_refine_quality<3, false>;
       u32 grid = grid_for(ne, qb);
-      if (list) {
-        // the listed edges' goodness is written by the kernel, the rest is 0
-        if (!q_in) CK(cudaMemsetAsync(q, 0, sizeof(double) * ne, s));
-        grid = std::min(grid, resident_blocks(kq, qb));
-      }
+      if (list) grid = std::min(grid, resident_blocks(kq, qb));
       CK(launch_kernel(kq, dim3(grid), dim3(qb), 0, s, ne, list, nlist, m.ask_down(1, 0),
           m.ask_down(dim, 0), eo.offs, eo.adj, eo.dirs, m.coords(), qual_floor, m.segview(),
-          m.fp32_filter ? fp32_stats_dev() : nullptr, cand, q, any, inverted));
+          m.fp32_filter ? fp32_stats_dev() : nullptr, cand, q,
+          listed ? listed->keys : nullptr, any, inverted));
       CK_LAUNCH();
     }
   } else {
@@ -774,7 +779,18 @@ static u32* choose_refinement(Mesh& m, u32* cand, double qual_floor, double** qu
   // candidate": with none it settles in its first batch of rounds to the
   // empty set, and its first read-back brings the flags of mailbox slots
   // 1-3 with it (one host wait fewer per pass).
-  u32* ind = ne ? find_indset(m, 1, cand, q, !deferred) : nullptr;
+  u32* ind = nullptr;
+  if (ne) {
+    IndsetIn in = listed ? *listed : indset_in(m, ne, cand, q);
+    if (listed) *listed = IndsetIn();
+    try {
+      ind = find_indset(m, 1, in, q, !deferred);
+    } catch (...) {
+      in.free(s);
+      dev_free(q, s);
+      throw;
+    }
+  }
   if (deferred) {
     if (m.parallel && !m.seg) m.ensure_ghosting(1);
     dev_free(q, s);
@@ -810,8 +826,7 @@ static bool refine_deferred(Mesh& m)
 }
 
 static u32 refine_common(Mesh& m, u32* cand, double qual_floor, bool uniform,
-    bool zeroed = false, u32 const* list = nullptr, u32 const* nlist = nullptr,
-    double* q_in = nullptr)
+    bool zeroed = false, IndsetIn* listed = nullptr)
 {
   cudaStream_t s = m.s;
   PassStats& st = last_pass_stats();
@@ -820,8 +835,7 @@ static u32 refine_common(Mesh& m, u32* cand, double qual_floor, bool uniform,
   st.elems_in = m.count(m.dim);
   u32 ne = m.count(1);
   bool const deferred = refine_deferred(m);
-  u32* ind = choose_refinement(m, cand, qual_floor, nullptr, uniform, deferred, zeroed, list,
-      nlist, q_in);
+  u32* ind = choose_refinement(m, cand, qual_floor, nullptr, uniform, deferred, zeroed, listed);
   if (!ind) return 0;
   seg_tally(m, 1, ind);
   // the split edges' scan, with their list and the surviving edges' maps
@@ -860,33 +874,36 @@ u32 refine_by_size(Mesh& m, double qual_floor)
   u32 ne = m.count(1);
   Tag* h = m.find_tag(0, "adapt_size");
   if (!h) throw Failure(E_ARG, "mesh has no adapt_size vertex field");
-  u32* cand = dalloc<u32>(ne, s);
-  u32* clist = dalloc<u32>(ne ? ne : 1, s);
-  // the edges' goodness, zeroed by the candidate kernel; refine_common's
-  // selection owns it from there
-  double* q = m.dim >= 2 ? dalloc<double>(ne ? ne : 1, s) : nullptr;
+  // triangles and tets: the candidates as a list, their keys written by the
+  // quality kernel; edge meshes: as flags
+  bool const listed = m.dim >= 2 && ne;
+  u32* cand = listed ? nullptr : dalloc<u32>(ne, s);
+  IndsetIn in;
+  if (listed) in.alloc(ne, s);
   // mailbox slot 0: the candidates listed; slot 3: any candidate
   u32* nlist = m.mb->dev + 0;
+  in.nlist = nlist;
   u32* any = m.mb->dev + 3;
   CK(cudaMemsetAsync(nlist, 0, 4 * sizeof(u32), s));  // slots 0-3
   if (ne) {
-    PROBE(P_REFINE_CANDIDATES, s, 8.0 * ne + 32.0 * m.counts[0] + 4.0 * ne);
+    PROBE(P_REFINE_CANDIDATES, s, 8.0 * ne + 32.0 * m.counts[0] + 12.0 * ne);
     CK(launch_kernel(k_refine_candidates, dim3(grid_for(ne, EDGE_TILE)), dim3(BLOCK), 0, s, ne, m.ask_down(1, 0), m.coords(),
         static_cast<double const*>(h->data), m.segview(),
-        m.fp32_filter ? fp32_stats_dev() : nullptr, cand, any, m.mb->dev + 1, clist, nlist, q));
+        m.fp32_filter ? fp32_stats_dev() : nullptr, cand, any, m.mb->dev + 1, in.own_list,
+        nlist, in.keys, in.out));
     CK_LAUNCH();
   }
   // no separate check for "any candidate": with none, the quality kernel
   // keeps none and refine_common returns 0 after its single read-back
   u32 r = 0;
   try {
-    r = refine_common(m, cand, qual_floor, false, ne != 0, clist, nlist, q);
+    r = refine_common(m, cand, qual_floor, false, ne != 0, listed ? &in : nullptr);
   } catch (...) {
-    dev_free(clist, s);
+    in.free(s);
     dev_free(cand, s);
     throw;
   }
-  dev_free(clist, s);
+  in.free(s);
   dev_free(cand, s);
   return r;
 }
@@ -914,7 +931,7 @@ u32 refine_sets(Mesh& m, double qual_floor, u32* cand_out, u32* good_out,
     CK(launch_kernel(k_refine_candidates, dim3(grid_for(ne, EDGE_TILE)), dim3(BLOCK), 0, s, ne, m.ask_down(1, 0), m.coords(),
         static_cast<double const*>(h->data), m.segview(),
         m.fp32_filter ? fp32_stats_dev() : nullptr, cand_out, any, nullptr, nullptr, nullptr,
-        nullptr));
+        nullptr, nullptr));
     CK_LAUNCH();
   }
   CK(cudaMemcpyAsync(good_out, cand_out, sizeof(u32) * ne, cudaMemcpyDeviceToDevice, s));

@@ -235,12 +235,16 @@ void* pinned_scratch();
 // small pinned host mailbox for reading several device scalars at once.
 // Slots, by the step that writes them (steps of one mesh run one at a time,
 // so steps that never overlap share slots):
-//   44-50   independent-set rounds: grid barrier, "anything left" flags,
-//           rounds run, barrier error (one launch runs every round)
-//   1-3     refinement: any good candidate, any inverted child, any candidate
-//   4-7     coarsening selection: any collapse kept (4), codes flag (5, not
-//           read), listed candidates (7); swap selection: interior
-//           candidates (5, not read), any swap kept (6)
+//   44-50   independent set: blocks done, largest depth, list lengths of the
+//           rounds, rounds run (or the largest depth), a wait that gave up
+//           (one launch decides the set); 51: candidates listed for a set
+//           from a filter
+//   0-3     refinement: candidates listed, any good candidate, any inverted
+//           child, any candidate
+//   4-7     coarsening selection: any collapse kept (4), codes flag, then
+//           candidate vertices listed (5, not read), listed edges (7); swap
+//           selection: interior candidates (5, not read), any swap kept (6),
+//           kept edges listed (7, not read)
 //   8-11    refinement build: split entities per domain dimension
 //   16-22   coarsening build: products and survivors per dimension, kept
 //           vertices (22)

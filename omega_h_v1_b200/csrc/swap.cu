@@ -261,8 +261,9 @@ __global__ void k_swap_quality(u32 ne, u32 const* __restrict__ te_offs,
     u32 const* __restrict__ te, u32 const* __restrict__ te_dirs,
     u32 const* __restrict__ voe1, u32 const* __restrict__ vot,
     double const* __restrict__ x, double const* __restrict__ eq, Fp32Stats* fs,
-    u32* __restrict__ cand, double* __restrict__ quals, u32* __restrict__ ring_sizes,
-    u32* __restrict__ codes, u32* any)
+    u32* __restrict__ cand, double* __restrict__ quals,
+    unsigned long long* __restrict__ keys, u32* __restrict__ list, u32* nlist,
+    u32* __restrict__ ind, u32* __restrict__ ring_sizes, u32* __restrict__ codes, u32* any)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -305,6 +306,7 @@ __global__ void k_swap_quality(u32 ne, u32 const* __restrict__ te_offs,
       if (!filtered) choose_edge_swap(rs, ex, rx, perfect_tet_quality(), &code, &q);
       if (!filtered && q > old_minq) {
         quals[i] = q;
+        keys[i] = indset_key(q);
         ring_sizes[i] = rs;
         codes[i] = code;
         keep = 1;
@@ -313,12 +315,24 @@ __global__ void k_swap_quality(u32 ne, u32 const* __restrict__ te_offs,
       }
     }
   }
-  if (i < ne && !keep) {  // every edge's goodness and ring size is written here
+  if (i < ne) ind[i] = 0;
+  if (i < ne && !keep) {  // every edge's goodness, key and ring size is written here
     quals[i] = 0.0;
+    keys[i] = 0ull;
     ring_sizes[i] = 0;
   }
   if (fs) fp32_count_warp(fs, decided, rechecked, audited, flipped);
-  if (__any_sync(0xffffffffu, keep) && (threadIdx.x & 31) == 0) atomicOr(any, 1u);
+  // the kept edges listed for the independent set, a warp's in one update
+  u32 const m = __ballot_sync(0xffffffffu, keep != 0);
+  if (!m) return;
+  u32 const lane = threadIdx.x & 31;
+  u32 base = 0;
+  if (lane == 0) {
+    raise_flag(any);
+    base = atomicAdd(nlist, (u32)__popc(m));
+  }
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (keep) list[base + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
 __device__ inline u32 count_swap_ents(u32 rs, u32 dim)
@@ -445,6 +459,7 @@ __global__ void k_swap_fit(u32 ne, u32 nc, u32 const* __restrict__ gen_offs,
 struct SwapSel {
   u32* cand = nullptr;
   double* quals = nullptr;
+  IndsetIn in;  // the independent set's
   u32* rs = nullptr;
   u32* codes = nullptr;
   u32* ind = nullptr;
@@ -452,6 +467,7 @@ struct SwapSel {
   {
     dev_free(cand, s);
     dev_free(quals, s);
+    in.free(s);
     dev_free(rs, s);
     dev_free(codes, s);
     dev_free(ind, s);
@@ -487,13 +503,16 @@ static bool swap_select(Mesh& m, double gq, u32 nlayers, SwapSel& sel, u32* sliv
   // sliver, or on the boundary) is skipped by the quality kernel, whose
   // "any swap kept" flag (mailbox slot 6) is the one read
   u32* any = m.mb->dev + 6;
-  CK(cudaMemsetAsync(m.mb->dev + 5, 0, 2 * sizeof(u32), s));  // slots 5-6
+  CK(cudaMemsetAsync(m.mb->dev + 5, 0, 3 * sizeof(u32), s));  // slots 5-7
+  u32* nlist = m.mb->dev + 7;  // the kept edges listed
   CK(launch_kernel(k_unmark_boundary, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, m.dim, static_cast<u32 const*>(cd->data),
       sel.cand, m.mb->dev + 5));
   CK_LAUNCH();
   if (interior_out)
     CK(cudaMemcpyAsync(interior_out, sel.cand, sizeof(u32) * ne, cudaMemcpyDeviceToDevice, s));
   sel.quals = dalloc<double>(ne, s);
+  sel.in.alloc(ne, s);
+  sel.in.nlist = nlist;
   sel.rs = dalloc<u32>(ne, s);
   sel.codes = dalloc<u32>(ne, s);
   UpAdj const& te = m.ask_up(1, 3);
@@ -503,10 +522,10 @@ static bool swap_select(Mesh& m, double gq, u32 nlayers, SwapSel& sel, u32* sliv
   u32 const qb = std::min<u32>(tuned(TK_QUALITY_BLOCK), 128u);
   CK(launch_kernel(k_swap_quality, dim3(grid_for(ne, qb)), dim3(qb), 0, s, ne, te.offs, te.adj, te.dirs, m.ask_down(1, 0),
       m.ask_down(3, 0), m.coords(), eq, m.fp32_filter ? fp32_stats_dev() : nullptr, sel.cand,
-      sel.quals, sel.rs, sel.codes, any));
+      sel.quals, sel.in.keys, sel.in.own_list, nlist, sel.in.out, sel.rs, sel.codes, any));
   CK_LAUNCH();
   if (!deferred && !read_u32(any, s)) return false;
-  sel.ind = find_indset(m, 1, sel.cand, sel.quals, !deferred);
+  sel.ind = find_indset(m, 1, sel.in, sel.quals, !deferred);
   return true;
 }
 
