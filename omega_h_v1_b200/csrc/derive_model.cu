@@ -168,7 +168,8 @@ __global__ void k_cc_init(u32 n, u32 const* __restrict__ cd, u32 d, u32* __restr
 }
 
 // entity u and every other entity classified on d that shares with it a
-// side classified on d are in one component
+// side classified on d are in one component (a pair hooked once, by its
+// larger member: each finds the other in the side's row)
 __global__ void k_cc_hook(u32 n, u32 spd, u32 const* __restrict__ sod,
     u32 const* __restrict__ cds, u32 const* __restrict__ offs, u32 const* __restrict__ adj,
     u32 const* __restrict__ cdd, u32 d, u32* parent, u32* fail)
@@ -182,7 +183,7 @@ __global__ void k_cc_hook(u32 n, u32 spd, u32 const* __restrict__ sod,
   if (cds[sd] != d) return;
   for (u32 j = offs[sd]; j < offs[sd + 1]; ++j) {
     u32 o = adj[j];
-    if (o == u || cdd[o] != d) continue;
+    if (o >= u || cdd[o] != d) continue;
     u32 ra = uf_find(parent, u, fail), rb = uf_find(parent, o, fail);
     u32 it = 0;
     while (ra != rb) {

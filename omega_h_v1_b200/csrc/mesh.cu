@@ -867,39 +867,49 @@ __global__ void k_edge_tet_star(u32 n, u32 const* __restrict__ so,
 
 constexpr u32 STAR_BUF = 256;
 
-// get_ent_star_general (star.cpp:14-34); pass 0 counts, pass 1 fills
-__global__ void k_star_general(u32 n, u32 const* __restrict__ hl_offs,
+// get_ent_star_general (star.cpp:14-34); pass 0 counts, pass 1 fills. A warp
+// per entity: its lanes take 32 consecutive lows of its highs at a time,
+// each drops its own if an earlier lane has it (a match over the warp) or
+// if it is among those kept so far, and the rest are kept in lane order,
+// which is the order the reference's loop keeps them in. (A thread per
+// entity searched its list in local memory, some 90 lows against up to 14
+// kept ones one after another: 45 us at any size, 6 now on a small mesh.)
+constexpr u32 STAR_WARPS = BLOCK / 32;
+
+__global__ void __launch_bounds__(BLOCK) k_star_general(u32 n, u32 const* __restrict__ hl_offs,
     u32 const* __restrict__ hl, u32 const* __restrict__ loh, u32 lph,
     u32 const* __restrict__ star_offs, u32* __restrict__ deg_out,
     u32* __restrict__ star, u32* err)
 {
   pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ u32 s_kept[STAR_WARPS][STAR_BUF];
+  u32 const lane = threadIdx.x & 31;
+  u32* const kept = s_kept[threadIdx.x >> 5];
+  u32 const i = (blockIdx.x * BLOCK + threadIdx.x) >> 5;
   if (i >= n) return;
-  u32 buf[STAR_BUF];
+  u32 const f = hl_offs[i], nuse = (hl_offs[i + 1] - f) * lph;
   u32 size = 0;
-  for (u32 j = hl_offs[i]; j < hl_offs[i + 1]; ++j) {
-    u32 h = hl[j];
-    for (u32 k = 0; k < lph; ++k) {
-      u32 sl = loh[h * lph + k];
-      if (sl == i) continue;
-      bool have = false;
-      for (u32 a = 0; a < size; ++a)
-        if (buf[a] == sl) {
-          have = true;
-          break;
-        }
-      if (have) continue;
-      if (size == STAR_BUF) {
-        atomicOr(err, 1u);
-        continue;
-      }
-      buf[size++] = sl;
+  for (u32 b = 0; b < nuse; b += 32) {
+    u32 const c = b + lane;
+    u32 sl = INV;
+    if (c < nuse) sl = loh[(size_t)hl[f + c / lph] * lph + c % lph];
+    u32 const peers = __match_any_sync(0xffffffffu, sl);
+    bool fresh = sl != INV && sl != i && lane == (u32)(__ffs(peers) - 1);
+    for (u32 a = 0; a < size; ++a)
+      if (kept[a] == sl) fresh = false;
+    u32 const m = __ballot_sync(0xffffffffu, fresh);
+    u32 const at = size + __popc(m & ((1u << lane) - 1u));
+    if (fresh && at < STAR_BUF) kept[at] = sl;
+    size += __popc(m);
+    if (size > STAR_BUF) {
+      if (lane == 0) atomicOr(err, 1u);
+      size = STAR_BUF;
     }
+    __syncwarp();
   }
   if (star)
-    for (u32 a = 0; a < size; ++a) star[star_offs[i] + a] = buf[a];
-  else
+    for (u32 a = lane; a < size; a += 32) star[star_offs[i] + a] = kept[a];
+  else if (lane == 0)
     deg_out[i] = size;
 }
 
@@ -924,44 +934,51 @@ __global__ void k_dual_from_sides(u32 ne, u32 spe, u32 const* __restrict__ soe,
   }
 }
 
-__global__ void k_dual_from_verts(u32 dim, u32 ne, u32 const* __restrict__ voe,
+// The other element with a side's vertices: the first one, in the order of
+// the side's first vertex's row, that has them all. A thread per side reads
+// DUAL_BATCH elements of that row, and their vertices, at a time. (Filtering
+// the first row by the others' rows searched those for every element of it:
+// 42 us at any size, 5 now on a small mesh.)
+constexpr u32 DUAL_BATCH = 4;
+
+template <u32 DIM>
+__global__ void k_dual_from_verts(u32 ne, u32 const* __restrict__ voe,
     u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev,
     u32* __restrict__ out, u32* err)
 {
   pdl_wait();
-  u32 spe = deg(dim, dim - 1), vpe = deg(dim, 0), vps = deg(dim - 1, 0);
+  constexpr u32 VPE = DIM + 1, SPE = DIM + 1, VPS = DIM;
   u32 idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= ne * spe) return;
-  u32 i = idx / spe, j = idx % spe;
-  u32 buf[STAR_BUF];
-  u32 n = 0;
-  for (u32 k = 0; k < vps; ++k) {
-    u32 v = voe[(size_t)i * vpe + canon(dim, dim - 1, 0, j, k)];
-    u32 f = ev_offs[v], e = ev_offs[v + 1];
-    if (k) {
-      u32 nn = 0;
-      for (u32 a = 0; a < n; ++a) {
+  if (idx >= ne * SPE) return;
+  u32 const i = idx / SPE, j = idx % SPE;
+  u32 v[VPS];
+#pragma unroll
+  for (u32 k = 0; k < VPS; ++k) v[k] = voe[(size_t)i * VPE + canon(DIM, DIM - 1, 0, j, k)];
+  u32 const f = ev_offs[v[0]], e = ev_offs[v[0] + 1];
+  if (e - f > STAR_BUF + 1) atomicOr(err, 1u);  // (its own row holds element i too)
+  u32 found = INV;
+  for (u32 a = f; a < e && found == INV; a += DUAL_BATCH) {
+    u32 o[DUAL_BATCH], w[DUAL_BATCH][VPE];
+#pragma unroll
+    for (u32 q = 0; q < DUAL_BATCH; ++q) o[q] = a + q < e ? ev[a + q] : i;
+#pragma unroll
+    for (u32 q = 0; q < DUAL_BATCH; ++q)
+#pragma unroll
+      for (u32 k = 0; k < VPE; ++k) w[q][k] = voe[(size_t)o[q] * VPE + k];
+#pragma unroll
+    for (u32 q = 0; q < DUAL_BATCH; ++q) {
+      bool all = true;  // (it has v[0], whose row this is)
+#pragma unroll
+      for (u32 k = 1; k < VPS; ++k) {
         bool has = false;
-        for (u32 b = f; b < e; ++b)
-          if (ev[b] == buf[a]) {
-            has = true;
-            break;
-          }
-        if (has) buf[nn++] = buf[a];
+#pragma unroll
+        for (u32 l = 0; l < VPE; ++l) has = has || w[q][l] == v[k];
+        all = all && has;
       }
-      n = nn;
-    } else {
-      for (u32 a = f; a < e; ++a)
-        if (ev[a] != i) {
-          if (n == STAR_BUF) {
-            atomicOr(err, 1u);
-            break;
-          }
-          buf[n++] = ev[a];
-        }
+      if (found == INV && o[q] != i && all) found = o[q];
     }
   }
-  out[idx] = n ? buf[0] : INV;
+  out[idx] = found;
 }
 
 // bridge graphs (bridge_graph.cpp): degree then fill
@@ -1925,7 +1942,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     u32* err = mb->dev + 60;
     CK(cudaMemsetAsync(err, 0, sizeof(u32), s));
     if (n) {
-      CK(launch_kernel(k_star_general, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, hl.offs, hl.adj, loh, lph,
+      CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.adj, loh, lph,
           nullptr, degree, nullptr, err));
       CK_LAUNCH();
     }
@@ -1934,7 +1951,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     g.nadj = read_u32(g.offs + n, s);
     g.adj = dalloc<u32>(g.nadj, s);
     if (n) {
-      CK(launch_kernel(k_star_general, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, hl.offs, hl.adj, loh, lph, g.offs,
+      CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.adj, loh, lph, g.offs,
           nullptr, g.adj, err));
       CK_LAUNCH();
     }
@@ -1963,7 +1980,8 @@ u32 const* Mesh::ask_dual()
     u32* err = mb->dev + 61;
     CK(cudaMemsetAsync(err, 0, sizeof(u32), s));
     if (nel) {
-      CK(launch_kernel(k_dual_from_verts, dim3(grid_for((u64)nel * spe)), dim3(BLOCK), 0, s, dim, nel, voe, ev.offs,
+      auto k = dim == 3 ? k_dual_from_verts<3> : dim == 2 ? k_dual_from_verts<2> : k_dual_from_verts<1>;
+      CK(launch_kernel(k, dim3(grid_for((u64)nel * spe)), dim3(BLOCK), 0, s, nel, voe, ev.offs,
           ev.adj, out, err));
       CK_LAUNCH();
     }
