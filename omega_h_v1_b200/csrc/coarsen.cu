@@ -99,60 +99,109 @@ struct ExposedSides {
   u32 const* cds;     // class_dim of dimension ed - 1
 };
 
-__device__ inline u32 exposed_sides_code(u32 i, u32 code, u32 const* __restrict__ voe,
-    ExposedSides const& x)
+// the directions of edge i = (v0, v1) that use j of its upward row exposes
+template <u32 ED>
+__device__ inline u32 exposed_by_use(u32 j, u32 v0, u32 v1, ExposedSides const& x)
 {
-  u32 const ed = x.ed, vpt = deg(ed, 0), spt = deg(ed, ed - 1);
-  for (u32 j = x.u_offs[i]; j < x.u_offs[i + 1]; ++j) {
-    u32 t = x.u_adj[j], dir = x.u_dirs[j];
-    u32 tcd = x.cdt[t];
-    for (u32 k = 0; k < 2; ++k) {
-      if (!collapses(code, k)) continue;
-      u32 va = voe[i * 2 + (1 - k)];
-      for (u32 l = 0; l < 2; ++l) {
-        u32 eev = canon(ed, 1, 0, dir, l);
-        if (x.vot[(size_t)t * vpt + eev] == va) {
-          u32 side = x.sot[(size_t)t * spt + opp(ed, 0, eev)];
-          if (x.cds[side] != tcd) code &= ~(1u << k);
-          break;
-        }
-      }
-    }
-  }
-  return code;
+  constexpr u32 VPT = ED + 1, SPT = ED + 1;
+  u32 const t = x.u_adj[j], dir = x.u_dirs[j];
+  u32 const e0 = canon(ED, 1, 0, dir, 0), e1 = canon(ED, 1, 0, dir, 1);
+  u32 const tcd = x.cdt[t];
+  u32 const p0 = x.vot[(size_t)t * VPT + e0], p1 = x.vot[(size_t)t * VPT + e1];
+  // the sides opposite the edge's two places in the entity
+  u32 const c0 = x.cds[x.sot[(size_t)t * SPT + opp(ED, 0, e0)]];
+  u32 const c1 = x.cds[x.sot[(size_t)t * SPT + opp(ED, 0, e1)]];
+  // (direction k: the side opposite the vertex that stays, 1 - k)
+  bool const x0 = p0 == v1 ? c0 != tcd : p1 == v1 && c1 != tcd;
+  bool const x1 = p0 == v0 ? c0 != tcd : p1 == v0 && c1 != tcd;
+  return (x0 ? 1u : 0u) | (x1 ? 2u : 0u);
 }
 
 // The class checks of every edge with a code (the basic check, then the
 // exposed sides for faces, then for elements: nxs of them), the code
 // written back, each edge's collapse qualities zeroed, and the edges still
 // with a code listed (a warp's appends in one counter update): one launch
-// for what were a kernel per check and one for the list
-__global__ void k_coarsen_class_list(u32 ne, u32 const* __restrict__ voe,
+// for what were a kernel per check and one for the list. A thread per edge
+// makes the basic check; the edges that pass it are listed in shared memory
+// and a group of CLASS_GROUP lanes takes each, a lane a use of its faces and
+// of its elements: a use is a chain of four dependent loads, and an edge has
+// some ten. (A thread per edge through both rows: 37 us a launch over a 39^3
+// coarsening, now 16.)
+constexpr u32 CLASS_GROUP = 8;
+
+__global__ void __launch_bounds__(BLOCK) k_coarsen_class_list(u32 ne, u32 const* __restrict__ voe,
     u32 const* __restrict__ cdv, u32 const* __restrict__ cde, ExposedSides xs0,
     ExposedSides xs1, u32 nxs, u32* __restrict__ codes, u32* __restrict__ list, u32* count,
     double2* __restrict__ q2)
 {
   pdl_wait();
+  constexpr u32 FULL = 0xffffffffu;
+  __shared__ u32 s_edge[BLOCK];
+  __shared__ u32 s_code[BLOCK];
+  __shared__ u32 s_n;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  u32 const lane = threadIdx.x & 31, below = (1u << lane) - 1u;
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool on = false;
+  u32 code = DONT_COLLAPSE;
   if (i < ne) {
     q2[i] = make_double2(0.0, 0.0);
-    u32 code = codes[i];
-    if (code != DONT_COLLAPSE) {
-      code = basic_class_code(i, code, voe, cdv, cde);
-      if (code != DONT_COLLAPSE && nxs > 0) code = exposed_sides_code(i, code, voe, xs0);
-      if (code != DONT_COLLAPSE && nxs > 1) code = exposed_sides_code(i, code, voe, xs1);
-      codes[i] = code;
+    u32 const was = codes[i];
+    if (was != DONT_COLLAPSE) {
+      code = basic_class_code(i, was, voe, cdv, cde);
+      if (code == DONT_COLLAPSE) codes[i] = code;
     }
-    on = code != 0;
   }
-  u32 mask = __ballot_sync(0xffffffffu, on);
-  if (!mask) return;
-  u32 lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
-  u32 base = 0;
-  if (lane == leader) base = atomicAdd(count, (u32)__popc(mask));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (on) list[base + __popc(mask & ((1u << lane) - 1u))] = i;
+  u32 m = __ballot_sync(FULL, code != DONT_COLLAPSE);
+  if (m) {
+    u32 base = 0;
+    if (lane == 0) base = atomicAdd(&s_n, (u32)__popc(m));
+    base = __shfl_sync(FULL, base, 0);
+    if (code != DONT_COLLAPSE) {
+      s_edge[base + __popc(m & below)] = i;
+      s_code[base + __popc(m & below)] = code;
+    }
+  }
+  __syncthreads();
+  u32 const n = s_n;
+  u32 const lg = lane % CLASS_GROUP;
+  u32 const gmask = ((1u << CLASS_GROUP) - 1u) << (lane & ~(CLASS_GROUP - 1));
+  // (every warp takes the same number of steps: its lanes vote together)
+  for (u32 b = 0; b < n; b += BLOCK / CLASS_GROUP) {
+    u32 const t = b + threadIdx.x / CLASS_GROUP;
+    bool on = false;
+    u32 e = 0;
+    if (t < n) {
+      e = s_edge[t];
+      u32 const v0 = voe[(size_t)e * 2], v1 = voe[(size_t)e * 2 + 1];
+      u32 out = 0;
+      u32 f0 = 0, n0 = 0, f1 = 0, n1 = 0;
+      if (nxs > 0) {
+        f0 = xs0.u_offs[e];
+        n0 = xs0.u_offs[e + 1] - f0;
+      }
+      if (nxs > 1) {
+        f1 = xs1.u_offs[e];
+        n1 = xs1.u_offs[e + 1] - f1;
+      }
+      for (u32 j = lg; j < max(n0, n1); j += CLASS_GROUP) {
+        if (j < n0) out |= exposed_by_use<2>(f0 + j, v0, v1, xs0);
+        if (j < n1) out |= exposed_by_use<3>(f1 + j, v0, v1, xs1);
+      }
+      out = __reduce_or_sync(gmask, out);
+      u32 const c = s_code[t] & ~out;
+      if (lg == 0) {
+        codes[e] = c;
+        on = c != DONT_COLLAPSE;
+      }
+    }
+    m = __ballot_sync(FULL, on);
+    if (!m) continue;
+    u32 base = 0;
+    if (lane == 0) base = atomicAdd(count, (u32)__popc(m));
+    base = __shfl_sync(FULL, base, 0);
+    if (on) list[base + __popc(m & below)] = e;
+  }
 }
 
 // coarsen_quality (coarsen_qualities.cpp:12-79): worst element of the cavity
