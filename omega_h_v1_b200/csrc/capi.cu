@@ -225,7 +225,7 @@ unsigned const* osh_up(osh_t h, unsigned low, unsigned high)
   API_TRY
   Mesh* m = M(h);
   need(low <= high && high <= m->dim, "bad dimensions");
-  u32 const* r = m->ask_up(low, high).adj;
+  u32 const* r = m->ask_up_apart(low, high).adj;
   sync(m);
   return r;
   API_CATCH(nullptr)
@@ -247,7 +247,7 @@ unsigned const* osh_up_dirs(osh_t h, unsigned low, unsigned high)
   API_TRY
   Mesh* m = M(h);
   need(low <= high && high <= m->dim, "bad dimensions");
-  u32 const* r = m->ask_up(low, high).dirs;
+  u32 const* r = m->ask_up_apart(low, high).dirs;
   sync(m);
   return r;
   API_CATCH(nullptr)

@@ -91,8 +91,7 @@ __device__ inline u32 basic_class_code(u32 i, u32 code, u32 const* __restrict__ 
 struct ExposedSides {
   u32 ed;
   u32 const* u_offs;  // up(1, ed)
-  u32 const* u_adj;
-  u32 const* u_dirs;
+  u32 const* u_uses;
   u32 const* vot;     // down(ed, 0)
   u32 const* sot;     // down(ed, ed - 1)
   u32 const* cdt;     // class_dim of dimension ed
@@ -103,8 +102,8 @@ struct ExposedSides {
 template <u32 ED>
 __device__ inline u32 exposed_by_use(u32 j, u32 v0, u32 v1, ExposedSides const& x)
 {
-  constexpr u32 VPT = ED + 1, SPT = ED + 1;
-  u32 const t = x.u_adj[j], dir = x.u_dirs[j];
+  constexpr u32 VPT = ED + 1, SPT = ED + 1, EPT = deg(ED, 1);
+  u32 const use = x.u_uses[j], t = use / EPT, dir = use % EPT;
   u32 const e0 = canon(ED, 1, 0, dir, 0), e1 = canon(ED, 1, 0, dir, 1);
   u32 const tcd = x.cdt[t];
   u32 const p0 = x.vot[(size_t)t * VPT + e0], p1 = x.vot[(size_t)t * VPT + e1];
@@ -249,7 +248,7 @@ template <u32 DIM, bool F32>
 __global__ void k_coarsen_quality(u32 const* __restrict__ list,
     u32 const* __restrict__ nlist, u32 const* __restrict__ voe1, u32 const* __restrict__ voe,
     u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev,
-    u32 const* __restrict__ ev_dirs, double const* __restrict__ x,
+    double const* __restrict__ x,
     double const* __restrict__ eq, double floor_q, SegView sv, Fp32Stats* fs,
     u32* __restrict__ codes, double* __restrict__ out, u32* any)
 {
@@ -277,7 +276,7 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
       load3(x, gen, ex[vpe - 1]);
       FirstMin om{1.0, 0};
       if (eq)
-        for (u32 k = f + lane; k < e; k += 32) first_min_add(om, eq[ev[k]], k - f + 1);
+        for (u32 k = f + lane; k < e; k += 32) first_min_add(om, eq[ev[k] / vpe], k - f + 1);
       double old_minq = warp_first_min(om);
       // with the filter: the cavity's estimates first; the direction is
       // rejected on them when the worst element is surely below the floor or
@@ -292,11 +291,12 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
         all = (e - f) > 64 * 32;
         u32 c = 0;
         for (u32 k = f + lane; k < e; k += 32, ++c) {
-          u32 const* ve = voe + (size_t)ev[k] * vpe;
+          u32 const use = ev[k];
+          u32 const* ve = voe + (size_t)(use / vpe) * vpe;
           bool adjacent = false;
           for (u32 l = 0; l < vpe; ++l) adjacent = adjacent || ve[l] == gen;
           if (adjacent) continue;
-          u32 base = opp(dim, 0, ev_dirs[k]);
+          u32 base = opp(dim, 0, use % vpe);
           for (u32 l = 0; l + 1 < vpe; ++l) load3(x, ve[canon(dim, dim - 1, 0, base, l)], ex[l]);
           Q32 q = tet_quality_f32(ex, k6);
           upper = fminf(upper, q32_hi(q));
@@ -316,11 +316,12 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
         u32 c = 0;
         for (u32 k = f + lane; k < e; k += 32, ++c) {
           if (filtered && !all && !((need >> c) & 1ull)) continue;
-          u32 const* ve = voe + (size_t)ev[k] * vpe;
+          u32 const use = ev[k];
+          u32 const* ve = voe + (size_t)(use / vpe) * vpe;
           bool adjacent = false;
           for (u32 l = 0; l < vpe; ++l) adjacent = adjacent || ve[l] == gen;
           if (adjacent) continue;
-          u32 base = opp(dim, 0, ev_dirs[k]);
+          u32 base = opp(dim, 0, use % vpe);
           for (u32 l = 0; l + 1 < vpe; ++l) load3(x, ve[canon(dim, dim - 1, 0, base, l)], ex[l]);
           double q = dim == 3 ? tet_quality(ex, perfect) : tri_quality(ex, 1, perfect);
           if (use32 && filtered && fs->audit) fp32_note_error(fs, tet_quality_f32(ex, k6), q);
@@ -334,11 +335,12 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
         // estimate against its double value
         FirstMin m64{1.0, 0};
         for (u32 k = f + lane; k < e; k += 32) {
-          u32 const* ve = voe + (size_t)ev[k] * vpe;
+          u32 const use = ev[k];
+          u32 const* ve = voe + (size_t)(use / vpe) * vpe;
           bool adjacent = false;
           for (u32 l = 0; l < vpe; ++l) adjacent = adjacent || ve[l] == gen;
           if (adjacent) continue;
-          u32 base = opp(dim, 0, ev_dirs[k]);
+          u32 base = opp(dim, 0, use % vpe);
           for (u32 l = 0; l + 1 < vpe; ++l) load3(x, ve[canon(dim, dim - 1, 0, base, l)], ex[l]);
           double q = tet_quality(ex, perfect);
           fp32_note_error(fs, tet_quality_f32(ex, k6), q);
@@ -380,7 +382,7 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
 
 template <u32 VG>
 __global__ void k_collapses_to_verts_grouped(u32 nv, u32 const* __restrict__ ue_offs,
-    u32 const* __restrict__ ue, u32 const* __restrict__ ue_dirs,
+    u32 const* __restrict__ ue,
     u32 const* __restrict__ codes, double const* __restrict__ q2, u32* __restrict__ cand,
     unsigned long long* __restrict__ keys, double* __restrict__ colq, u32* __restrict__ list,
     u32* nlist, u32* __restrict__ ind)
@@ -394,9 +396,9 @@ __global__ void k_collapses_to_verts_grouped(u32 nv, u32 const* __restrict__ ue_
   u32 pos = INV;  // position of the lane's best entry; INV: no collapse seen
   u32 const rb = i < nv ? ue_offs[i] : 0u, re = i < nv ? ue_offs[i + 1] : 0u;
   for (u32 j = rb + lg; j < re; j += VG) {
-    u32 e = ue[j], d = ue_dirs[j];
-    if (!collapses(codes[e], d)) continue;
-    double q = q2[e * 2 + d];
+    u32 const u = ue[j];  // edge * 2 + the vertex's place in it
+    if (!collapses(codes[u >> 1], u & 1u)) continue;
+    double q = q2[u];
     if (pos == INV || q > maxq) {
       maxq = q;
       pos = j;
@@ -428,7 +430,7 @@ __global__ void k_collapses_to_verts_grouped(u32 nv, u32 const* __restrict__ ue_
 
 template <u32 VG>
 __global__ void k_vertex_dest_grouped(u32 nv, u32 const* __restrict__ ue_offs,
-    u32 const* __restrict__ ue, u32 const* __restrict__ ue_dirs,
+    u32 const* __restrict__ ue,
     u32 const* __restrict__ voe1, u32 const* __restrict__ ind,
     double const* __restrict__ colq, u32 const* __restrict__ codes,
     double const* __restrict__ q2, u32* __restrict__ gen_vert)
@@ -447,9 +449,9 @@ __global__ void k_vertex_dest_grouped(u32 nv, u32 const* __restrict__ ue_offs,
   if (maxq == 1e10) maxq = -1e10;
   u32 first = INV;
   for (u32 j = ue_offs[i] + lg; j < ue_offs[i + 1]; j += VG) {
-    u32 e = ue[j], d = ue_dirs[j];
-    if (!collapses(codes[e], d)) continue;
-    double q = q2[e * 2 + d];
+    u32 const u = ue[j];
+    if (!collapses(codes[u >> 1], u & 1u)) continue;
+    double q = q2[u];
     if (q == 1e10) q = -1e10;
     if (q == maxq) {
       first = j;
@@ -459,7 +461,7 @@ __global__ void k_vertex_dest_grouped(u32 nv, u32 const* __restrict__ ue_offs,
   for (u32 o = VG / 2; o; o >>= 1) first = min(first, __shfl_xor_sync(gmask, first, o));
   if (lg == 0) {
     u32 g = INV;
-    if (first != INV) g = voe1[ue[first] * 2 + (1 - ue_dirs[first])];
+    if (first != INV) g = voe1[ue[first] ^ 1u];  // the edge's other end
     gen_vert[i] = g;
   }
 }
@@ -556,7 +558,7 @@ __global__ void k_same_conn(u32 n, u32 const* __restrict__ voe, u32 const* __res
 // coarsen_conserve_cavity (coarsen_conserve.cpp:15-55)
 __global__ void k_coarsen_conserve(u32 nv, u32 nc, u32 nsame,
     u32 const* __restrict__ gen_offs_v, u32 const* __restrict__ gen_offs_e,
-    u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev,
+    u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev, UseDiv div,
     double const* __restrict__ in, double const* __restrict__ sizes,
     double* __restrict__ gen)
 {
@@ -567,15 +569,15 @@ __global__ void k_coarsen_conserve(u32 nv, u32 nc, u32 nsame,
   double sum[MAX_NCOMPS];
   for (u32 c = 0; c < nc; ++c) sum[c] = 0;
   for (u32 j = f; j < e; ++j)
-    for (u32 c = 0; c < nc; ++c) sum[c] = sum[c] + in[(size_t)ev[j] * nc + c];
+    for (u32 c = 0; c < nc; ++c) sum[c] = sum[c] + in[(size_t)use_high(div, ev[j]) * nc + c];
   double cav = 0;
   for (u32 j = f; j < e; ++j) {
-    u32 el = ev[j];
+    u32 el = use_high(div, ev[j]);
     if (gen_offs_e[el] == gen_offs_e[el + 1]) continue;
     cav += sizes[gen_offs_e[el] + nsame];
   }
   for (u32 j = f; j < e; ++j) {
-    u32 el = ev[j];
+    u32 el = use_high(div, ev[j]);
     if (gen_offs_e[el] == gen_offs_e[el + 1]) continue;
     u32 ge = gen_offs_e[el];
     double sc = sizes[ge + nsame] / cav;
@@ -642,7 +644,7 @@ __device__ void qr_solve2(double (*q)[MAX_PTS], double (*r)[4], double const* b,
 
 __global__ void k_coarsen_fit(u32 nv, u32 nc, u32 nsame, u32 const* __restrict__ gen_offs_v,
     u32 const* __restrict__ gen_offs_e, u32 const* __restrict__ ev_offs,
-    u32 const* __restrict__ ev, double const* __restrict__ oldx,
+    u32 const* __restrict__ ev, UseDiv div, double const* __restrict__ oldx,
     double const* __restrict__ newx, double const* __restrict__ in,
     double* __restrict__ gen)
 {
@@ -658,7 +660,7 @@ __global__ void k_coarsen_fit(u32 nv, u32 nc, u32 nsame, u32 const* __restrict__
   if (fit) {
     double a[MAX_PTS][4];
     for (u32 j = 0; j < npts; ++j) {
-      u32 oe = ev[f + j];
+      u32 oe = use_high(div, ev[f + j]);
       a[j][0] = 1.0;
       a[j][1] = oldx[oe * 3 + 0];
       a[j][2] = oldx[oe * 3 + 1];
@@ -669,15 +671,15 @@ __global__ void k_coarsen_fit(u32 nv, u32 nc, u32 nsame, u32 const* __restrict__
   for (u32 j = 0; j < nc; ++j) {
     double b[MAX_PTS], c[4], avg = 0;
     if (fit) {
-      for (u32 k = 0; k < npts; ++k) b[k] = in[(size_t)ev[f + k] * nc + j];
+      for (u32 k = 0; k < npts; ++k) b[k] = in[(size_t)use_high(div, ev[f + k]) * nc + j];
       qr_solve2(q, r, b, npts, c);
     } else {
       avg = 0;
-      for (u32 k = f; k < e; ++k) avg += in[(size_t)ev[k] * nc + j];
+      for (u32 k = f; k < e; ++k) avg += in[(size_t)use_high(div, ev[k]) * nc + j];
       avg /= (e - f);
     }
     for (u32 k = f; k < e; ++k) {
-      u32 oe = ev[k];
+      u32 oe = use_high(div, ev[k]);
       if (gen_offs_e[oe] == gen_offs_e[oe + 1]) continue;
       u32 ge = gen_offs_e[oe];
       if (fit) {
@@ -715,7 +717,7 @@ static void coarsen_transfer(Mesh& m, Mesh& out, u32 const* gen_offs_v,
       expand_scaled(t.data, same_e, 1, ne, nc, 8, data, s);
       if (nv) {
         CK(launch_kernel(k_coarsen_conserve, dim3(grid_for(nv)), dim3(BLOCK), 0, s, nv, nc, nsame, gen_offs_v,
-            gen_offs_e, ev.offs, ev.adj, static_cast<double const*>(t.data), sizes,
+            gen_offs_e, ev.offs, ev.uses, use_div(deg(dim, 0)), static_cast<double const*>(t.data), sizes,
             data + (size_t)nsame * nc));
         CK_LAUNCH();
       }
@@ -735,7 +737,7 @@ static void coarsen_transfer(Mesh& m, Mesh& out, u32 const* gen_offs_v,
     expand_scaled(t.data, same_e, 1, ne, nc, 8, data, s);
     if (nv) {
       CK(launch_kernel(k_coarsen_fit, dim3(ceil_div(nv, 128)), dim3(128), 0, s, nv, nc, nsame, gen_offs_v, gen_offs_e,
-          ev.offs, ev.adj, oldx, newx, static_cast<double const*>(t.data),
+          ev.offs, ev.uses, use_div(deg(dim, 0)), oldx, newx, static_cast<double const*>(t.data),
           data + (size_t)nsame * nc));
       CK_LAUNCH();
     }
@@ -780,7 +782,7 @@ static bool coarsen_select(Mesh& m, u32* codes, double qual_floor, bool require_
     Tag* cdt = m.find_tag(ed, "class_dim");
     Tag* cds = m.find_tag(ed - 1, "class_dim");
     if (!cdt || !cds) throw Failure(E_ARG, "coarsening needs class_dim on every dimension");
-    xs[nxs++] = ExposedSides{ed, u.offs, u.adj, u.dirs, m.ask_down(ed, 0),
+    xs[nxs++] = ExposedSides{ed, u.offs, u.uses, m.ask_down(ed, 0),
         m.ask_down(ed, ed - 1), static_cast<u32 const*>(cdt->data),
         static_cast<u32 const*>(cds->data)};
   }
@@ -815,7 +817,7 @@ static bool coarsen_select(Mesh& m, u32* codes, double qual_floor, bool require_
             : m.fp32_filter ? k_coarsen_quality<3, true> : k_coarsen_quality<3, false>;
     CK(launch_kernel(kq, dim3(blocks),
         dim3(qb), 0, s, clist, ncand, voe1, m.ask_down(dim, 0),
-        ev.offs, ev.adj, ev.dirs, m.coords(), eq, qual_floor, m.segview(),
+        ev.offs, ev.uses, m.coords(), eq, qual_floor, m.segview(),
         m.fp32_filter ? fp32_stats_dev() : nullptr, codes, sel.q2, any));
     CK_LAUNCH();
   }
@@ -843,8 +845,8 @@ static bool coarsen_select(Mesh& m, u32* codes, double qual_floor, bool require_
     u32 const vg = tuned(TK_VERT_GROUP);
     auto k = vg == 4 ? k_collapses_to_verts_grouped<4>
            : vg == 16 ? k_collapses_to_verts_grouped<16> : k_collapses_to_verts_grouped<8>;
-    CK(launch_kernel(k, dim3(grid_for((u64)nv * vg)), dim3(BLOCK), 0, s, nv, ue.offs, ue.adj,
-        ue.dirs, codes, sel.q2, sel.cand, in.keys, sel.colq, in.own_list, nlist,
+    CK(launch_kernel(k, dim3(grid_for((u64)nv * vg)), dim3(BLOCK), 0, s, nv, ue.offs, ue.uses,
+        codes, sel.q2, sel.cand, in.keys, sel.colq, in.own_list, nlist,
         in.out));
     CK_LAUNCH();
   }
@@ -859,8 +861,8 @@ static bool coarsen_select(Mesh& m, u32* codes, double qual_floor, bool require_
     u32 const vg = tuned(TK_VERT_GROUP);
     auto k = vg == 4 ? k_vertex_dest_grouped<4>
            : vg == 16 ? k_vertex_dest_grouped<16> : k_vertex_dest_grouped<8>;
-    CK(launch_kernel(k, dim3(grid_for((u64)nv * vg)), dim3(BLOCK), 0, s, nv, ue.offs, ue.adj,
-        ue.dirs, voe1, sel.ind, sel.colq, codes, sel.q2, sel.gen_vert));
+    CK(launch_kernel(k, dim3(grid_for((u64)nv * vg)), dim3(BLOCK), 0, s, nv, ue.offs, ue.uses,
+        voe1, sel.ind, sel.colq, codes, sel.q2, sel.gen_vert));
     CK_LAUNCH();
   }
   return true;

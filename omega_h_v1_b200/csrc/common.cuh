@@ -184,6 +184,30 @@ __host__ __device__ inline u32 opp(u32 elem, u32 dim, u32 j)
   return (0x1023u >> (4 * j)) & 0xfu;                   // {3,2,0,1}
 }
 
+// A use -- an upward adjacency's entry -- is one word: high * lph + dir, the
+// place of the low entity in down(high, low) with lph lows to a high. UseDiv
+// takes it apart where lph is known at run time only (a multiply and a shift
+// for 2, 3, 4 and 6).
+struct UseDiv {
+  u32 lph, mul, sh;
+};
+
+inline UseDiv use_div(u32 lph)
+{
+  switch (lph) {
+    case 2: return {2, 0x80000000u, 0};
+    case 3: return {3, 0xaaaaaaabu, 1};
+    case 4: return {4, 0x40000000u, 0};
+    case 6: return {6, 0xaaaaaaabu, 2};
+    default: return {1, 0, 0};
+  }
+}
+
+__device__ __forceinline__ u32 use_high(UseDiv d, u32 use)
+{
+  return d.lph == 1 ? use : __umulhi(use, d.mul) >> d.sh;
+}
+
 // ---------------------------------------------------------------------------
 // geometry (size.hpp, quality.hpp, algebra.hpp)
 

@@ -72,8 +72,8 @@ __global__ void k_side_normals(u32 ns, u32 D, u32 const* __restrict__ vos,
 // hinges (derive_model.cpp:78-138): on the boundary if any adjacent side is;
 // the crease angle is between the first two boundary sides in row order (a
 // missing second side reads side 0, as the reference's zeroed pair does)
-__global__ void k_hinge_class(u32 nh, u32 const* __restrict__ offs, u32 const* __restrict__ adj,
-    u32 const* __restrict__ bside, double const* __restrict__ nrm, double cos_lo,
+__global__ void k_hinge_class(u32 nh, u32 const* __restrict__ offs,
+    u32 const* __restrict__ uses, UseDiv div, u32 const* __restrict__ bside, double const* __restrict__ nrm, double cos_lo,
     double cos_hi, u32* __restrict__ bh, u32* __restrict__ crease, double* __restrict__ dots,
     u32* __restrict__ namb, u32* __restrict__ amb)
 {
@@ -81,8 +81,10 @@ __global__ void k_hinge_class(u32 nh, u32 const* __restrict__ offs, u32 const* _
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nh) return;
   u32 a[2] = {0, 0}, na = 0;
-  for (u32 j = offs[i]; j < offs[i + 1]; ++j)
-    if (bside[adj[j]] && na < 2) a[na++] = adj[j];
+  for (u32 j = offs[i]; j < offs[i + 1]; ++j) {
+    u32 const sd = use_high(div, uses[j]);
+    if (bside[sd] && na < 2) a[na++] = sd;
+  }
   u32 b = na > 0 ? 1u : 0u, c = 0;
   if (b) {
     double d = dot3(nrm + (size_t)a[0] * 3, nrm + (size_t)a[1] * 3);
@@ -117,7 +119,7 @@ __global__ void k_hinge_cd(u32 nh, u32 D, u32 const* __restrict__ bh,
 
 // 3D vertices (derive_model.cpp:140-216): the lowest class_dim of their
 // edges, one lower again at a corner of more than two crease edges
-__global__ void k_vertex_class(u32 nv, u32 const* __restrict__ offs, u32 const* __restrict__ adj,
+__global__ void k_vertex_class(u32 nv, u32 const* __restrict__ offs, u32 const* __restrict__ uses,
     u32 const* __restrict__ crease, u32 const* __restrict__ hcd, u32* __restrict__ vcd)
 {
   pdl_wait();
@@ -125,7 +127,7 @@ __global__ void k_vertex_class(u32 nv, u32 const* __restrict__ offs, u32 const* 
   if (i >= nv) return;
   u32 nin = 0, d = 3;
   for (u32 j = offs[i]; j < offs[i + 1]; ++j) {
-    u32 e = adj[j];
+    u32 e = uses[j] / 2;
     if (crease[e]) ++nin;
     if (hcd[e] < d) d = hcd[e];
   }
@@ -171,8 +173,8 @@ __global__ void k_cc_init(u32 n, u32 const* __restrict__ cd, u32 d, u32* __restr
 // side classified on d are in one component (a pair hooked once, by its
 // larger member: each finds the other in the side's row)
 __global__ void k_cc_hook(u32 n, u32 spd, u32 const* __restrict__ sod,
-    u32 const* __restrict__ cds, u32 const* __restrict__ offs, u32 const* __restrict__ adj,
-    u32 const* __restrict__ cdd, u32 d, u32* parent, u32* fail)
+    u32 const* __restrict__ cds, u32 const* __restrict__ offs, u32 const* __restrict__ uses,
+    UseDiv div, u32 const* __restrict__ cdd, u32 d, u32* parent, u32* fail)
 {
   pdl_wait();
   u32 t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -182,7 +184,7 @@ __global__ void k_cc_hook(u32 n, u32 spd, u32 const* __restrict__ sod,
   u32 sd = sod[t];
   if (cds[sd] != d) return;
   for (u32 j = offs[sd]; j < offs[sd + 1]; ++j) {
-    u32 o = adj[j];
+    u32 o = use_high(div, uses[j]);
     if (o >= u || cdd[o] != d) continue;
     u32 ra = uf_find(parent, u, fail), rb = uf_find(parent, o, fail);
     u32 it = 0;
@@ -231,16 +233,18 @@ __global__ void k_cc_ids(u32 n, u32 const* __restrict__ parent, u32 const* __res
 
 // project_class_id_onto (derive_model.cpp:392-412): the last upward entity
 // (row order) with the same class_dim gives its class_id
-__global__ void k_project_ids(u32 n, u32 const* __restrict__ offs, u32 const* __restrict__ adj,
-    u32 const* __restrict__ cd_hi, u32 const* __restrict__ cid_hi,
+__global__ void k_project_ids(u32 n, u32 const* __restrict__ offs, u32 const* __restrict__ uses,
+    UseDiv div, u32 const* __restrict__ cd_hi, u32 const* __restrict__ cid_hi,
     u32 const* __restrict__ cd_lo, u32* __restrict__ cid_lo)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   u32 c = cd_lo[i], id = cid_lo[i];
-  for (u32 j = offs[i]; j < offs[i + 1]; ++j)
-    if (cd_hi[adj[j]] == c) id = cid_hi[adj[j]];
+  for (u32 j = offs[i]; j < offs[i + 1]; ++j) {
+    u32 const h = use_high(div, uses[j]);
+    if (cd_hi[h] == c) id = cid_hi[h];
+  }
   cid_lo[i] = id;
 }
 
@@ -283,7 +287,7 @@ void Mesh::derive_model(double crease_angle)
   CK(cudaMemsetAsync(namb, 0, sizeof(u32), s));
   double cc = std::cos(crease_angle);
   if (nh) {
-    CK(launch_kernel(k_hinge_class, dim3(grid_for(nh)), dim3(BLOCK), 0, s, nh, sh.offs, sh.adj, bside, nrm, cc - 1e-9,
+    CK(launch_kernel(k_hinge_class, dim3(grid_for(nh)), dim3(BLOCK), 0, s, nh, sh.offs, sh.uses, use_div(deg(D - 1, D - 2)), bside, nrm, cc - 1e-9,
         cc + 1e-9, bh, crease, dots, namb, amb));
     CK_LAUNCH();
   }
@@ -324,7 +328,7 @@ void Mesh::derive_model(double crease_angle)
     UpAdj const& ev = ask_up(0, 1, false);
     cd[0] = dalloc<u32>(nv, s);
     if (nv) {
-      CK(launch_kernel(k_vertex_class, dim3(grid_for(nv)), dim3(BLOCK), 0, s, nv, ev.offs, ev.adj, crease, cd[D - 2],
+      CK(launch_kernel(k_vertex_class, dim3(grid_for(nv)), dim3(BLOCK), 0, s, nv, ev.offs, ev.uses, crease, cd[D - 2],
           cd[0]));
       CK_LAUNCH();
     }
@@ -363,7 +367,7 @@ void Mesh::derive_model(double crease_angle)
       CK(launch_kernel(k_cc_init, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, cd[d], d, cid[d]));
       CK_LAUNCH();
       CK(launch_kernel(k_cc_hook, dim3(grid_for((u64)n * spd)), dim3(BLOCK), 0, s, n, spd, sod, cd[d - 1], dos.offs,
-          dos.adj, cd[d], d, cid[d], fail));
+          dos.uses, use_div(spd), cd[d], d, cid[d], fail));
       CK_LAUNCH();
       CK(launch_kernel(k_cc_flatten, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, cid[d], roots, fail));
       CK_LAUNCH();
@@ -385,7 +389,7 @@ void Mesh::derive_model(double crease_angle)
     u32 d = D - dd, nl = count(d);
     UpAdj const& u = ask_up(d, d + 1, true);
     if (nl) {
-      CK(launch_kernel(k_project_ids, dim3(grid_for(nl)), dim3(BLOCK), 0, s, nl, u.offs, u.adj, cd[d + 1], cid[d + 1],
+      CK(launch_kernel(k_project_ids, dim3(grid_for(nl)), dim3(BLOCK), 0, s, nl, u.offs, u.uses, use_div(deg(d + 1, d)), cd[d + 1], cid[d + 1],
           cd[d], cid[d]));
       CK_LAUNCH();
     }

@@ -157,7 +157,7 @@ __global__ void k_element_gradients_any(u32 dim, u32 ne, u32 const* __restrict__
 constexpr u32 RECOVER_BATCH = 4;
 
 __global__ void __launch_bounds__(BLOCK) k_recover_by_volume(u32 nv, u32 const* __restrict__ offs,
-    u32 const* __restrict__ adj, double const* __restrict__ sizes, u32 nc,
+    u32 const* __restrict__ uses, UseDiv div, double const* __restrict__ sizes, u32 nc,
     double const* __restrict__ f, double* __restrict__ out)
 {
   pdl_wait();
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(BLOCK) k_recover_by_volume(u32 nv, u32 const* 
     u32 e[RECOVER_BATCH];
     double es[RECOVER_BATCH], fe[RECOVER_BATCH];
 #pragma unroll
-    for (u32 k = 0; k < RECOVER_BATCH; ++k) e[k] = adj[j + k];
+    for (u32 k = 0; k < RECOVER_BATCH; ++k) e[k] = use_high(div, uses[j + k]);
 #pragma unroll
     for (u32 k = 0; k < RECOVER_BATCH; ++k) {
       es[k] = sizes[e[k]];
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(BLOCK) k_recover_by_volume(u32 nv, u32 const* 
     }
   }
   for (; j < e1; ++j) {
-    u32 const e = adj[j];
+    u32 const e = use_high(div, uses[j]);
     double const es = sizes[e];
     size_sum += es;
     sum += es * f[(size_t)e * nc + c];
@@ -276,7 +276,7 @@ void recover_by_volume(Mesh& m, char const* name)
   double* out = dalloc<double>((size_t)nv * nc, s);
   if (nv && nc) {
     CK(launch_kernel(k_recover_by_volume, dim3(grid_for((u64)nv * nc)), dim3(BLOCK), 0, s, nv, ve.offs,
-        ve.adj, sizes, nc, static_cast<double const*>(m.find_tag(dim, name)->data), out));
+        ve.uses, use_div(deg(dim, 0)), sizes, nc, static_cast<double const*>(m.find_tag(dim, name)->data), out));
     CK_LAUNCH();
   }
   dev_free(sizes, s);

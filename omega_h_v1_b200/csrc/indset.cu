@@ -33,8 +33,7 @@ static_assert(COOP_CTL_SLOT + COOP_CTL_WORDS == INDSET_FETCH_SLOTS, "mailbox slo
 struct Nbrs {
   u32 mode;
   u32 const* offs;   // up(ent, via)
-  u32 const* adj;
-  u32 const* dirs;
+  u32 const* uses;
   u32 const* down;   // down(via, ent) or verts_of_edges
   u32 per;           // entities per via-entity
 };
@@ -100,17 +99,14 @@ template <int G, u32 PER>
 __device__ inline void load_neighbors(Nbrs const& g, u32 i, u32 j, u32 re, u32* o)
 {
   if (PER == 1) {
-    u32 e[2], d[2];
+    u32 u[2];
 #pragma unroll
-    for (u32 k = 0; k < 2; ++k) {
-      bool const on = j + k * G < re;
-      e[k] = on ? g.adj[j + k * G] : INV;
-      d[k] = on ? g.dirs[j + k * G] : 0u;
-    }
+    for (u32 k = 0; k < 2; ++k) u[k] = j + k * G < re ? g.uses[j + k * G] : INV;
 #pragma unroll
-    for (u32 k = 0; k < 2; ++k) o[k] = e[k] != INV ? g.down[(size_t)e[k] * 2 + (1 - d[k])] : INV;
+    for (u32 k = 0; k < 2; ++k) o[k] = u[k] != INV ? g.down[u[k] ^ 1u] : INV;
   } else {
-    u32 const* ds = g.down + (size_t)g.adj[j] * PER;
+    u32 const use = g.uses[j];
+    u32 const* ds = g.down + (use - use % PER);
 #pragma unroll
     for (u32 k = 0; k < PER; ++k) o[k] = ds[k];
 #pragma unroll
@@ -237,9 +233,9 @@ __device__ void indset_rounds(u32 n, Nbrs const& g, Key const* was, u32* st, u32
       };
       for (u32 j = rb + lg; j < re; j += G) {
         if (g.mode == 0) {
-          visit(g.down[g.adj[j] * 2 + (1 - g.dirs[j])]);
+          visit(g.down[g.uses[j] ^ 1u]);
         } else {
-          u32 const* ds = g.down + (size_t)g.adj[j] * g.per;
+          u32 const* ds = g.down + (g.uses[j] - g.uses[j] % g.per);
           for (u32 k = 0; k < g.per; ++k)
             if (ds[k] != i) visit(ds[k]);
         }
@@ -623,16 +619,14 @@ u32* find_indset(Mesh& m, u32 ent_dim, IndsetIn& in, double const* good, bool ch
     UpAdj const& u = m.ask_up(0, 1, false);
     g.mode = 0;
     g.offs = u.offs;
-    g.adj = u.adj;
-    g.dirs = u.dirs;
+    g.uses = u.uses;
     g.down = m.ask_down(1, 0);
     g.per = 2;
   } else if (ent_dim == 1 && m.dim >= 2) {
     UpAdj const& u = m.ask_up(1, m.dim, false);
     g.mode = 1;
     g.offs = u.offs;
-    g.adj = u.adj;
-    g.dirs = u.dirs;
+    g.uses = u.uses;
     g.down = m.ask_down(m.dim, 1);
     g.per = deg(m.dim, 1);
   } else {
@@ -978,15 +972,15 @@ void interp_coords_to_elems(Mesh& m)
 // ---------------------------------------------------------------------------
 // marking (mark.cpp)
 
-__global__ void k_mark_down(u32 n, u32 const* __restrict__ offs, u32 const* __restrict__ adj,
-    u32 const* __restrict__ marked, u32* __restrict__ out)
+__global__ void k_mark_down(u32 n, u32 const* __restrict__ offs, u32 const* __restrict__ uses,
+    UseDiv div, u32 const* __restrict__ marked, u32* __restrict__ out)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   u32 r = 0;
   for (u32 j = offs[i]; j < offs[i + 1]; ++j)
-    if (marked[adj[j]]) {
+    if (marked[use_high(div, uses[j])]) {
       r = 1;
       break;
     }
@@ -999,7 +993,7 @@ u32* mark_down(Mesh& m, u32 high, u32 low, u32 const* marked)
   UpAdj const& u = m.ask_up(low, high, false);
   u32* out = dalloc<u32>(n, m.s);
   if (n) {
-    CK(launch_kernel(k_mark_down, dim3(grid_for(n)), dim3(BLOCK), 0, m.s, n, u.offs, u.adj, marked, out));
+    CK(launch_kernel(k_mark_down, dim3(grid_for(n)), dim3(BLOCK), 0, m.s, n, u.offs, u.uses, use_div(deg(high, low)), marked, out));
     CK_LAUNCH();
   }
   return out;

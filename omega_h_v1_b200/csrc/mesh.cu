@@ -2,10 +2,10 @@
 //
 // Adjacency kernels (all one pass over their inputs, no host round trips
 // except where an output size must be known to allocate):
-//   up_from_down   counting by atomics, one scan, atomic fill, then a
-//                  warp-per-row rank sort that restores the deterministic
-//                  row order of the reference's CPU invert_map
-//                  (invert_map.cpp:92-136) and splits use -> (high, dir)
+//   up_from_down   counting by atomics, one scan, atomic fill of one word a
+//                  use, then (where the order is asked for) a sort of each
+//                  row in place that restores the deterministic row order of
+//                  the reference's CPU invert_map (invert_map.cpp:92-136)
 //   reflect_down   one thread per (high entity, local low slot); searches the
 //                  first vertex's upward list (reflect_down.cpp:13-38,
 //                  find_by_verts.hpp:14-55)
@@ -134,6 +134,7 @@ void Mesh::clear_contents()
       down[h][l] = nullptr;
       if (have_up[l][h]) {
         dev_free(up[l][h].offs, s);
+        dev_free(up[l][h].uses, s);
         dev_free(up[l][h].adj, s);
         dev_free(up[l][h].dirs, s);
         dev_free(up[l][h].pre, s);
@@ -368,77 +369,26 @@ __global__ void k_count_lows(u32 const* __restrict__ loh, u32 nuses, u32* cnt)
 }
 
 // cnt holds each row's count: a row's uses take its slots from the end down
-// (their order is arbitrary either way; the rows are ranked or marked
+// (their order is arbitrary either way; the rows are sorted or marked
 // unsorted afterwards), so no cursor array is zeroed for the fill
 __global__ void k_fill_uses(u32 const* __restrict__ loh, u32 nuses,
-    u32 const* __restrict__ offs, u32* cnt, u32* __restrict__ tmp)
+    u32 const* __restrict__ offs, u32* cnt, u32* __restrict__ uses)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nuses) return;
   u32 l = loh[i];
   u32 slot = atomicSub(&cnt[l], 1u) - 1u;
-  tmp[offs[l] + slot] = i;
+  uses[offs[l] + slot] = i;
 }
 
-// One warp per row: every lane ranks its element against the whole row and
-// writes it to its sorted position (rows hold distinct use indices).
-__global__ void k_rank_rows(u32 const* __restrict__ offs, u32 const* __restrict__ tmp,
-    u32 nrows, u32 lph, u32* __restrict__ adj, u32* __restrict__ dirs)
-{
-  pdl_wait();
-  u32 row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  u32 lane = threadIdx.x & 31;
-  if (row >= nrows) return;
-  u32 f = offs[row], len = offs[row + 1] - f;
-  for (u32 base = 0; base < len; base += 32) {
-    u32 idx = base + lane;
-    u32 my = idx < len ? tmp[f + idx] : INV;
-    u32 rank = 0;
-    for (u32 cb = 0; cb < len; cb += 32) {
-      u32 other = (cb + lane < len) ? tmp[f + cb + lane] : INV;
-      u32 lim = len - cb < 32 ? len - cb : 32;
-      for (u32 j = 0; j < lim; ++j) {
-        u32 v = __shfl_sync(0xffffffffu, other, j);
-        rank += (v < my) ? 1u : 0u;
-      }
-    }
-    if (idx < len) {
-      adj[f + rank] = my / lph;
-      dirs[f + rank] = my % lph;
-    }
-  }
-}
-
-// Each row (the uses of one low entity, filled in arbitrary order) is
-// sorted by a group of G lanes holding K elements each: a bitonic network
-// over N = G*K slots in registers, partners across lanes exchanged by
-// shuffles, the missing slots padded with the largest key. Rows longer than
-// N (rare: N is at least 2.5x the mean degree) are ranked by the group from
-// global memory after the network, outside any shuffle.
+// A bitonic network over N = G*K keys held by G lanes, K each (key k of lane
+// l is the network's k*G + l): partners across lanes by shuffles.
 template <int G, int K>
-__global__ void __launch_bounds__(256)
-k_sort_rows(u32 const* __restrict__ offs, u32 const* __restrict__ pre,
-    u32 const* __restrict__ tmp, u32 nrows, u32 lph, u32* __restrict__ adj,
-    u32* __restrict__ dirs)
+__device__ __forceinline__ void sort_keys(u32 (&v)[K], u32 l)
 {
-  pdl_wait();
-  constexpr int N = G * K;
-  u32 row = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  u32 l = threadIdx.x % G;
-  u32 f = 0, len = 0;
-  if (row < nrows) {
-    f = offs[row] + (pre ? pre[row] : 0u);
-    len = offs[row + 1] - f;
-  }
-  u32 v[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    u32 idx = k * G + l;
-    v[k] = (idx < len && len <= (u32)N) ? tmp[f + idx] : 0xffffffffu;
-  }
-#pragma unroll
-  for (int size = 2; size <= N; size <<= 1) {
+  for (int size = 2; size <= G * K; size <<= 1) {
 #pragma unroll
     for (int j = size >> 1; j > 0; j >>= 1) {
       u32 nv[K];
@@ -456,69 +406,86 @@ k_sort_rows(u32 const* __restrict__ offs, u32 const* __restrict__ pre,
       for (int k = 0; k < K; ++k) v[k] = nv[k];
     }
   }
-  if (len <= (u32)N) {
+}
+
+// Each row (the uses of one low entity, filled in arbitrary order), or with
+// pre its part after the first pre[row] (a carried row's, in order and below
+// the rest), is sorted in place by a group of G lanes holding K elements
+// each, the missing slots padded with the largest key. Rows longer than
+// N = G*K (rare: N is at least 2.5x the mean) are the whole warp's after
+// that, one at a time: up to 32 by the same network, more by one in memory
+// whose every compare ascends (a merge starts with its half mirrored), so
+// that the slots past the end, largest keys all, never move and are left out.
+// Bound by the network's issue on the vertices of an 80^3 adapt (2 M rows of
+// 14 edges, 2 M of 24 tets: 0.98 -> 0.87 ms, and no pass packing highs and directions before it);
+// a few long rows given to their group's two lanes instead of the warp held a
+// launch of a small pass 26 us (now 7).
+template <int G, int K>
+__global__ void __launch_bounds__(256)
+k_sort_rows(u32 const* __restrict__ offs, u32 const* __restrict__ pre, u32 nrows, u32* uses)
+{
+  pdl_wait();
+  constexpr u32 N = G * K, FULL = 0xffffffffu;
+  u32 row = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+  u32 l = threadIdx.x % G, lane = threadIdx.x % 32;
+  u32 f = 0, len = 0;
+  if (row < nrows) {
+    f = offs[row] + (pre ? pre[row] : 0u);
+    len = offs[row + 1] - f;
+  }
+  u32 const held = len <= N ? len : 0;
+  u32 v[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      u32 idx = k * G + l;
-      if (idx < len) {
-        adj[f + idx] = v[k] / lph;
-        dirs[f + idx] = v[k] % lph;
+  for (int k = 0; k < K; ++k) v[k] = k * G + l < held ? uses[f + k * G + l] : INV;
+  sort_keys<G, K>(v, l);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (k * G + l < held) uses[f + k * G + l] = v[k];
+  for (u32 rest = __ballot_sync(FULL, l == 0 && len > N); rest; rest &= rest - 1) {
+    u32 const src = __ffs(rest) - 1;
+    u32* a = uses + __shfl_sync(FULL, f, src);
+    u32 const n = __shfl_sync(FULL, len, src);
+    if (N < 32 && n <= 32) {
+      u32 w[1] = {lane < n ? a[lane] : INV};
+      sort_keys<32, 1>(w, lane);
+      if (lane < n) a[lane] = w[0];
+      continue;
+    }
+    for (u32 size = 2; size < 2 * n; size <<= 1)
+      for (u32 j = size >> 1; j > 0; j >>= 1) {
+        u32 const flip = j == size >> 1 ? size - 1 : j;
+        for (u32 i = lane; i < n; i += 32) {
+          u32 const o = i ^ flip;
+          if (o <= i || o >= n) continue;
+          u32 const x = a[i], y = a[o];
+          if (y < x) {
+            a[i] = y;
+            a[o] = x;
+          }
+        }
+        __syncwarp();
       }
-    }
-  } else {
-    for (u32 a = l; a < len; a += G) {
-      u32 x = tmp[f + a], rank = 0;
-      for (u32 b = 0; b < len; ++b) rank += (tmp[f + b] < x) ? 1u : 0u;
-      adj[f + rank] = x / lph;
-      dirs[f + rank] = x % lph;
-    }
   }
 }
 
 template <int G, int K>
-static void launch_sort_rows(u32 const* offs, u32 const* pre, u32 const* tmp, u32 nrows,
-    u32 lph, u32* adj, u32* dirs, cudaStream_t s)
+static void launch_sort_rows(UpAdj const& u, u32 nrows, cudaStream_t s)
 {
   u64 threads = (u64)nrows * G;
-  CK(launch_kernel(k_sort_rows<G, K>, dim3(grid_for(threads)), dim3(256), 0, s, offs, pre, tmp, nrows, lph, adj, dirs));
+  CK(launch_kernel(k_sort_rows<G, K>, dim3(grid_for(threads)), dim3(256), 0, s, u.offs, u.pre,
+      nrows, u.uses));
   CK_LAUNCH();
 }
 
-// sort every row (or, given pre, every row's part after its first pre[l]
-// uses); nsort = the uses to be sorted in all
-static void rank_rows(u32 const* offs, u32 const* pre, u32 const* tmp, u32 nrows, u32 nsort,
-    u32 lph, u32* adj, u32* dirs, cudaStream_t s)
-{
-  double avg = nrows ? (double)nsort / nrows : 1.0;
-  double want = 2.5 * avg;
-  if (want <= 2) launch_sort_rows<2, 1>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-  else if (want <= 4) launch_sort_rows<4, 1>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-  else if (want <= 8) launch_sort_rows<8, 1>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-  else if (want <= 16) launch_sort_rows<16, 1>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-  else if (want <= 32) launch_sort_rows<32, 1>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-  else if (want <= 64) launch_sort_rows<32, 2>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-  else launch_sort_rows<32, 4>(offs, pre, tmp, nrows, lph, adj, dirs, s);
-}
-
-// as k_fill_uses, the row's slots taken from its end down
-__global__ void k_fill_uses_split(u32 const* __restrict__ loh, u32 nuses, u32 lph,
-    u32 const* __restrict__ offs, u32* cnt, u32* __restrict__ adj, u32* __restrict__ dirs)
-{
-  pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nuses) return;
-  u32 l = loh[i];
-  u32 slot = offs[l] + atomicSub(&cnt[l], 1u) - 1u;
-  adj[slot] = i / lph;
-  dirs[slot] = i % lph;
-}
-
-__global__ void k_join_uses(u32 n, u32 lph, u32 const* __restrict__ adj,
-    u32 const* __restrict__ dirs, u32* __restrict__ uses)
+__global__ void k_split_uses(u32 n, UseDiv div, u32 const* __restrict__ uses,
+    u32* __restrict__ adj, u32* __restrict__ dirs)
 {
   pdl_wait();
   u32 j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) uses[j] = adj[j] * lph + dirs[j];
+  if (j >= n) return;
+  u32 const u = uses[j], h = use_high(div, u);
+  adj[j] = h;
+  dirs[j] = u - h * div.lph;
 }
 
 void up_from_down_unsorted(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* loh,
@@ -534,81 +501,39 @@ void up_from_down_unsorted(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* 
     CK_LAUNCH();
   }
   out.offs = exscan_new(cnt, nlows, s);
-  out.adj = dalloc<u32>(nuses, s);
-  out.dirs = dalloc<u32>(nuses, s);
+  out.uses = dalloc<u32>(nuses, s);
   if (nuses) {
-    PROBE(P_UP_FILL, s, 4.0 * nuses + 4.0 * (nlows + 1.0) + 4.0 * nlows + 8.0 * nuses);
-    CK(launch_kernel(k_fill_uses_split, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, lph, out.offs, cnt,
-        out.adj, out.dirs));
+    PROBE(P_UP_FILL, s, 4.0 * nuses + 4.0 * (nlows + 1.0) + 4.0 * nlows + 4.0 * nuses);
+    CK(launch_kernel(k_fill_uses, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, out.offs,
+        cnt, out.uses));
     CK_LAUNCH();
   }
   dev_free(cnt, s);
 }
 
-// the packed uses of each row's part after its first pre[l] (the part the
-// sort reorders), a thread per row: a carried row's tail holds only the
-// uses of the entities the pass made, so most rows have none
-__global__ void k_join_tails(u32 nlows, u32 lph, u32 const* __restrict__ offs,
-    u32 const* __restrict__ pre, u32 const* __restrict__ adj, u32 const* __restrict__ dirs,
-    u32* __restrict__ uses)
-{
-  pdl_wait();
-  for (u32 l = blockIdx.x * blockDim.x + threadIdx.x; l < nlows; l += gridDim.x * blockDim.x)
-    for (u32 p = offs[l] + pre[l], e = offs[l + 1]; p < e; ++p) uses[p] = adj[p] * lph + dirs[p];
-}
-
+// every row in place (given pre: every row's part after its first pre[l] uses)
 void sort_up_rows(u32 high, u32 low, u32 nhighs, u32 nlows, UpAdj const& u,
     cudaStream_t s)
 {
-  u32 lph = deg(high, low);
-  u32 nuses = nhighs * lph;
+  u32 nuses = nhighs * deg(high, low);
   if (!nuses || !nlows) return;
-  u32* uses = dalloc<u32>(nuses, s);
-  if (u.pre) {
-    CK(launch_kernel(k_join_tails, dim3(std::min<u32>(grid_for(nlows), 148u * 8u)),
-        dim3(BLOCK), 0, s, nlows, lph, u.offs, u.pre, u.adj, u.dirs, uses));
-  } else {
-    CK(launch_kernel(k_join_uses, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, nuses, lph, u.adj,
-        u.dirs, uses));
-  }
-  CK_LAUNCH();
-  {
-    u32 nsort = u.pre ? nuses - u.npre : nuses;
-    PROBE(P_UP_RANK, s, 12.0 * nsort + 4.0 * (nlows + 1.0));
-    rank_rows(u.offs, u.pre, uses, nlows, nsort, lph, u.adj, u.dirs, s);
-  }
-  dev_free(uses, s);
+  u32 nsort = u.pre ? nuses - u.npre : nuses;
+  PROBE(P_UP_RANK, s, 8.0 * nsort + 4.0 * (nlows + 1.0));
+  double want = 2.5 * (double)nsort / nlows;
+  if (want <= 2) launch_sort_rows<2, 1>(u, nlows, s);
+  else if (want <= 4) launch_sort_rows<4, 1>(u, nlows, s);
+  else if (want <= 8) launch_sort_rows<8, 1>(u, nlows, s);
+  else if (want <= 16) launch_sort_rows<16, 1>(u, nlows, s);
+  else if (want <= 32) launch_sort_rows<32, 1>(u, nlows, s);
+  else if (want <= 64) launch_sort_rows<32, 2>(u, nlows, s);
+  else launch_sort_rows<32, 4>(u, nlows, s);
 }
 
 void up_from_down(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* loh,
     UpAdj& out, cudaStream_t s)
 {
-  u32 lph = deg(high, low);
-  u32 nuses = nhighs * lph;
-  u32* cnt = dalloc<u32>((size_t)nlows + 1, s);
-  CK(cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s));
-  if (nuses) {
-    PROBE(P_UP_COUNT, s, 4.0 * nuses + 4.0 * nlows);
-    CK(launch_kernel(k_count_lows, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, cnt));
-    CK_LAUNCH();
-  }
-  out.offs = exscan_new(cnt, nlows, s);
-  u32* tmp = dalloc<u32>(nuses, s);
-  out.adj = dalloc<u32>(nuses, s);
-  out.dirs = dalloc<u32>(nuses, s);
-  if (nuses) {
-    {
-      PROBE(P_UP_FILL, s, 8.0 * nuses + 4.0 * (nlows + 1.0) + 4.0 * nlows);
-      CK(launch_kernel(k_fill_uses, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, out.offs, cnt, tmp));
-      CK_LAUNCH();
-    }
-    if (nlows) {
-      PROBE(P_UP_RANK, s, 12.0 * nuses + 4.0 * (nlows + 1.0));
-      rank_rows(out.offs, nullptr, tmp, nlows, nuses, lph, out.adj, out.dirs, s);
-    }
-  }
-  dev_free(tmp, s);
-  dev_free(cnt, s);
+  up_from_down_unsorted(high, low, nhighs, nlows, loh, out, s);
+  sort_up_rows(high, low, nhighs, nlows, out, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -816,12 +741,12 @@ __global__ void k_reflect_keyed(const __grid_constant__ ReflectJobs jobs)
 // ---------------------------------------------------------------------------
 // star graphs (star.cpp)
 
-__global__ void k_vertex_edge_star(u32 nadj, u32 const* __restrict__ adj,
-    u32 const* __restrict__ dirs, u32 const* __restrict__ voe, u32* __restrict__ star)
+__global__ void k_vertex_edge_star(u32 nadj, u32 const* __restrict__ uses,
+    u32 const* __restrict__ voe, u32* __restrict__ star)
 {
   pdl_wait();
   u32 j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nadj) star[j] = voe[adj[j] * 2 + (1 - dirs[j])];
+  if (j < nadj) star[j] = voe[uses[j] ^ 1u];  // (the edge's other end)
 }
 
 __global__ void k_scale_offsets(u32 const* __restrict__ in, u32 n1, u32 k,
@@ -832,13 +757,13 @@ __global__ void k_scale_offsets(u32 const* __restrict__ in, u32 n1, u32 k,
   if (i < n1) out[i] = in[i] * k;
 }
 
-__global__ void k_edge_tri_star(u32 nadj, u32 const* __restrict__ adj,
-    u32 const* __restrict__ dirs, u32 const* __restrict__ eot, u32* __restrict__ star)
+__global__ void k_edge_tri_star(u32 nadj, u32 const* __restrict__ uses,
+    u32 const* __restrict__ eot, u32* __restrict__ star)
 {
   pdl_wait();
   u32 j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nadj) return;
-  u32 t = adj[j], d = dirs[j];
+  u32 t = uses[j] / 3, d = uses[j] % 3;
   star[j * 2 + 0] = eot[t * 3 + (d + 1) % 3];
   star[j * 2 + 1] = eot[t * 3 + (d + 2) % 3];
 }
@@ -853,8 +778,8 @@ __global__ void k_sum_degrees(u32 n, u32 const* __restrict__ a, u32 const* __res
 
 __global__ void k_edge_tet_star(u32 n, u32 const* __restrict__ so,
     u32 const* __restrict__ ts_offs, u32 const* __restrict__ ts,
-    u32 const* __restrict__ roe_offs, u32 const* __restrict__ roe,
-    u32 const* __restrict__ roe_dirs, u32 const* __restrict__ eor, u32* __restrict__ star)
+    u32 const* __restrict__ roe_offs, u32 const* __restrict__ roe_uses,
+    u32 const* __restrict__ eor, u32* __restrict__ star)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -862,7 +787,7 @@ __global__ void k_edge_tet_star(u32 n, u32 const* __restrict__ so,
   u32 o = so[i];
   for (u32 j = ts_offs[i]; j < ts_offs[i + 1]; ++j) star[o++] = ts[j];
   for (u32 j = roe_offs[i]; j < roe_offs[i + 1]; ++j)
-    star[o++] = eor[roe[j] * 6 + tet_opp_edge(roe_dirs[j])];
+    star[o++] = eor[roe_uses[j] / 6 * 6 + tet_opp_edge(roe_uses[j] % 6)];
 }
 
 constexpr u32 STAR_BUF = 256;
@@ -877,7 +802,7 @@ constexpr u32 STAR_BUF = 256;
 constexpr u32 STAR_WARPS = BLOCK / 32;
 
 __global__ void __launch_bounds__(BLOCK) k_star_general(u32 n, u32 const* __restrict__ hl_offs,
-    u32 const* __restrict__ hl, u32 const* __restrict__ loh, u32 lph,
+    u32 const* __restrict__ hl_uses, u32 const* __restrict__ loh, UseDiv div,
     u32 const* __restrict__ star_offs, u32* __restrict__ deg_out,
     u32* __restrict__ star, u32* err)
 {
@@ -887,12 +812,12 @@ __global__ void __launch_bounds__(BLOCK) k_star_general(u32 n, u32 const* __rest
   u32* const kept = s_kept[threadIdx.x >> 5];
   u32 const i = (blockIdx.x * BLOCK + threadIdx.x) >> 5;
   if (i >= n) return;
-  u32 const f = hl_offs[i], nuse = (hl_offs[i + 1] - f) * lph;
+  u32 const lph = div.lph, f = hl_offs[i], nuse = (hl_offs[i + 1] - f) * lph;
   u32 size = 0;
   for (u32 b = 0; b < nuse; b += 32) {
     u32 const c = b + lane;
     u32 sl = INV;
-    if (c < nuse) sl = loh[(size_t)hl[f + c / lph] * lph + c % lph];
+    if (c < nuse) sl = loh[(size_t)use_high(div, hl_uses[f + c / lph]) * lph + c % lph];
     u32 const peers = __match_any_sync(0xffffffffu, sl);
     bool fresh = sl != INV && sl != i && lane == (u32)(__ffs(peers) - 1);
     for (u32 a = 0; a < size; ++a)
@@ -916,20 +841,23 @@ __global__ void __launch_bounds__(BLOCK) k_star_general(u32 n, u32 const* __rest
 // ---------------------------------------------------------------------------
 // element dual (dual.cpp)
 
-__global__ void k_dual_from_sides(u32 ne, u32 spe, u32 const* __restrict__ soe,
-    u32 const* __restrict__ es_offs, u32 const* __restrict__ es, u32* __restrict__ out)
+__global__ void k_dual_from_sides(u32 ne, UseDiv div, u32 const* __restrict__ soe,
+    u32 const* __restrict__ es_offs, u32 const* __restrict__ es_uses, u32* __restrict__ out)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ne) return;
+  u32 const spe = div.lph;
   for (u32 j = 0; j < spe; ++j) {
     u32 s = soe[i * spe + j];
     u32 o = INV;
-    for (u32 k = es_offs[s]; k < es_offs[s + 1]; ++k)
-      if (es[k] != i) {
-        o = es[k];
+    for (u32 k = es_offs[s]; k < es_offs[s + 1]; ++k) {
+      u32 const h = use_high(div, es_uses[k]);
+      if (h != i) {
+        o = h;
         break;
       }
+    }
     out[i * spe + j] = o;
   }
 }
@@ -943,7 +871,7 @@ constexpr u32 DUAL_BATCH = 4;
 
 template <u32 DIM>
 __global__ void k_dual_from_verts(u32 ne, u32 const* __restrict__ voe,
-    u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev,
+    u32 const* __restrict__ ev_offs, u32 const* __restrict__ ev_uses,
     u32* __restrict__ out, u32* err)
 {
   pdl_wait();
@@ -960,7 +888,7 @@ __global__ void k_dual_from_verts(u32 ne, u32 const* __restrict__ voe,
   for (u32 a = f; a < e && found == INV; a += DUAL_BATCH) {
     u32 o[DUAL_BATCH], w[DUAL_BATCH][VPE];
 #pragma unroll
-    for (u32 q = 0; q < DUAL_BATCH; ++q) o[q] = a + q < e ? ev[a + q] : i;
+    for (u32 q = 0; q < DUAL_BATCH; ++q) o[q] = a + q < e ? ev_uses[a + q] / VPE : i;
 #pragma unroll
     for (u32 q = 0; q < DUAL_BATCH; ++q)
 #pragma unroll
@@ -1309,35 +1237,37 @@ __global__ void k_new_ids(u32 n, u32 const* __restrict__ same, u32* __restrict__
 }
 
 // The uses of the entities the pass made (generated uses first..nuses-1 of
-// the new down(high, low), lph per high entity): cnt holds each row's kept +
+// the new down(high, low)): cnt holds each row's kept +
 // generated uses, and the generated ones take the slots after the kept
 // ones, from the row's end down (their order within a row is arbitrary
 // either way: the rows are marked unsorted). The fill kernels below run
 // these on their threads past the old rows, so the two parts of a row's
 // fill, which write disjoint slots, share one launch.
 struct UpGen {
-  u32 first, nuses, lph;
+  u32 first, nuses;
   u32 const* loh;
   u32* cnt;
 };
 
 __device__ inline void up_gen_fill(UpGen const& g, u32 k, u32 const* __restrict__ offs,
-    u32* __restrict__ adj, u32* __restrict__ dirs)
+    u32* __restrict__ uses)
 {
   u32 const u = g.first + k;
   if (u >= g.nuses) return;
   u32 l = g.loh[u];
   u32 slot = offs[l] + atomicSub(&g.cnt[l], 1u) - 1u;
-  adj[slot] = u / g.lph;
-  dirs[slot] = u % g.lph;
+  uses[slot] = u;
 }
 
 constexpr u32 FILL_BATCH = 8;
 
+// LPH: lows per high entity. A use moves with its high: u / LPH is looked up,
+// u % LPH stays.
+template <u32 LPH>
 __global__ void k_up_surv_fill(u32 nl_old, u32 const* __restrict__ same_l,
     u32 const* __restrict__ newid_h, u32 const* __restrict__ offs_old,
-    u32 const* __restrict__ adj_old, u32 const* __restrict__ dirs_old,
-    u32 const* __restrict__ offs, u32* __restrict__ adj, u32* __restrict__ dirs, UpGen gen)
+    u32 const* __restrict__ uses_old, u32 const* __restrict__ offs, u32* __restrict__ uses,
+    UpGen gen)
 {
   pdl_wait();
   u32 j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1357,71 +1287,50 @@ __global__ void k_up_surv_fill(u32 nl_old, u32 const* __restrict__ same_l,
   // one run of the old array and of the new one, so the warp reads and
   // writes them coalesced, unless one of them is by an entity that did not
   // survive (its row then took a new use in its place). Most runs of a pass
-  // that changes little are such (91 -> 71 us a launch over a 48^3 adapt).
+  // that changes little are such (91 -> 71 us a launch over a 48^3 adapt
+  // with a high and a direction apart; one word a use then took the eleven
+  // launches of an 80^3 adapt from 3.87 to 2.57 ms).
   u32 const lane = threadIdx.x & 31;
   if (__all_sync(0xffffffffu, clean)) {
     u32 const u0 = __shfl_sync(0xffffffffu, r0, 0);
     u32 const n = __shfl_sync(0xffffffffu, e, 31) - u0;
     u32 const w0 = __shfl_sync(0xffffffffu, w, 0);
     if (n <= 32 * FILL_BATCH) {
-      u32 a[FILL_BATCH], d[FILL_BATCH];
+      u32 a[FILL_BATCH], h[FILL_BATCH];
 #pragma unroll
-      for (u32 k = 0; k < FILL_BATCH; ++k) {
-        u32 const u = k * 32 + lane;
-        a[k] = d[k] = 0;
-        if (u < n) {
-          a[k] = adj_old[u0 + u];
-          d[k] = dirs_old[u0 + u];
-        }
-      }
+      for (u32 k = 0; k < FILL_BATCH; ++k) a[k] = k * 32 + lane < n ? uses_old[u0 + k * 32 + lane] : 0u;
       bool all = true;
 #pragma unroll
       for (u32 k = 0; k < FILL_BATCH; ++k)
         if (k * 32 + lane < n) {
-          a[k] = newid_h[a[k]];
-          all = all && a[k] != INV;
+          h[k] = newid_h[a[k] / LPH];
+          all = all && h[k] != INV;
         }
       if (__all_sync(0xffffffffu, all)) {
 #pragma unroll
-        for (u32 k = 0; k < FILL_BATCH; ++k) {
-          u32 const u = k * 32 + lane;
-          if (u < n) {
-            adj[w0 + u] = a[k];
-            dirs[w0 + u] = d[k];
-          }
-        }
+        for (u32 k = 0; k < FILL_BATCH; ++k)
+          if (k * 32 + lane < n) uses[w0 + k * 32 + lane] = h[k] * LPH + a[k] % LPH;
         return;
       }
     }
   }
   if (j >= nl_old) {
-    up_gen_fill(gen, j - nl_old, offs, adj, dirs);
+    up_gen_fill(gen, j - nl_old, offs, uses);
     return;
   }
   if (!kept) return;
   // FILL_BATCH uses per round, predicated past the row's end (INV marks
-  // those: no high entity has that id), so most rows take one round of
-  // loads and one of gathers
+  // those: no use has that index), so most rows take one round of loads
+  // and one of gathers
   for (u32 r = r0; r < e; r += FILL_BATCH) {
-    u32 a[FILL_BATCH], d[FILL_BATCH];
+    u32 a[FILL_BATCH], h[FILL_BATCH];
 #pragma unroll
-    for (u32 k = 0; k < FILL_BATCH; ++k) {
-      a[k] = INV;
-      d[k] = 0;
-      if (r + k < e) {
-        a[k] = adj_old[r + k];
-        d[k] = dirs_old[r + k];
-      }
-    }
+    for (u32 k = 0; k < FILL_BATCH; ++k) a[k] = r + k < e ? uses_old[r + k] : INV;
 #pragma unroll
-    for (u32 k = 0; k < FILL_BATCH; ++k) a[k] = a[k] != INV ? newid_h[a[k]] : INV;
+    for (u32 k = 0; k < FILL_BATCH; ++k) h[k] = a[k] != INV ? newid_h[a[k] / LPH] : INV;
 #pragma unroll
     for (u32 k = 0; k < FILL_BATCH; ++k)
-      if (a[k] != INV) {
-        adj[w] = a[k];
-        dirs[w] = d[k];
-        ++w;
-      }
+      if (h[k] != INV) uses[w++] = h[k] * LPH + a[k] % LPH;
   }
 }
 
@@ -1441,11 +1350,10 @@ struct UpFillJob {
   u32 const* same_l;
   u32 const* newid_h;
   u32 const* offs_old;
-  u32 const* adj_old;
-  u32 const* dirs_old;
+  u32 const* uses_old;
   u32 const* offs;
-  u32* adj;
-  u32* dirs;
+  u32* uses;
+  UseDiv div;
   UpGen gen;
 };
 struct UpFillJobs {
@@ -1461,18 +1369,17 @@ __global__ void k_up_surv_fill_grouped(const __grid_constant__ UpFillJobs jobs)
   u32 const* __restrict__ same_l = jb.same_l;
   u32 const* __restrict__ newid_h = jb.newid_h;
   u32 const* __restrict__ offs_old = jb.offs_old;
-  u32 const* __restrict__ adj_old = jb.adj_old;
-  u32 const* __restrict__ dirs_old = jb.dirs_old;
+  u32 const* __restrict__ uses_old = jb.uses_old;
   u32 const* __restrict__ offs = jb.offs;
-  u32* __restrict__ adj = jb.adj;
-  u32* __restrict__ dirs = jb.dirs;
+  u32* __restrict__ uses = jb.uses;
+  UseDiv const div = jb.div;
   UpGen const gen = jb.gen;
   u32 const t = blockIdx.x * blockDim.x + threadIdx.x;
   u32 const j = t / CG, g = t % CG;
   if (j >= nl_old) {
     // past the rows' groups (a multiple of CG threads): one thread per
     // generated use
-    up_gen_fill(gen, t - nl_old * CG, offs, adj, dirs);
+    up_gen_fill(gen, t - nl_old * CG, offs, uses);
     return;
   }
   u32 const nj = same_l[j];
@@ -1486,14 +1393,13 @@ __global__ void k_up_surv_fill_grouped(const __grid_constant__ UpFillJobs jobs)
     u32 const u = base + g;
     u32 na = INV, d = 0;
     if (u < e) {
-      na = newid_h[adj_old[u]];
-      d = dirs_old[u];
+      u32 const old = uses_old[u], h = use_high(div, old);
+      na = newid_h[h];
+      d = old - h * div.lph;
     }
     u32 const kept = (__ballot_sync(gmask, na != INV) & gmask) >> gbase;
     if (na != INV) {
-      u32 const pos = w + __popc(kept & below);
-      adj[pos] = na;
-      dirs[pos] = d;
+      uses[w + __popc(kept & below)] = na * div.lph + d;
     }
     w += __popc(kept);
   }
@@ -1655,29 +1561,28 @@ void carry_up_fill(Mesh& m, Mesh& out, UpCarry& c, UpFillJobs& grouped, u32& ngr
   cudaStream_t s = out.s;
   UpAdj const& old = m.up[c.low][c.high];
   UpAdj& u = c.u;
-  u.adj = dalloc<u32>(c.nuses, s);
-  u.dirs = dalloc<u32>(c.nuses, s);
+  u.uses = dalloc<u32>(c.nuses, s);
   u32 const cg = tuned(TK_CARRY_GROUP), gb = tuned(TK_GATHER_BLOCK);
   u64 const ngen = c.nuses > c.first ? c.nuses - c.first : 0;
-  UpGen const gen{c.first, c.nuses, c.lph, c.loh, c.cnt};
+  UpGen const gen{c.first, c.nuses, c.loh, c.cnt};
   if (c.long_rows) {
-    grouped.j[ngrouped++] = UpFillJob{c.nl_old, c.same_l, c.newid_h, old.offs, old.adj,
-        old.dirs, u.offs, u.adj, u.dirs, gen};
+    grouped.j[ngrouped++] = UpFillJob{c.nl_old, c.same_l, c.newid_h, old.offs, old.uses,
+        u.offs, u.uses, use_div(c.lph), gen};
     gmost = std::max<u64>(gmost, (u64)c.nl_old * cg + ngen);
-    gbytes += 8.0 * (c.nl_old + 1) + 8.0 * c.nuses_old + 4.0 * c.nh_old + 4.0 * (c.nl + 1) +
-        8.0 * c.first + 20.0 * ngen;
+    gbytes += 8.0 * (c.nl_old + 1) + 4.0 * c.nuses_old + 4.0 * c.nh_old + 4.0 * (c.nl + 1) +
+        4.0 * c.first + 16.0 * ngen;
   } else if (c.nl_old || ngen) {
-    // each array once: same_l and the old offsets, the old rows' highs and
-    // directions, the highs' new ids, the new offsets, the kept uses (first)
-    // written as highs and directions; per generated use its low, the
-    // row's offset and count, and the use written
+    // each array once: same_l and the old offsets, the old rows' uses, the
+    // highs' new ids, the new offsets, the kept uses (first) written; per
+    // generated use its low, the row's offset and count, and the use written
     // (the fill of edge and face rows, the largest single kernel of an
     // adapt, is probed on its own: carry_up_fill)
-    PROBE(P_CARRY_UP_FILL, s, 8.0 * (c.nl_old + 1) + 8.0 * c.nuses_old + 4.0 * c.nh_old +
-        4.0 * (c.nl + 1) + 8.0 * c.first + 20.0 * ngen);
-    CK(launch_kernel(k_up_surv_fill, dim3(grid_for((u64)c.nl_old + ngen, gb)), dim3(gb), 0,
-        s, c.nl_old, c.same_l, c.newid_h, old.offs, old.adj, old.dirs, u.offs, u.adj, u.dirs,
-        gen));
+    PROBE(P_CARRY_UP_FILL, s, 8.0 * (c.nl_old + 1) + 4.0 * c.nuses_old + 4.0 * c.nh_old +
+        4.0 * (c.nl + 1) + 4.0 * c.first + 16.0 * ngen);
+    auto kf = c.lph == 2 ? k_up_surv_fill<2> : c.lph == 3 ? k_up_surv_fill<3>
+            : c.lph == 4 ? k_up_surv_fill<4> : k_up_surv_fill<6>;
+    CK(launch_kernel(kf, dim3(grid_for((u64)c.nl_old + ngen, gb)), dim3(gb), 0, s, c.nl_old,
+        c.same_l, c.newid_h, old.offs, old.uses, u.offs, u.uses, gen));
     CK_LAUNCH();
   }
 }
@@ -1847,10 +1752,8 @@ UpAdj const& Mesh::ask_up(u32 low, u32 high, bool sorted)
     UpAdj u;
     u.offs = dalloc<u32>((size_t)n + 1, s);
     iota_u32(u.offs, n + 1, 1, s);
-    u.adj = dalloc<u32>(n, s);
-    iota_u32(u.adj, n, 1, s);
-    u.dirs = dalloc<u32>(n, s);
-    fill_u32(u.dirs, n, 0, s);
+    u.uses = dalloc<u32>(n, s);
+    iota_u32(u.uses, n, 1, s);
     up[low][high] = u;
     up_sorted[low][high] = true;
   } else {
@@ -1865,6 +1768,23 @@ UpAdj const& Mesh::ask_up(u32 low, u32 high, bool sorted)
   }
   have_up[low][high] = true;
   return up[low][high];
+}
+
+UpAdj const& Mesh::ask_up_apart(u32 low, u32 high)
+{
+  ask_up(low, high, true);
+  UpAdj& u = up[low][high];
+  if (!u.adj) {
+    u32 const lph = deg(high, low), n = counts[high] * lph;
+    u.adj = dalloc<u32>(n, s);
+    u.dirs = dalloc<u32>(n, s);
+    if (n) {
+      CK(launch_kernel(k_split_uses, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, use_div(lph),
+          u.uses, u.adj, u.dirs));
+      CK_LAUNCH();
+    }
+  }
+  return u;
 }
 
 Graph const& Mesh::ask_star(u32 low, u32 high)
@@ -1894,7 +1814,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     CK(cudaMemcpyAsync(g.offs, ev.offs, sizeof(u32) * (n + 1), cudaMemcpyDeviceToDevice, s));
     g.adj = dalloc<u32>(g.nadj, s);
     if (g.nadj) {
-      CK(launch_kernel(k_vertex_edge_star, dim3(grid_for(g.nadj)), dim3(BLOCK), 0, s, g.nadj, ev.adj, ev.dirs, voe, g.adj));
+      CK(launch_kernel(k_vertex_edge_star, dim3(grid_for(g.nadj)), dim3(BLOCK), 0, s, g.nadj, ev.uses, voe, g.adj));
       CK_LAUNCH();
     }
   } else if (low == 1 && high == 2) {
@@ -1909,7 +1829,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     CK_LAUNCH();
     g.adj = dalloc<u32>(g.nadj, s);
     if (nuse) {
-      CK(launch_kernel(k_edge_tri_star, dim3(grid_for(nuse)), dim3(BLOCK), 0, s, nuse, te.adj, te.dirs, eot, g.adj));
+      CK(launch_kernel(k_edge_tri_star, dim3(grid_for(nuse)), dim3(BLOCK), 0, s, nuse, te.uses, eot, g.adj));
       CK_LAUNCH();
     }
   } else if (low == 1 && high == 3 && has_dim(2)) {
@@ -1929,7 +1849,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     g.adj = dalloc<u32>(g.nadj, s);
     if (n) {
       CK(launch_kernel(k_edge_tet_star, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, g.offs, ts.offs, ts.adj, re.offs,
-          re.adj, re.dirs, eor, g.adj));
+          re.uses, eor, g.adj));
       CK_LAUNCH();
     }
   } else {
@@ -1942,7 +1862,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     u32* err = mb->dev + 60;
     CK(cudaMemsetAsync(err, 0, sizeof(u32), s));
     if (n) {
-      CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.adj, loh, lph,
+      CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.uses, loh, use_div(lph),
           nullptr, degree, nullptr, err));
       CK_LAUNCH();
     }
@@ -1951,7 +1871,7 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     g.nadj = read_u32(g.offs + n, s);
     g.adj = dalloc<u32>(g.nadj, s);
     if (n) {
-      CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.adj, loh, lph, g.offs,
+      CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.uses, loh, use_div(lph), g.offs,
           nullptr, g.adj, err));
       CK_LAUNCH();
     }
@@ -1971,7 +1891,7 @@ u32 const* Mesh::ask_dual()
     u32 const* soe = ask_down(dim, dim - 1);
     UpAdj const& es = ask_up(dim - 1, dim, false);
     if (nel) {
-      CK(launch_kernel(k_dual_from_sides, dim3(grid_for(nel)), dim3(BLOCK), 0, s, nel, spe, soe, es.offs, es.adj, out));
+      CK(launch_kernel(k_dual_from_sides, dim3(grid_for(nel)), dim3(BLOCK), 0, s, nel, use_div(spe), soe, es.offs, es.uses, out));
       CK_LAUNCH();
     }
   } else {
@@ -1982,7 +1902,7 @@ u32 const* Mesh::ask_dual()
     if (nel) {
       auto k = dim == 3 ? k_dual_from_verts<3> : dim == 2 ? k_dual_from_verts<2> : k_dual_from_verts<1>;
       CK(launch_kernel(k, dim3(grid_for((u64)nel * spe)), dim3(BLOCK), 0, s, nel, voe, ev.offs,
-          ev.adj, out, err));
+          ev.uses, out, err));
       CK_LAUNCH();
     }
     if (read_u32(err, s)) throw Failure(E_ARG, "vertex with more than 256 elements");

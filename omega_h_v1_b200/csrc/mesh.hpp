@@ -6,9 +6,10 @@
 // Layout in HBM (all u32 local ids, f64 fields, u64 global numbers):
 //   down[d][0]        verts_of_ents, deg(d,0) per entity, entity-major
 //   down[h][l]        lows_of_highs (0 < l < h), deg(h,l) per high entity
-//   up[l][h]          CSR: offs[n_l+1], adj[n_uses], dirs[n_uses]; each row
-//                     sorted by use index (high * deg + dir), which is the
-//                     order the reference's CPU invert_map produces
+//   up[l][h]          CSR: offs[n_l+1], uses[n_uses], a use being the index
+//                     high * deg + dir; ascending in a row, which is the
+//                     order the reference's CPU invert_map produces, once an
+//                     ordered row is asked for
 //   tags[d]           ordered list of named arrays, n_d * ncomps values each
 //   globals[d]        u64 global numbers (parallel meshes only)
 #pragma once
@@ -36,12 +37,15 @@ inline u32 tag_esz(u32 type)
 
 struct UpAdj {
   u32* offs = nullptr;
-  u32* adj = nullptr;
-  u32* dirs = nullptr;
+  u32* uses = nullptr;  // high * lph + dir (UseDiv)
   // rows carried through a pass: the first pre[l] uses of row l are already
   // in order and precede the rest (null when nothing is known)
   u32* pre = nullptr;
   u32 npre = 0;  // sum of pre
+  // the highs and the directions apart, as the C API returns them: written
+  // when first asked for (Mesh::ask_up_apart)
+  u32* adj = nullptr;
+  u32* dirs = nullptr;
 };
 
 struct Graph {
@@ -155,6 +159,8 @@ struct Mesh {
   // depend on (edge rings, transfers, vertex_dest, the C API). Rows built
   // for order-free consumers are sorted in place on the first ordered ask.
   UpAdj const& ask_up(u32 low, u32 high, bool sorted = true);
+  // the same, ordered, with adj and dirs written
+  UpAdj const& ask_up_apart(u32 low, u32 high);
   Graph const& ask_star(u32 low, u32 high);
   u32 const* ask_dual();
 

@@ -117,14 +117,14 @@ template <u32 DIM, bool F32>
 __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
     u32 const* __restrict__ nlist, u32 const* __restrict__ voe1,
     u32 const* __restrict__ voe, u32 const* __restrict__ eo_offs,
-    u32 const* __restrict__ eo, u32 const* __restrict__ eo_dirs,
-    double const* __restrict__ x, double qual_floor, SegView sv, Fp32Stats* fs,
+    u32 const* __restrict__ eo, double const* __restrict__ x, double qual_floor, SegView sv, Fp32Stats* fs,
     u32* __restrict__ cand, double* __restrict__ out, unsigned long long* __restrict__ keys,
     u32* any, u32* inverted)
 {
   pdl_wait();
   constexpr u32 dim = DIM;  // the element dimension (2 or 3): loops over
                             // an element's vertices unroll, corners stay in registers
+  constexpr u32 EPE = deg(DIM, 1);
   u32 const n = list ? *nlist : ne;
   for (u32 base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     u32 const t = base + threadIdx.x;
@@ -156,10 +156,11 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
         unsigned long long need = 0;  // children (2 per element) that can hold the minimum
         bool all = 2 * (e - f) > 64;
         for (u32 j = f; j < e; ++j) {
-          u32 const* ve = voe + (size_t)eo[j] * vpe;
+          u32 const use = eo[j], dir = use % EPE;
+          u32 const* ve = voe + (size_t)(use / EPE) * vpe;
           for (u32 k = 0; k < 2; ++k) {
             double ex[4][3];
-            refine_child(dim, ve, eo_dirs[j], k, x, split, ex);
+            refine_child(dim, ve, dir, k, x, split, ex);
             Q32 q = tet_quality_f32(ex, k6);
             float lo = q32_lo(q);
             upright = upright && lo > 0.0f;
@@ -174,11 +175,12 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
           filtered = 2;
           rechecked = true;
           for (u32 j = f; j < e; ++j) {
-            u32 const* ve = voe + (size_t)eo[j] * vpe;
+            u32 const use = eo[j], dir = use % EPE;
+          u32 const* ve = voe + (size_t)(use / EPE) * vpe;
             for (u32 k = 0; k < 2; ++k) {
               if (!all && !((need >> (2 * (j - f) + k)) & 1ull)) continue;
               double ex[4][3];
-              refine_child(dim, ve, eo_dirs[j], k, x, split, ex);
+              refine_child(dim, ve, dir, k, x, split, ex);
               double q = tet_quality(ex, perfect);
               if (fs->audit) fp32_note_error(fs, tet_quality_f32(ex, k6), q);
               if (q < minq) minq = q;
@@ -191,10 +193,11 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
           audited = true;
           double m64 = 1;
           for (u32 j = f; j < e; ++j) {
-            u32 const* ve = voe + (size_t)eo[j] * vpe;
+            u32 const use = eo[j], dir = use % EPE;
+          u32 const* ve = voe + (size_t)(use / EPE) * vpe;
             for (u32 k = 0; k < 2; ++k) {
               double ex[4][3];
-              refine_child(dim, ve, eo_dirs[j], k, x, split, ex);
+              refine_child(dim, ve, dir, k, x, split, ex);
               double q = tet_quality(ex, perfect);
               fp32_note_error(fs, tet_quality_f32(ex, k6), q);
               if (q < m64) m64 = q;
@@ -207,10 +210,11 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
       }
       if (!filtered) {
         for (u32 j = f; j < e; ++j) {
-          u32 const* ve = voe + (size_t)eo[j] * vpe;
+          u32 const use = eo[j], dir = use % EPE;
+          u32 const* ve = voe + (size_t)(use / EPE) * vpe;
           for (u32 k = 0; k < 2; ++k) {
             double ex[4][3];
-            refine_child(dim, ve, eo_dirs[j], k, x, split, ex);
+            refine_child(dim, ve, dir, k, x, split, ex);
             double q = dim == 3 ? tet_quality(ex, perfect) : tri_quality(ex, 0, perfect);
             if (!(q > 0)) atomicOr(inverted, 1u);
             if (q < minq) minq = q;
@@ -333,7 +337,8 @@ __device__ inline void vertex_maps(VertexMaps const& vm, u32 i)
 // maps.
 struct SplitMark {
   u32 const* offs;  // up(1, dd) of the mesh being refined
-  u32 const* adj;
+  u32 const* uses;
+  UseDiv div;
   u32* marks;
   u32 gen;
 };
@@ -353,7 +358,7 @@ __global__ void k_mark_split_domains(u32 const* __restrict__ list,
     for (u32 q = 0; q < 2; ++q) {
       SplitMark const& d = sm.d[q];
       if (!d.marks) continue;
-      for (u32 j = d.offs[e], f = d.offs[e + 1]; j < f; ++j) d.marks[d.adj[j]] = d.gen;
+      for (u32 j = d.offs[e], f = d.offs[e + 1]; j < f; ++j) d.marks[use_high(d.div, d.uses[j])] = d.gen;
     }
   }
   if (vm.zero)
@@ -515,7 +520,8 @@ static u32 refine_build(Mesh& m, EdgeSplits const& es, bool deferred, bool unifo
     if (!uniform && nd && m.have_up[1][dd]) {
       SplitMark& d = sm.d[dd - 2];
       d.offs = m.up[1][dd].offs;
-      d.adj = m.up[1][dd].adj;
+      d.uses = m.up[1][dd].uses;
+      d.div = use_div(deg(dd, 1));
       d.marks = stream_marks(KEPT_SPLIT + dd, nd, s, &d.gen);
       any_sparse = true;
       sp[dd].offs = dalloc<u32>((size_t)nd + 1, s);
@@ -767,7 +773,7 @@ static u32* choose_refinement(Mesh& m, u32* cand, double qual_floor, double** qu
       u32 grid = grid_for(ne, qb);
       if (list) grid = std::min(grid, resident_blocks(kq, qb));
       CK(launch_kernel(kq, dim3(grid), dim3(qb), 0, s, ne, list, nlist, m.ask_down(1, 0),
-          m.ask_down(dim, 0), eo.offs, eo.adj, eo.dirs, m.coords(), qual_floor, m.segview(),
+          m.ask_down(dim, 0), eo.offs, eo.uses, m.coords(), qual_floor, m.segview(),
           m.fp32_filter ? fp32_stats_dev() : nullptr, cand, q,
           listed ? listed->keys : nullptr, any, inverted));
       CK_LAUNCH();

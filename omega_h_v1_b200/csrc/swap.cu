@@ -112,7 +112,7 @@ void swap_table_host(u32 rs, u32* ntri, u32* nmesh, u32* nint, u32* tris, u32* i
 // find_edge_ring (edge_ring.cpp:12-74): the ring vertices of an edge, in the
 // order that walks around it starting from its first upward tet
 __device__ u32 find_edge_ring(u32 edge, u32 const* __restrict__ te_offs,
-    u32 const* __restrict__ te, u32 const* __restrict__ te_dirs,
+    u32 const* __restrict__ te,
     u32 const* __restrict__ voe1, u32 const* __restrict__ vot, u32* ev, u32* rv)
 {
   u32 f = te_offs[edge], e = te_offs[edge + 1];
@@ -122,7 +122,7 @@ __device__ u32 find_edge_ring(u32 edge, u32 const* __restrict__ te_offs,
   ev[1] = voe1[edge * 2 + 1];
   u32 ta[MAX_EDGE_SWAP], tb[MAX_EDGE_SWAP];
   for (u32 i = 0; i < rs; ++i) {
-    u32 t = te[f + i], d = te_dirs[f + i];
+    u32 t = te[f + i] / 6, d = te[f + i] % 6;
     u32 const* tv = vot + (size_t)t * 4;
     u32 align = (tv[tet_edge_vert(d, 0)] != ev[0]) ? 1u : 0u;
     u32 o = tet_opp_edge(d);
@@ -258,7 +258,7 @@ __global__ void k_unmark_boundary(u32 n, u32 dim, u32 const* __restrict__ cd,
 
 // swap_quality (swap_qualities.cpp:13-61)
 __global__ void k_swap_quality(u32 ne, u32 const* __restrict__ te_offs,
-    u32 const* __restrict__ te, u32 const* __restrict__ te_dirs,
+    u32 const* __restrict__ te,
     u32 const* __restrict__ voe1, u32 const* __restrict__ vot,
     double const* __restrict__ x, double const* __restrict__ eq, Fp32Stats* fs,
     u32* __restrict__ cand, double* __restrict__ quals,
@@ -272,9 +272,9 @@ __global__ void k_swap_quality(u32 ne, u32 const* __restrict__ te_offs,
   if (i < ne && cand[i]) {
     double old_minq = 1;
     for (u32 j = te_offs[i]; j < te_offs[i + 1]; ++j)
-      if (eq[te[j]] < old_minq) old_minq = eq[te[j]];
+      if (eq[te[j] / 6] < old_minq) old_minq = eq[te[j] / 6];
     u32 ev[2], rv[MAX_EDGE_SWAP];
-    u32 rs = find_edge_ring(i, te_offs, te, te_dirs, voe1, vot, ev, rv);
+    u32 rs = find_edge_ring(i, te_offs, te, voe1, vot, ev, rv);
     if (rs > MAX_EDGE_SWAP || rs < 3) {
       cand[i] = 0;
     } else {
@@ -354,14 +354,14 @@ __global__ void k_swap_counts(u32 ne, u32 dim, u32 const* __restrict__ ind,
 __global__ void k_swap_cavity(u32 ne, u32 dim, u32 const* __restrict__ ind,
     u32 const* __restrict__ codes, u32 const* __restrict__ gen_offs,
     u32 const* __restrict__ te_offs, u32 const* __restrict__ te,
-    u32 const* __restrict__ te_dirs, u32 const* __restrict__ voe1,
+    u32 const* __restrict__ voe1,
     u32 const* __restrict__ vot, u32* __restrict__ out)
 {
   pdl_wait();
   u32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ne || !ind[i]) return;
   u32 ev[2], rv[MAX_EDGE_SWAP];
-  u32 rs = find_edge_ring(i, te_offs, te, te_dirs, voe1, vot, ev, rv);
+  u32 rs = find_edge_ring(i, te_offs, te, voe1, vot, ev, rv);
   u32 code = codes[i];
   u32 vpe = deg(dim, 0);
   u32* o = out + (size_t)gen_offs[i] * vpe;
@@ -429,7 +429,7 @@ __global__ void k_swap_conserve(u32 ne, u32 nc, u32 nsame, u32 const* __restrict
   double sum[MAX_NCOMPS];
   for (u32 c = 0; c < nc; ++c) sum[c] = 0;
   for (u32 j = te_offs[i]; j < te_offs[i + 1]; ++j)
-    for (u32 c = 0; c < nc; ++c) sum[c] = sum[c] + in[(size_t)te[j] * nc + c];
+    for (u32 c = 0; c < nc; ++c) sum[c] = sum[c] + in[(size_t)(te[j] / 6) * nc + c];
   u32 f = gen_offs[i], e = gen_offs[i + 1];
   double cav = 0;
   for (u32 j = f; j < e; ++j) cav += sizes[nsame + j];
@@ -450,7 +450,7 @@ __global__ void k_swap_fit(u32 ne, u32 nc, u32 const* __restrict__ gen_offs,
   u32 f = te_offs[i], e = te_offs[i + 1];
   for (u32 c = 0; c < nc; ++c) {
     double avg = 0;
-    for (u32 k = f; k < e; ++k) avg += in[(size_t)te[k] * nc + c];
+    for (u32 k = f; k < e; ++k) avg += in[(size_t)(te[k] / 6) * nc + c];
     avg /= (e - f);
     for (u32 g = gen_offs[i]; g < gen_offs[i + 1]; ++g) gen[(size_t)g * nc + c] = avg;
   }
@@ -520,7 +520,7 @@ static bool swap_select(Mesh& m, double gq, u32 nlayers, SwapSel& sel, u32* sliv
   PROBE(P_SWAP_QUALITY, s, 4.0 * (ne + 1) + 8.0 * 6.0 * m.counts[3] + 8.0 * ne +
       16.0 * m.counts[3] + 24.0 * m.counts[0] + 8.0 * m.counts[3] + 4.0 * ne + 16.0 * ne);
   u32 const qb = std::min<u32>(tuned(TK_QUALITY_BLOCK), 128u);
-  CK(launch_kernel(k_swap_quality, dim3(grid_for(ne, qb)), dim3(qb), 0, s, ne, te.offs, te.adj, te.dirs, m.ask_down(1, 0),
+  CK(launch_kernel(k_swap_quality, dim3(grid_for(ne, qb)), dim3(qb), 0, s, ne, te.offs, te.uses, m.ask_down(1, 0),
       m.ask_down(3, 0), m.coords(), eq, m.fp32_filter ? fp32_stats_dev() : nullptr, sel.cand,
       sel.quals, sel.in.keys, sel.in.own_list, nlist, sel.in.out, sel.rs, sel.codes, any));
   CK_LAUNCH();
@@ -628,7 +628,7 @@ static bool swap_build(Mesh& m, SwapSel const& sel, bool deferred)
     u32* conn = dalloc<u32>((size_t)(nsame + ngen) * vpe, s);
     expand_scaled(m.ask_down(ed, 0), same_offs, 1, n, vpe, 4, conn, s);
     CK(launch_kernel(k_swap_cavity, dim3(ceil_div(ne, 128)), dim3(128), 0, s, ne, ed, sel.ind, sel.codes, gen_offs, te.offs,
-        te.adj, te.dirs, voe1, vot, conn + (size_t)nsame * vpe));
+        te.uses, voe1, vot, conn + (size_t)nsame * vpe));
     CK_LAUNCH();
     out->set_ents(ed, nsame + ngen, conn);
     if (m.full) {
@@ -657,7 +657,7 @@ static bool swap_build(Mesh& m, SwapSel const& sel, bool deferred)
           double* data = dalloc<double>((size_t)(nsame + ngen) * nc, s);
           expand_scaled(t.data, same_offs, 1, n, nc, 8, data, s);
           CK(launch_kernel(k_swap_conserve, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, nc, nsame, gen_offs, te.offs,
-              te.adj, sizes, static_cast<double const*>(t.data), data + (size_t)nsame * nc));
+              te.uses, sizes, static_cast<double const*>(t.data), data + (size_t)nsame * nc));
           CK_LAUNCH();
           out->add_tag(ed, T_F64, t.name.c_str(), nc, t.transfer, data);
         }
@@ -668,7 +668,7 @@ static bool swap_build(Mesh& m, SwapSel const& sel, bool deferred)
         u32 nc = t.ncomps;
         double* data = dalloc<double>((size_t)(nsame + ngen) * nc, s);
         expand_scaled(t.data, same_offs, 1, n, nc, 8, data, s);
-        CK(launch_kernel(k_swap_fit, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, nc, gen_offs, te.offs, te.adj,
+        CK(launch_kernel(k_swap_fit, dim3(grid_for(ne)), dim3(BLOCK), 0, s, ne, nc, gen_offs, te.offs, te.uses,
             static_cast<double const*>(t.data), data + (size_t)nsame * nc));
         CK_LAUNCH();
         out->add_tag(ed, T_F64, t.name.c_str(), nc, t.transfer, data);
