@@ -207,35 +207,7 @@ __global__ void __launch_bounds__(BLOCK) k_coarsen_class_list(u32 ne, u32 const*
 // after collapsing each allowed direction. One warp per candidate edge (from
 // a compact list): the lanes share the collapsing vertex's elements, so a
 // few candidates with long rows no longer idle the other lanes of a warp.
-// Each minimum is reduced as (value, position) pairs, so the value kept is
-// the one the sequential loop keeps: the first in row order among equals
-// (which decides the sign of a zero), with NaN never taken.
-struct FirstMin {
-  double v;
-  u32 k;  // 0 = the loop's initial value, else 1 + position in the row
-};
-
-__device__ inline void first_min_add(FirstMin& m, double q, u32 k)
-{
-  if (q < m.v) {
-    m.v = q;
-    m.k = k;
-  }
-}
-
-__device__ inline double warp_first_min(FirstMin m)
-{
-  for (int o = 16; o; o >>= 1) {
-    double ov = __shfl_xor_sync(0xffffffffu, m.v, o);
-    u32 ok = __shfl_xor_sync(0xffffffffu, m.k, o);
-    if (ov < m.v || (ov == m.v && ok < m.k)) {
-      m.v = ov;
-      m.k = ok;
-    }
-  }
-  return m.v;
-}
-
+// Each minimum is reduced as (value, position) pairs (FirstMin).
 __device__ inline float warp_minf(float v)
 {
   for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -277,7 +249,7 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
       FirstMin om{1.0, 0};
       if (eq)
         for (u32 k = f + lane; k < e; k += 32) first_min_add(om, eq[ev[k] / vpe], k - f + 1);
-      double old_minq = warp_first_min(om);
+      double old_minq = lanes_first_min(32, om);
       // with the filter: the cavity's estimates first; the direction is
       // rejected on them when the worst element is surely below the floor or
       // surely no better than before; otherwise only the elements whose
@@ -327,7 +299,7 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
           if (use32 && filtered && fs->audit) fp32_note_error(fs, tet_quality_f32(ex, k6), q);
           first_min_add(mm, q, k - f + 1);
         }
-        minq = warp_first_min(mm);
+        minq = lanes_first_min(32, mm);
       }
       bool drop = rejected32 || minq < fq || (eq && minq <= old_minq);
       if (use32 && filtered && fs->audit) {
@@ -346,7 +318,7 @@ __global__ void k_coarsen_quality(u32 const* __restrict__ list,
           fp32_note_error(fs, tet_quality_f32(ex, k6), q);
           first_min_add(m64, q, k - f + 1);
         }
-        double q64 = warp_first_min(m64);
+        double q64 = lanes_first_min(32, m64);
         bool drop64 = q64 < fq || (eq && q64 <= old_minq);
         bool flip = drop64 != drop || (!drop && q64 != minq);
         ++naudited;

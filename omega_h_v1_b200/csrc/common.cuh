@@ -208,6 +208,36 @@ __device__ __forceinline__ u32 use_high(UseDiv d, u32 use)
   return d.lph == 1 ? use : __umulhi(use, d.mul) >> d.sh;
 }
 
+// A minimum taken by several lanes, as (value, position) pairs: the value kept
+// is the one a sequential loop keeps, the first among equals (which decides
+// the sign of a zero), with NaN never taken.
+struct FirstMin {
+  double v;
+  u32 k;  // 0 = the loop's initial value, else 1 + position in the row
+};
+
+__device__ inline void first_min_add(FirstMin& m, double q, u32 k)
+{
+  if (q < m.v) {
+    m.v = q;
+    m.k = k;
+  }
+}
+
+// over groups of n lanes (a power of two), by whole warps
+__device__ inline double lanes_first_min(u32 n, FirstMin m)
+{
+  for (u32 o = n / 2; o; o >>= 1) {
+    double ov = __shfl_xor_sync(0xffffffffu, m.v, o);
+    u32 ok = __shfl_xor_sync(0xffffffffu, m.k, o);
+    if (ov < m.v || (ov == m.v && ok < m.k)) {
+      m.v = ov;
+      m.k = ok;
+    }
+  }
+  return m.v;
+}
+
 // ---------------------------------------------------------------------------
 // geometry (size.hpp, quality.hpp, algebra.hpp)
 

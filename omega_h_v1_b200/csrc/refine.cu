@@ -94,6 +94,57 @@ __device__ inline void refine_child(u32 dim, u32 const* __restrict__ ve, u32 dir
   ex[vpe - 1][2] = split[2];
 }
 
+// an edge has five tets in the mean or two triangles, two children each
+template <u32 DIM>
+constexpr u32 QUALITY_LANES = DIM == 3 ? 16 : 4;
+
+// the listed edges of k_refine_quality below, several lanes an edge
+template <u32 DIM>
+__device__ __forceinline__ void refine_quality_short(u32 n, u32 const* __restrict__ list,
+    u32 const* __restrict__ voe1, u32 const* __restrict__ voe, u32 const* __restrict__ eo_offs,
+    u32 const* __restrict__ eo, double const* __restrict__ x, double qual_floor,
+    SegView const& sv, double* __restrict__ out, unsigned long long* __restrict__ keys, u32* any,
+    u32* inverted)
+{
+  constexpr u32 EPE = deg(DIM, 1), VPE = deg(DIM, 0);
+  double const perfect = DIM == 3 ? perfect_tet_quality() : perfect_tri_quality();
+  u32 const threads = gridDim.x * blockDim.x;
+  u32 lanes = QUALITY_LANES<DIM>;
+  while ((u64)n * lanes > threads) lanes >>= 1;
+  u32 const t0 = blockIdx.x * blockDim.x + threadIdx.x, t = t0 / lanes, sub = t0 % lanes;
+  u32 i = 0;
+  double fl = 0;
+  FirstMin m{1.0, 0};
+  if (t < n) {
+    i = list[t];
+    u32 const a = voe1[i * 2], b = voe1[i * 2 + 1];
+    double split[3];
+    for (u32 c = 0; c < 3; ++c) {
+      double acc = 0;
+      acc += x[a * 3 + c];
+      acc += x[b * 3 + c];
+      split[c] = acc / 2u;
+    }
+    fl = seg_floor(sv, a, qual_floor);
+    u32 const f = eo_offs[i], nch = 2 * (eo_offs[i + 1] - f);
+    for (u32 c = sub; c < nch; c += lanes) {
+      u32 const use = eo[f + c / 2];
+      double ex[4][3];
+      refine_child(DIM, voe + (size_t)(use / EPE) * VPE, use % EPE, c % 2, x, split, ex);
+      double const q = DIM == 3 ? tet_quality(ex, perfect) : tri_quality(ex, 0, perfect);
+      if (!(q > 0)) atomicOr(inverted, 1u);
+      first_min_add(m, q, c + 1);
+    }
+  }
+  double const minq = lanes_first_min(lanes, m);
+  bool const keep = t < n && !(minq < fl);
+  if (keep && sub == 0) {
+    out[i] = minq;
+    keys[i] = indset_key(minq);
+  }
+  if (__any_sync(0xffffffffu, keep) && (threadIdx.x & 31) == 0) raise_flag(any);
+}
+
 // refine_quality (refine_qualities.cpp:16-82) for edges, require_better = 0:
 // the worst child of every element around the edge, split at its midpoint.
 // With the filter: the children's estimates first; the edge is rejected on
@@ -104,6 +155,12 @@ __device__ inline void refine_child(u32 dim, u32 const* __restrict__ ve, u32 dir
 // candidate edge, each lane some of its children, at 105 registers against
 // 82; and one wave of resident blocks striding over the edges, which left
 // the passes with many candidates to the threads that drew the most.)
+//
+// A short list (one that leaves the grid at least two lanes an edge) is not
+// bound by the children's arithmetic but by one thread's chain of them, ten
+// an edge: the edge's children are dealt to as many lanes as the grid has
+// for it, up to QUALITY_LANES (the passes of a 6^3 adapt 14-19 -> 5 us a launch,
+// the last ones of a 48^3 one 16 -> 5).
 //
 // With a list (the candidate kernel's, nlist of them): a grid of the blocks
 // that fit at once strides over the listed edges in block-wide steps (the
@@ -126,6 +183,11 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
                             // an element's vertices unroll, corners stay in registers
   constexpr u32 EPE = deg(DIM, 1);
   u32 const n = list ? *nlist : ne;
+  if (!F32 && list && 2ull * n <= gridDim.x * blockDim.x) {
+    refine_quality_short<DIM>(n, list, voe1, voe, eo_offs, eo, x, qual_floor, sv, out, keys, any,
+        inverted);
+    return;
+  }
   for (u32 base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     u32 const t = base + threadIdx.x;
     u32 const i = t < n ? (list ? list[t] : t) : 0u;
@@ -176,7 +238,7 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
           rechecked = true;
           for (u32 j = f; j < e; ++j) {
             u32 const use = eo[j], dir = use % EPE;
-          u32 const* ve = voe + (size_t)(use / EPE) * vpe;
+            u32 const* ve = voe + (size_t)(use / EPE) * vpe;
             for (u32 k = 0; k < 2; ++k) {
               if (!all && !((need >> (2 * (j - f) + k)) & 1ull)) continue;
               double ex[4][3];
@@ -194,7 +256,7 @@ __global__ void k_refine_quality(u32 ne, u32 const* __restrict__ list,
           double m64 = 1;
           for (u32 j = f; j < e; ++j) {
             u32 const use = eo[j], dir = use % EPE;
-          u32 const* ve = voe + (size_t)(use / EPE) * vpe;
+            u32 const* ve = voe + (size_t)(use / EPE) * vpe;
             for (u32 k = 0; k < 2; ++k) {
               double ex[4][3];
               refine_child(dim, ve, dir, k, x, split, ex);
@@ -771,7 +833,9 @@ static u32* choose_refinement(Mesh& m, u32* cand, double qual_floor, double** qu
       auto kq = dim == 2 ? k_refine_quality<2, false>
               : m.fp32_filter ? k_refine_quality<3, true> : k_refine_quality<3, false>;
       u32 grid = grid_for(ne, qb);
-      if (list) grid = std::min(grid, resident_blocks(kq, qb));
+      if (list)
+        grid = std::min(grid_for((u64)ne * (dim == 2 ? QUALITY_LANES<2> : QUALITY_LANES<3>), qb),
+            resident_blocks(kq, qb));
       CK(launch_kernel(kq, dim3(grid), dim3(qb), 0, s, ne, list, nlist, m.ask_down(1, 0),
           m.ask_down(dim, 0), eo.offs, eo.uses, m.coords(), qual_floor, m.segview(),
           m.fp32_filter ? fp32_stats_dev() : nullptr, cand, q,
