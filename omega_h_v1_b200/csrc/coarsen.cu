@@ -490,41 +490,68 @@ __global__ void k_collapse_to_ent(u32 n, u32 const* __restrict__ voe,
   will_gen[i] = wg;
 }
 
-// coarsen_elem (coarsen_topology.cpp:9-34) writing straight into the new
-// connectivity after the same entities, with remap_conn applied
-// (coarsen_common.cpp:29-33)
-// a thread per generating entity, from their list in order (the t-th
-// generates the t-th product)
-__global__ void k_coarsen_topology(u32 ed, u32 ngen, u32 const* __restrict__ gen_list,
-    u32 const* __restrict__ voe, u32 const* __restrict__ gen_vert,
-    u32 const* __restrict__ gen_dir, u32 const* __restrict__ same_v,
-    u32* __restrict__ out)
+// The new connectivity of every dimension, in one launch (a block's dimension
+// is the one whose blocks it lies among): the surviving entities' vertices,
+// renumbered, then coarsen_elem (coarsen_topology.cpp:9-34) of the generating
+// entities, a thread each from their list in order (the t-th generates the
+// t-th product), with remap_conn applied (coarsen_common.cpp:29-33). Two
+// launches a dimension were 24 us of a small pass, this one is 9 (39^3
+// coarsening, with the vertices' and the labels' copies in one launch too:
+// 3.50 -> 3.40 ms).
+struct ConnJob {
+  u32 first;  // block
+  u32 n, ngen;
+  u32 const* voe;
+  u32 const* same_e;
+  u32 const* gen_list;
+  u32 const* gen_vert;
+  u32 const* gen_dir;
+  u32* out;      // the survivors' rows
+  u32* gen_out;  // the products'
+};
+struct ConnJobs {
+  ConnJob j[3];  // dimensions 1 to 3 (those there are)
+};
+
+template <u32 ED>
+__device__ inline void coarsen_conn(ConnJob const& jb, u32 t, u32 const* __restrict__ same_v)
 {
-  pdl_wait();
-  u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ngen) return;
-  u32 const i = gen_list[t];
-  u32 vpe = deg(ed, 0);
-  u32* o = out + (size_t)t * vpe;
-  u32 b = opp(ed, 0, gen_dir[i]);
-  for (u32 j = 0; j + 1 < vpe; ++j)
-    o[j] = same_v[voe[(size_t)i * vpe + canon(ed, ed - 1, 0, b, j)]];
-  o[vpe - 1] = same_v[gen_vert[i]];
+  constexpr u32 VPE = ED + 1;
+  u32 const* __restrict__ voe = jb.voe;
+  if (t < jb.n) {
+    u32 const o = jb.same_e[t];
+    if (o == jb.same_e[t + 1]) return;
+    u32 v[VPE];
+#pragma unroll
+    for (u32 j = 0; j < VPE; ++j) v[j] = voe[(size_t)t * VPE + j];
+#pragma unroll
+    for (u32 j = 0; j < VPE; ++j) jb.out[(size_t)o * VPE + j] = same_v[v[j]];
+    return;
+  }
+  t -= jb.n;
+  if (t >= jb.ngen) return;
+  u32 const i = jb.gen_list[t];
+  u32* o = jb.gen_out + (size_t)t * VPE;
+  u32 const b = opp(ED, 0, jb.gen_dir[i]);
+  for (u32 j = 0; j + 1 < VPE; ++j)
+    o[j] = same_v[voe[(size_t)i * VPE + canon(ED, ED - 1, 0, b, j)]];
+  o[VPE - 1] = same_v[jb.gen_vert[i]];
 }
 
-// expansion of the surviving entities' vertices, renumbered
-template <u32 VPE>
-__global__ void k_same_conn(u32 n, u32 const* __restrict__ voe, u32 const* __restrict__ same_e,
-    u32 const* __restrict__ same_v, u32* __restrict__ out)
+__global__ void k_coarsen_conn(const __grid_constant__ ConnJobs jobs, u32 dim,
+    u32 const* __restrict__ same_v)
 {
   pdl_wait();
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || same_e[i] == same_e[i + 1]) return;
-  u32 o = same_e[i], v[VPE];
-#pragma unroll
-  for (u32 j = 0; j < VPE; ++j) v[j] = voe[(size_t)i * VPE + j];
-#pragma unroll
-  for (u32 j = 0; j < VPE; ++j) out[(size_t)o * VPE + j] = same_v[v[j]];
+  u32 ed = dim;
+  while (blockIdx.x < jobs.j[ed - 1].first) --ed;
+  ConnJob const& jb = jobs.j[ed - 1];
+  u32 const t = (blockIdx.x - jb.first) * blockDim.x + threadIdx.x;
+  if (ed == 1)
+    coarsen_conn<1>(jb, t, same_v);
+  else if (ed == 2)
+    coarsen_conn<2>(jb, t, same_v);
+  else
+    coarsen_conn<3>(jb, t, same_v);
 }
 
 // coarsen_conserve_cavity (coarsen_conserve.cpp:15-55)
@@ -942,7 +969,7 @@ static bool coarsen_build(Mesh& m, CoarsenSel const& sel, bool deferred)
   last_pass_stats().nselected = nv - nv_out;
   Mesh* out = m.spawn();
   out->set_ents(0, nv_out, nullptr);
-  // tags_subset (subset.cpp:15-43): every vertex tag survives (one launch)
+  // tags_subset (subset.cpp:15-43): every vertex tag survives
   std::vector<ExpandJob> vjobs;
   for (auto const& t : m.tags[0]) {
     u32 esz = tag_esz(t.type);
@@ -967,57 +994,48 @@ static bool coarsen_build(Mesh& m, CoarsenSel const& sel, bool deferred)
     jb.width = 1;
     vjobs.push_back(jb);
   }
-  expand_many(vjobs, s);
   if (m.parallel) inherit_globals(*out, 0);
-  // every dimension's label copies launched together after the loop (the
-  // generated lists and offsets they read are freed after that launch)
-  std::vector<ExpandJob> copies;
-  u32* free_after[8] = {};
-  u32 nfree = 0;
-  for (u32 dd = 0; dd < dim; ++dd) {
-    u32 ed = dim - dd;
+  // every dimension's connectivity in one launch, and the label copies of all
+  // of them in one with the vertices' tags
+  ConnJobs cj{};
+  u32 nblocks = 0;
+  for (u32 ed = 1; ed <= dim; ++ed) {
     u32 n = m.count(ed), vpe = deg(ed, 0);
-    u32 const* voe = m.ask_down(ed, 0);
     u32 ngen = m.mb->host[16 + 2 * (ed - 1)], nsame = m.mb->host[17 + 2 * (ed - 1)];
-    u32* gen_offs = gen_offs_of[ed];
-    u32* same_e = same_of[ed];
-    u32* gvert = gvert_of[ed];
-    u32* gdir = gdir_of[ed];
     u32 nout = nsame + ngen;
     u32* conn = dalloc<u32>((size_t)nout * vpe, s);
-    if (n) {
-      auto k = vpe == 2 ? k_same_conn<2> : vpe == 3 ? k_same_conn<3> : k_same_conn<4>;
-      CK(launch_kernel(k, dim3(grid_for(n)), dim3(BLOCK), 0, s, n, voe, same_e, same_v, conn));
-      CK_LAUNCH();
-      if (ngen) {
-        CK(launch_kernel(k_coarsen_topology, dim3(grid_for(ngen)), dim3(BLOCK), 0, s, ed, ngen,
-            gen_list_of[ed], voe, gvert, gdir, same_v, conn + (size_t)nsame * vpe));
-        CK_LAUNCH();
-      }
-    }
-    dev_free(gvert, s);
-    dev_free(gdir, s);
+    cj.j[ed - 1] = ConnJob{nblocks, n, ngen, m.ask_down(ed, 0), same_of[ed], gen_list_of[ed],
+        gvert_of[ed], gdir_of[ed], conn, conn + (size_t)nsame * vpe};
+    nblocks += ceil_div(n + ngen, BLOCK);
     out->set_ents(ed, nout, conn);
     // setup_coarsen (inherit.cpp:140-157)
     Doms d;
     d.ndoms[0] = n;
-    d.offs[0] = same_e;
+    d.offs[0] = same_of[ed];
     d.ngen[0] = nsame;
     d.ndoms[ed] = n;
-    d.offs[ed] = gen_offs;
+    d.offs[ed] = gen_offs_of[ed];
     d.ngen[ed] = ngen;
     d.list[ed] = gen_list_of[ed];
     d.nlist[ed] = ngen;
     d.finish();
-    inherit_class(m, *out, ed, d, nullptr, &copies);
-    free_after[nfree++] = gen_list_of[ed];
+    inherit_class(m, *out, ed, d, nullptr, &vjobs);
     if (m.parallel) inherit_globals(*out, ed);
-    if (ed == dim) coarsen_transfer(m, *out, gen_offs_v, gen_offs, same_e, nsame, ngen);
-    free_after[nfree++] = gen_offs;
     nsame_of[ed] = nsame;
   }
-  expand_many(copies, s);
-  for (u32 k = 0; k < nfree; ++k) dev_free(free_after[k], s);
+  expand_many(vjobs, s);
+  if (nblocks) {
+    CK(launch_kernel(k_coarsen_conn, dim3(nblocks), dim3(BLOCK), 0, s, cj, dim, same_v));
+    CK_LAUNCH();
+  }
+  coarsen_transfer(m, *out, gen_offs_v, gen_offs_of[dim], same_of[dim], nsame_of[dim],
+      out->count(dim) - nsame_of[dim]);
+  for (u32 ed = 1; ed <= dim; ++ed) {
+    dev_free(gvert_of[ed], s);
+    dev_free(gdir_of[ed], s);
+    dev_free(gen_list_of[ed], s);
+    dev_free(gen_offs_of[ed], s);
+  }
   same_of[0] = same_v;
   nsame_of[0] = nv_out;
   // downward adjacency of the survivors carries over; the products are searched

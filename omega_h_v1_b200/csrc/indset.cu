@@ -719,10 +719,18 @@ void expand_scaled(void const* in, u32 const* offs, u32 k, u32 n, u32 width,
   CK_LAUNCH();
 }
 
-// Several row expansions in one launch: blockIdx.y picks the job, the x
-// blocks stride over its rows (the same copy as k_expand_scaled).
+// Several row expansions in one launch (the same copy as k_expand_scaled):
+// blockIdx.y picks the job, the x blocks stride over its rows. The jobs that
+// do not go by words (lists of a pass's few producing entities, wide rows)
+// share one y where a y each would not fit the GPU at once: most of those
+// blocks had nothing to do (12 -> 8 us a launch in the small passes of a 39^3
+// coarsening, 26 -> 15 in a 24^3 warp step's). Where they fit, taking the
+// jobs in turn costs more than it saves (7 against 5 us on a 6^3 adapt).
+constexpr u32 EXPAND_MAX = 16;  // (a coarsening or refinement pass of a 3D mesh has 11 to 14)
 struct ExpandJobs {
-  ExpandJob j[8];
+  ExpandJob j[EXPAND_MAX];
+  u32 nrest;    // the first jobs do not go by words:
+  u32 together;  // blockIdx.y 0 takes this many of them in turn
 };
 
 template <class T>
@@ -812,11 +820,12 @@ __device__ inline void expand_same_rows(ExpandJob const& jb, u32 warp, u32 nwarp
 __global__ void __launch_bounds__(512, 3) k_expand_many(const __grid_constant__ ExpandJobs jobs)
 {
   pdl_wait();
-  ExpandJob const jb = jobs.j[blockIdx.y];
   u32 const t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  u32 const words = jb.esz == 4 ? jb.width : jb.esz == 8 ? 2 * jb.width : 0;
-  if (words && words <= 4 && !jb.list && jb.k == 1) {
+  u32 const q0 = blockIdx.y ? blockIdx.y + jobs.together - 1 : 0;
+  if (q0 >= jobs.nrest) {
+    ExpandJob const jb = jobs.j[q0];
     u32 const warp = t0 / 32, nwarps = stride / 32;
+    u32 const words = jb.width * (jb.esz / 4);
     if (words == 1)
       expand_same_rows<1>(jb, warp, nwarps);
     else if (words == 2)
@@ -827,43 +836,58 @@ __global__ void __launch_bounds__(512, 3) k_expand_many(const __grid_constant__ 
       expand_same_rows<4>(jb, warp, nwarps);
     return;
   }
-  for (u32 t = t0; t < jb.n; t += stride) {
-    u32 const i = jb.list ? jb.list[t] : t;
-    u32 f = jb.offs[i] * jb.k, e = jb.offs[i + 1] * jb.k;
-    if (jb.esz == 4) {
-      copy_rows<u32>(jb.in, jb.out, i, f, e, jb.width);
-      if (jb.in2) copy_rows<u32>(jb.in2, jb.out2, i, f, e, jb.width);
-    } else if (jb.esz == 8) {
-      copy_rows<unsigned long long>(jb.in, jb.out, i, f, e, jb.width);
-      if (jb.in2) copy_rows<unsigned long long>(jb.in2, jb.out2, i, f, e, jb.width);
-    } else {
-      copy_rows<unsigned char>(jb.in, jb.out, i, f, e, jb.width);
-      if (jb.in2) copy_rows<unsigned char>(jb.in2, jb.out2, i, f, e, jb.width);
+  for (u32 q = q0, end = blockIdx.y ? q0 + 1 : jobs.together; q < end; ++q) {
+    ExpandJob const jb = jobs.j[q];
+    for (u32 t = t0; t < jb.n; t += stride) {
+      u32 const i = jb.list ? jb.list[t] : t;
+      u32 f = jb.offs[i] * jb.k, e = jb.offs[i + 1] * jb.k;
+      if (jb.esz == 4) {
+        copy_rows<u32>(jb.in, jb.out, i, f, e, jb.width);
+        if (jb.in2) copy_rows<u32>(jb.in2, jb.out2, i, f, e, jb.width);
+      } else if (jb.esz == 8) {
+        copy_rows<unsigned long long>(jb.in, jb.out, i, f, e, jb.width);
+        if (jb.in2) copy_rows<unsigned long long>(jb.in2, jb.out2, i, f, e, jb.width);
+      } else {
+        copy_rows<unsigned char>(jb.in, jb.out, i, f, e, jb.width);
+        if (jb.in2) copy_rows<unsigned char>(jb.in2, jb.out2, i, f, e, jb.width);
+      }
     }
   }
+}
+
+static bool expand_by_words(ExpandJob const& jb)
+{
+  u32 const words = jb.esz == 4 ? jb.width : jb.esz == 8 ? 2 * jb.width : 0;
+  return words && words <= 4 && !jb.list && jb.k == 1;
 }
 
 void expand_many(std::vector<ExpandJob> const& jobs, cudaStream_t s)
 {
   std::vector<ExpandJob> live;
-  for (ExpandJob const& jb : jobs)
-    if (jb.n && jb.width && jb.k) live.push_back(jb);
-  for (size_t at = 0; at < live.size(); at += 8) {
-    ExpandJobs pack;
-    u32 cnt = (u32)std::min<size_t>(8, live.size() - at), nmax = 0;
+  for (u32 words = 0; words < 2; ++words)
+    for (ExpandJob const& jb : jobs)
+      if (jb.n && jb.width && jb.k && expand_by_words(jb) == (words != 0)) live.push_back(jb);
+  u32 const gb = tuned(TK_GATHER_BLOCK);
+  for (size_t at = 0; at < live.size(); at += EXPAND_MAX) {
+    ExpandJobs pack{};
+    u32 cnt = (u32)std::min<size_t>(EXPAND_MAX, live.size() - at), blocks = 0;
     double bytes = 0;
     for (u32 q = 0; q < cnt; ++q) {
-      pack.j[q] = live[at + q];
-      nmax = std::max(nmax, pack.j[q].n);
-      bytes += 4.0 * (pack.j[q].n + 1) + (pack.j[q].in2 ? 4.0 : 2.0) *
-          (double)pack.j[q].n * pack.j[q].width * pack.j[q].esz * pack.j[q].k;
+      ExpandJob const& jb = pack.j[q] = live[at + q];
+      bool const words = expand_by_words(jb);
+      if (!words) ++pack.nrest;
+      blocks = std::max(blocks, grid_for(jb.n, gb * (words ? EXPAND_CHUNKS : 1u)));
+      bytes += 4.0 * (jb.n + 1) + (jb.in2 ? 4.0 : 2.0) *
+          (double)jb.n * jb.width * jb.esz * jb.k;
     }
     PROBE(P_EXPAND, s, bytes);
     // a grid-stride loop over at most 16 blocks of 256 threads per SM
     // (measured: a block per 256 rows was twice as slow on the 48^3 adapt)
-    u32 const gb = tuned(TK_GATHER_BLOCK);
-    dim3 grid(std::min<u32>(grid_for(nmax, gb), 148u * 16u * 256u / gb), cnt);
-    CK(launch_kernel(k_expand_many, dim3(grid), dim3(gb), 0, s, pack));
+    blocks = std::min<u32>(blocks, 148u * 16u * 256u / gb);
+    bool const fits = blocks * cnt <= resident_blocks(k_expand_many, gb);
+    pack.together = fits ? 1u : std::max(pack.nrest, 1u);
+    dim3 grid(blocks, cnt - pack.together + 1u);
+    CK(launch_kernel(k_expand_many, grid, dim3(gb), 0, s, pack));
     CK_LAUNCH();
   }
 }

@@ -61,8 +61,8 @@ void indset_check(Mesh& m);
 void expand_scaled(void const* in, u32 const* offs, u32 k, u32 n, u32 width,
     u32 esz, void* out, cudaStream_t s);
 
-// one row expansion (as expand_scaled); expand_many runs up to eight per
-// launch. list (optional): the rows that produce anything, n of them (the
+// one row expansion (as expand_scaled); expand_many runs up to sixteen
+// per launch. list (optional): the rows that produce anything, n of them (the
 // others are skipped without reading their offsets); in2 / out2 (optional):
 // a second array copied with the same offsets
 struct ExpandJob {

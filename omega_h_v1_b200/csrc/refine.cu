@@ -703,7 +703,7 @@ static u32 refine_build(Mesh& m, EdgeSplits const& es, bool deferred, bool unifo
   u32 ntj = 0, tmost = 0;
   double tbytes = 0;
   // the survivors' connectivity and every dimension's label copies, launched
-  // together after the loop (8 jobs to a launch)
+  // together after the loop
   std::vector<ExpandJob> copies;
   for (u32 prod = 0; prod <= dim; ++prod) {
     if (!m.full && 0 < prod && prod < dim) continue;
