@@ -283,16 +283,15 @@ void Mesh::derive_model(double crease_angle)
   u32* crease = dalloc<u32>(nh, s);
   double* dots = dalloc<double>(nh, s);
   u32* amb = dalloc<u32>(nh ? nh : 1, s);
-  u32* namb = mb->dev + 24;
-  CK(cudaMemsetAsync(namb, 0, sizeof(u32), s));
+  u32* namb = mb->dev + 63;
   double cc = std::cos(crease_angle);
   if (nh) {
     CK(launch_kernel(k_hinge_class, dim3(grid_for(nh)), dim3(BLOCK), 0, s, nh, sh.offs, sh.uses, use_div(deg(D - 1, D - 2)), bside, nrm, cc - 1e-9,
         cc + 1e-9, bh, crease, dots, namb, amb));
     CK_LAUNCH();
   }
-  mb->fetch(s, 25);
-  u32 na = mb->host[24];
+  mb->fetch(s);
+  u32 na = mb->take(s, 63);
   if (na) {
     // the reference's own test for the hinges inside the band
     std::vector<u32> idx(na), val(na);
@@ -355,8 +354,7 @@ void Mesh::derive_model(double crease_angle)
     dev_free(sc, s);
     dev_free(f, s);
   }
-  u32* fail = mb->dev + 25;
-  CK(cudaMemsetAsync(fail, 0, sizeof(u32), s));
+  u32* fail = mb->dev + 62;
   for (u32 d = 1; d <= D; ++d) {
     u32 n = count(d), spd = deg(d, d - 1);
     u32 const* sod = ask_down(d, d - 1);
@@ -380,8 +378,8 @@ void Mesh::derive_model(double crease_angle)
     dev_free(sc, s);
     dev_free(roots, s);
   }
-  mb->fetch(s, 26);
-  if (mb->host[25]) {
+  mb->fetch(s);
+  if (mb->take(s, 62)) {
     for (u32 d = 0; d <= D; ++d) dev_free(cid[d], s);
     throw Failure(E_TIMEOUT, "classification: a union-find walk exceeded its bound");
   }

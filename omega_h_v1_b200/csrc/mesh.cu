@@ -488,27 +488,41 @@ __global__ void k_split_uses(u32 n, UseDiv div, u32 const* __restrict__ uses,
   dirs[j] = u - h * div.lph;
 }
 
+constexpr u32 KEPT_COUNTS = 1u << 20;  // (4 MB a stream)
+
 void up_from_down_unsorted(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* loh,
     UpAdj& out, cudaStream_t s)
 {
   u32 lph = deg(high, low);
   u32 nuses = nhighs * lph;
-  u32* cnt = dalloc<u32>((size_t)nlows + 1, s);
-  CK(cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s));
+  out.offs = dalloc<u32>((size_t)nlows + 1, s);
+  out.uses = dalloc<u32>(nuses, s);
+  // The counts of up to KEPT_COUNTS rows are the stream's kept ones, zero on
+  // entry (the fill takes them back down to zero): a memset waits for what
+  // is before it and holds back what is after, 3 us of a small mesh's
+  // derivation that its bandwidth does not explain.
+  bool const kept = nlows <= KEPT_COUNTS && !stream_captures(s);
+  u32* cnt = kept ? stream_zero_scratch(KEPT_USES, (size_t)nlows + 1, s)
+                  : dalloc<u32>((size_t)nlows + 1, s);
+  if (!kept) CK(cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s));
   if (nuses) {
     PROBE(P_UP_COUNT, s, 4.0 * nuses + 4.0 * nlows);
     CK(launch_kernel(k_count_lows, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, cnt));
     CK_LAUNCH();
   }
-  out.offs = exscan_new(cnt, nlows, s);
-  out.uses = dalloc<u32>(nuses, s);
+  try {
+    exscan_u32(cnt, out.offs, nlows, s, nullptr, nullptr);
+  } catch (...) {
+    if (kept) cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s);
+    throw;
+  }
   if (nuses) {
     PROBE(P_UP_FILL, s, 4.0 * nuses + 4.0 * (nlows + 1.0) + 4.0 * nlows + 4.0 * nuses);
     CK(launch_kernel(k_fill_uses, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, out.offs,
         cnt, out.uses));
     CK_LAUNCH();
   }
-  dev_free(cnt, s);
+  if (!kept) dev_free(cnt, s);
 }
 
 // every row in place (given pre: every row's part after its first pre[l] uses)
@@ -1693,16 +1707,19 @@ u32 const* Mesh::ask_down(u32 high, u32 low)
     down[high][low] = out;
   } else if (high == 1 && dim == 3) {
     // edges in 3D bridge the vertex star (mesh.cpp:160-168)
-    Graph const& vv = ask_star(0, dim);
+    Graph const& vv = ask_star(0, dim, false);
     u32 nv = counts[0];
     u32* degree = dalloc<u32>(nv, s);
     if (nv) {
       CK(launch_kernel(k_bridge_degree, dim3(grid_for(nv)), dim3(BLOCK), 0, s, nv, vv.offs, 0, vv.adj, degree));
       CK_LAUNCH();
     }
-    u32* bo = exscan_new(degree, nv, s);
+    u32* bo = exscan_new(degree, nv, s, mb->dev + 59);
     dev_free(degree, s);
-    u32 ne = read_u32(bo + nv, s);
+    mb->fetch(s);
+    if (mb->host[60]) dev_free(bo, s);
+    check_star(0, dim);
+    u32 ne = mb->host[59];
     u32* voe = dalloc<u32>((size_t)ne * 2, s);
     if (nv) {
       CK(launch_kernel(k_bridge_edges, dim3(grid_for(nv)), dim3(BLOCK), 0, s, nv, vv.offs, vv.adj, bo, voe));
@@ -1712,7 +1729,7 @@ u32 const* Mesh::ask_down(u32 high, u32 low)
     set_ents(1, ne, voe);
   } else {
     // sides from the element dual (mesh.cpp:169-179)
-    u32 const* du = ask_dual();
+    u32 const* du = ask_dual(false);
     u32 nel = counts[dim];
     u32 spe = deg(dim, dim - 1);
     u32* degree = dalloc<u32>(nel, s);
@@ -1720,9 +1737,12 @@ u32 const* Mesh::ask_down(u32 high, u32 low)
       CK(launch_kernel(k_bridge_degree, dim3(grid_for(nel)), dim3(BLOCK), 0, s, nel, nullptr, spe, du, degree));
       CK_LAUNCH();
     }
-    u32* bo = exscan_new(degree, nel, s);
+    u32* bo = exscan_new(degree, nel, s, mb->dev + 59);
     dev_free(degree, s);
-    u32 ns = read_u32(bo + nel, s);
+    mb->fetch(s);
+    if (mb->host[61]) dev_free(bo, s);
+    check_dual();
+    u32 ns = mb->host[59];
     u32 vps = deg(dim - 1, 0);
     u32* vos = dalloc<u32>((size_t)ns * vps, s);
     if (nel) {
@@ -1787,10 +1807,11 @@ UpAdj const& Mesh::ask_up_apart(u32 low, u32 high)
   return u;
 }
 
-Graph const& Mesh::ask_star(u32 low, u32 high)
+Graph const& Mesh::ask_star(u32 low, u32 high, bool checked)
 {
   if (have_star[low][high]) return star[low][high];
   Graph g;
+  bool pending = false;
   if (low == high) {
     u32 n = counts[low];
     g.offs = dalloc<u32>((size_t)n + 1, s);
@@ -1860,31 +1881,47 @@ Graph const& Mesh::ask_star(u32 low, u32 high)
     u32 lph = deg(high, low);
     u32* degree = dalloc<u32>(n, s);
     u32* err = mb->dev + 60;
-    CK(cudaMemsetAsync(err, 0, sizeof(u32), s));
     if (n) {
       CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.uses, loh, use_div(lph),
           nullptr, degree, nullptr, err));
       CK_LAUNCH();
     }
-    g.offs = exscan_new(degree, n, s);
+    g.offs = exscan_new(degree, n, s, mb->dev + 59);
     dev_free(degree, s);
-    g.nadj = read_u32(g.offs + n, s);
+    mb->fetch(s);
+    g.nadj = mb->host[59];
     g.adj = dalloc<u32>(g.nadj, s);
     if (n) {
       CK(launch_kernel(k_star_general, dim3(grid_for(n, STAR_WARPS)), dim3(BLOCK), 0, s, n, hl.offs, hl.uses, loh, use_div(lph), g.offs,
           nullptr, g.adj, err));
       CK_LAUNCH();
     }
-    if (read_u32(err, s)) throw Failure(E_ARG, "star wider than 256 entries");
+    pending = true;
   }
   star[low][high] = g;
   have_star[low][high] = true;
+  if (pending && checked) {
+    mb->fetch(s);
+    check_star(low, high);
+  }
   return star[low][high];
 }
 
-u32 const* Mesh::ask_dual()
+void Mesh::check_star(u32 low, u32 high)
+{
+  if (!mb->take(s, 60)) return;
+  Graph& g = star[low][high];
+  dev_free(g.offs, s);
+  dev_free(g.adj, s);
+  g = Graph();
+  have_star[low][high] = false;
+  throw Failure(E_ARG, "star wider than 256 entries");
+}
+
+u32 const* Mesh::ask_dual(bool checked)
 {
   if (dual) return dual;
+  bool pending = false;
   u32 nel = count(dim), spe = deg(dim, dim - 1);
   u32* out = dalloc<u32>((size_t)nel * spe, s);
   if (has_dim(dim - 1)) {
@@ -1898,17 +1935,28 @@ u32 const* Mesh::ask_dual()
     u32 const* voe = ask_down(dim, 0);
     UpAdj const& ev = ask_up(0, dim);
     u32* err = mb->dev + 61;
-    CK(cudaMemsetAsync(err, 0, sizeof(u32), s));
     if (nel) {
       auto k = dim == 3 ? k_dual_from_verts<3> : dim == 2 ? k_dual_from_verts<2> : k_dual_from_verts<1>;
       CK(launch_kernel(k, dim3(grid_for((u64)nel * spe)), dim3(BLOCK), 0, s, nel, voe, ev.offs,
           ev.uses, out, err));
       CK_LAUNCH();
     }
-    if (read_u32(err, s)) throw Failure(E_ARG, "vertex with more than 256 elements");
+    pending = true;
   }
   dual = out;
+  if (pending && checked) {
+    mb->fetch(s);
+    check_dual();
+  }
   return dual;
+}
+
+void Mesh::check_dual()
+{
+  if (!mb->take(s, 61)) return;
+  dev_free(dual, s);
+  dual = nullptr;
+  throw Failure(E_ARG, "vertex with more than 256 elements");
 }
 
 // ---------------------------------------------------------------------------

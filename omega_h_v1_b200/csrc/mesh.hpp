@@ -161,8 +161,12 @@ struct Mesh {
   UpAdj const& ask_up(u32 low, u32 high, bool sorted = true);
   // the same, ordered, with adj and dirs written
   UpAdj const& ask_up_apart(u32 low, u32 high);
-  Graph const& ask_star(u32 low, u32 high);
-  u32 const* ask_dual();
+  // unchecked: whether a row was past the cap comes with the caller's next
+  // read-back of the mailbox, after which it calls check_star or check_dual
+  Graph const& ask_star(u32 low, u32 high, bool checked = true);
+  u32 const* ask_dual(bool checked = true);
+  void check_star(u32 low, u32 high);
+  void check_dual();
 
   Tag* find_tag(u32 d, char const* name);
   Tag& add_tag(u32 d, u32 type, char const* name, u32 ncomps, u32 transfer,

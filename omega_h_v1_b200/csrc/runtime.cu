@@ -751,6 +751,8 @@ __global__ void k_mailbox_post(u32 const* __restrict__ src, u32 n, u32* dst, u32
   if (i == 0) *reinterpret_cast<volatile u32*>(seq_at) = seq;
 }
 
+bool stream_captures(cudaStream_t s) { return capturing(s); }
+
 u32 const* Mailbox::read(cudaStream_t s, u32 const* src, u32 nwords)
 {
   if (nwords > 16) throw Failure(E_ARG, "mailbox read: at most 16 words");
@@ -761,6 +763,13 @@ u32 const* Mailbox::read(cudaStream_t s, u32 const* src, u32 nwords)
 void Mailbox::fetch(cudaStream_t s, u32 nslots)
 {
   post(s, dev, nslots > 64 ? 64 : nslots, 0);
+}
+
+u32 Mailbox::take(cudaStream_t s, u32 slot)
+{
+  u32 const v = host[slot];
+  if (v) CK(cudaMemsetAsync(dev + slot, 0, sizeof(u32), s));
+  return v;
 }
 
 void Mailbox::post(cudaStream_t s, u32 const* src, u32 nslots, u32 at)

@@ -88,14 +88,21 @@ void exscan_jobs(ScanJob const* jobs, u32 njobs, cudaStream_t s);
 
 // Scratch kept per (device, stream, key) between calls, zeroed when made or
 // grown. stream_zero_scratch: the caller leaves it zero again after each use
-// (keys KEPT_ROWS0 and KEPT_ROWS1: the search rows' counts, which the rows'
-// fill counts back down to zero). stream_marks: entries stamped with a
+// (keys KEPT_ROWS0 and KEPT_ROWS1: the search rows' counts, KEPT_USES: the
+// upward rows', which the rows' fill counts back down to zero). stream_marks: entries stamped with a
 // generation of the (stream, key), returned in *gen (never 0) and new on
 // every call, so no entry of an earlier use passes for a mark of this one
 // (KEPT_MARKS: the products' vertices of a pass's searches; KEPT_FUSED + d:
 // the collapses' fused entities of dimension d; KEPT_SPLIT + d: a
 // refinement's split domain entities of dimension d).
-enum : u32 { KEPT_ROWS0 = 1, KEPT_ROWS1 = 2, KEPT_MARKS = 3, KEPT_FUSED = 4, KEPT_SPLIT = 8 };
+enum : u32 {
+  KEPT_ROWS0 = 1,
+  KEPT_ROWS1 = 2,
+  KEPT_MARKS = 3,
+  KEPT_FUSED = 4,
+  KEPT_SPLIT = 8,
+  KEPT_USES = 12
+};
 u32* stream_zero_scratch(u32 key, size_t words, cudaStream_t s);
 
 // blocks of `block` threads (and `smem` bytes of dynamic shared memory) of a
@@ -228,6 +235,7 @@ unsigned long long sync_count();
 // synchronisations
 void host_stats(unsigned long long* allocs, double* sync_seconds);
 void stream_sync(cudaStream_t s);
+bool stream_captures(cudaStream_t s);  // (or cannot be asked)
 // 64 bytes of pinned host memory owned by the calling host thread, for small
 // device-to-host reads (a read into pageable memory is staged by the driver)
 void* pinned_scratch();
@@ -249,9 +257,11 @@ void* pinned_scratch();
 //   16-22   coarsening build: products and survivors per dimension, kept
 //           vertices (22)
 //   20-25   swap build: products and survivors per dimension
-//   24-25   classification (derive_model)
 //   30-31   size fields (a 64-bit word)
-//   60-61   adjacency derivation error flags
+//   59      adjacency derivation: a scan's total
+//   60-63   zero but where something is to be told (take puts them back): a
+//           star or a dual past its cap (60, 61); classification: a walk
+//           past its bound, hinges too close to the angle to call (62, 63)
 // fetch: a one-block kernel stores the slots into the pinned host copy
 // (mapped into the device's address space) and then a sequence word, after
 // a system-scope fence; the host spins on that word (asking the stream for
@@ -270,6 +280,8 @@ struct Mailbox {
   void release();
   void clear(cudaStream_t s);                 // zero the device slots
   void fetch(cudaStream_t s, u32 nslots = 64);  // the first nslots slots to host
+  // after a fetch: the slot's word, its device slot zeroed where it is not
+  u32 take(cudaStream_t s, u32 slot);
   // nwords (at most 16) 32-bit words of any device array, the same way,
   // into host[READ_SLOT..]; returns that host address
   static constexpr u32 READ_SLOT = SEQ_SLOT + 16;
