@@ -692,17 +692,20 @@ void Mailbox::init(cudaStream_t s)
       v.pop_back();
     }
   }
-  if (host) {  // (its sequence goes on: the host word holds the last number)
+  if (host) {  // (its numbers go on: the words posted hold the last ones)
     clear(s);
     return;
   }
   device = d;
-  // the sequence word on a line of its own
-  CK(cudaMallocHost(&host, (SEQ_SLOT + 32) * sizeof(u32)));
-  std::memset(host, 0, (SEQ_SLOT + 32) * sizeof(u32));
+  void* h = nullptr;
+  size_t const bytes = POSTED * sizeof(u64) + (READ_SLOT + 16) * sizeof(u32);
+  CK(cudaMallocHost(&h, bytes));
+  std::memset(h, 0, bytes);
+  posted = static_cast<unsigned long long volatile*>(h);
+  host = reinterpret_cast<u32*>(static_cast<char*>(h) + POSTED * sizeof(u64));
   void* hd = nullptr;
-  CK(cudaHostGetDevicePointer(&hd, host, 0));
-  hdev = static_cast<u32*>(hd);
+  CK(cudaHostGetDevicePointer(&hd, h, 0));
+  posted_dev = static_cast<unsigned long long*>(hd);
   seq = 0;
   // (not one of the kept blocks: it outlives any stream)
   void* p = nullptr;
@@ -720,15 +723,17 @@ void Mailbox::release()
     if (v.size() < SPARE_MAX) {
       v.push_back(*this);
       host = nullptr;
-      hdev = nullptr;
+      posted = nullptr;
+      posted_dev = nullptr;
       dev = nullptr;
       return;
     }
   }
-  if (host) cudaFreeHost(host);
+  if (host) cudaFreeHost(const_cast<unsigned long long*>(posted));
   if (dev) cudaFree(dev);
   host = nullptr;
-  hdev = nullptr;
+  posted = nullptr;
+  posted_dev = nullptr;
   dev = nullptr;
 }
 
@@ -737,18 +742,16 @@ void Mailbox::clear(cudaStream_t s)
   CK(cudaMemsetAsync(dev, 0, 64 * sizeof(u32), s));
 }
 
-// dst: the host words' device address; seq_at: the sequence word's
-__global__ void k_mailbox_post(u32 const* __restrict__ src, u32 n, u32* dst, u32* seq_at,
+// Each word goes to the host with the post's number in the same 64-bit store,
+// so the host has it when it sees the number: no word waits for another, nor
+// for a fence across the bus and a flag after it (6 -> 3 us a post).
+__global__ void k_mailbox_post(u32 const* __restrict__ src, u32 n, unsigned long long* dst,
     u32 seq)
 {
   pdl_wait();
   u32 i = threadIdx.x;
-  if (i < n) {
-    reinterpret_cast<volatile u32*>(dst)[i] = src[i];
-    __threadfence_system();  // this word reaches the host before the sequence word
-  }
-  __syncthreads();
-  if (i == 0) *reinterpret_cast<volatile u32*>(seq_at) = seq;
+  if (i < n)
+    reinterpret_cast<volatile unsigned long long*>(dst)[i] = (unsigned long long)seq << 32 | src[i];
 }
 
 bool stream_captures(cudaStream_t s) { return capturing(s); }
@@ -777,19 +780,26 @@ void Mailbox::post(cudaStream_t s, u32 const* src, u32 nslots, u32 at)
   u32 const want = ++seq;
   g_syncs.fetch_add(1, std::memory_order_relaxed);
   auto t0 = std::chrono::steady_clock::now();
-  CK(launch_kernel(k_mailbox_post, dim3(1), dim3(64), 0, s, src, nslots, hdev + at,
-      hdev + SEQ_SLOT, want));
+  CK(launch_kernel(k_mailbox_post, dim3(1), dim3(64), 0, s, src, nslots, posted_dev, want));
   CK_LAUNCH();
-  volatile u32* flag = host + SEQ_SLOT;
-  for (u64 it = 1; *flag != want; ++it) {
+  u32 got = 0;
+  auto arrived = [&] {
+    for (; got < nslots; ++got) {
+      unsigned long long const w = posted[got];
+      if ((u32)(w >> 32) != want) return false;
+      host[at + got] = (u32)w;
+    }
+    return true;
+  };
+  for (u64 it = 1; !arrived(); ++it) {
     if ((it & 255) != 0) continue;
     // now and then: a failed stream ends the wait with its error; a drained
-    // stream whose word has not arrived (it should have) falls back to a
+    // stream whose words have not arrived (they should have) falls back to a
     // copy and a synchronisation
     cudaError_t st = cudaStreamQuery(s);
     if (st == cudaErrorNotReady) continue;
     CK(st);
-    if (*flag == want) break;
+    if (arrived()) break;
     CK(cudaMemcpyAsync(host + at, src, nslots * sizeof(u32), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     break;

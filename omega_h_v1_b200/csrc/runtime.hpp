@@ -262,15 +262,17 @@ void* pinned_scratch();
 //   60-63   zero but where something is to be told (take puts them back): a
 //           star or a dual past its cap (60, 61); classification: a walk
 //           past its bound, hinges too close to the angle to call (62, 63)
-// fetch: a one-block kernel stores the slots into the pinned host copy
-// (mapped into the device's address space) and then a sequence word, after
-// a system-scope fence; the host spins on that word (asking the stream for
-// errors as it waits) instead of waiting for a copy and a stream
-// synchronisation, which woke the host 6-20 us after the copy ended.
+// fetch: a one-block kernel stores each slot into pinned host memory (mapped
+// into the device's address space) with the number of the post beside it;
+// the host spins on those words (asking the stream for errors as it waits)
+// instead of waiting for a copy and a stream synchronisation, which woke the
+// host 6-20 us after the copy ended.
 struct Mailbox {
-  static constexpr u32 SEQ_SLOT = 64;  // host[SEQ_SLOT]: the last fetch's number
-  u32* host = nullptr;   // pinned, 64 slots + the sequence word
-  u32* hdev = nullptr;   // host's device address
+  static constexpr u32 POSTED = 64;
+  // pinned and mapped, a word of the last post each: its number above its value
+  unsigned long long volatile* posted = nullptr;
+  unsigned long long* posted_dev = nullptr;  // the device's address of them
+  u32* host = nullptr;   // 64 slots and the words of read
   u32* dev = nullptr;    // device, 64 slots
   u32 seq = 0;
   int device = 0;
@@ -284,9 +286,9 @@ struct Mailbox {
   u32 take(cudaStream_t s, u32 slot);
   // nwords (at most 16) 32-bit words of any device array, the same way,
   // into host[READ_SLOT..]; returns that host address
-  static constexpr u32 READ_SLOT = SEQ_SLOT + 16;
+  static constexpr u32 READ_SLOT = 64;
   u32 const* read(cudaStream_t s, u32 const* src, u32 nwords);
-  // nslots words of src into host[at..] and the sequence word after them
+  // nslots words (at most 64) of src into host[at..]
   void post(cudaStream_t s, u32 const* src, u32 nslots, u32 at);
 };
 
