@@ -347,11 +347,11 @@ def run_ours(args, world, rank, local):
                 "algorithmic_bytes_per_launch": round(avg_bytes),
                 "bytes_rule": "each array read once and each output written once per "
                               "launch: same_l and the old offsets 8(rows+1), the old "
-                              "rows' highs and directions 8 uses, the highs' new ids "
+                              "rows' uses 4 uses, the highs' new ids "
                               "4 highs, the new offsets 4(rows+1), the kept uses "
-                              "written as highs and directions 8 kept, and per use "
+                              "written 4 kept, and per use "
                               "of the entities the pass made (filled in the same "
-                              "launch) its low, the row's count and the use written 20",
+                              "launch) its low, the row's offset and count and the use written 16",
                 "traffic": traffic,
                 "dram_frac": (round(traffic / (avg_ms / 1e3) / 1e9 / peak, 4)
                               if traffic else None),

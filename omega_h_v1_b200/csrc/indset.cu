@@ -24,7 +24,7 @@ PassStats& last_pass_stats()
 // control words of the single-launch rounds (mailbox slots 44-50)
 constexpr u32 COOP_CTL_SLOT = 44, COOP_CTL_WORDS = 7;
 // (what the rounds read back: the words below; the control words' layout
-// is given at k_indset_coop)
+// is given at k_indset)
 static_assert(COOP_CTL_SLOT + COOP_CTL_WORDS == INDSET_FETCH_SLOTS, "mailbox slots");
 
 // also zeroes the control words of the rounds
