@@ -12,7 +12,9 @@
 //   dual / stars   star.cpp, dual.cpp, bridge_graph.cpp, derive_sides.cpp
 #include <cfloat>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
+#include <mutex>
 
 #include "mesh.hpp"
 
@@ -501,26 +503,31 @@ void up_from_down_unsorted(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* 
   // entry (the fill takes them back down to zero): a memset waits for what
   // is before it and holds back what is after, 3 us of a small mesh's
   // derivation that its bandwidth does not explain.
+  // Host threads may share a stream: the one that has the counts has them
+  // until its fill is launched.
+  static std::mutex counts_of[16];
+  std::unique_lock<std::mutex> hold(counts_of[((uintptr_t)s >> 4) % 16], std::defer_lock);
   bool const kept = nlows <= KEPT_COUNTS && !stream_captures(s);
+  if (kept) hold.lock();
   u32* cnt = kept ? stream_zero_scratch(KEPT_USES, (size_t)nlows + 1, s)
                   : dalloc<u32>((size_t)nlows + 1, s);
   if (!kept) CK(cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s));
-  if (nuses) {
-    PROBE(P_UP_COUNT, s, 4.0 * nuses + 4.0 * nlows);
-    CK(launch_kernel(k_count_lows, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, cnt));
-    CK_LAUNCH();
-  }
   try {
+    if (nuses) {
+      PROBE(P_UP_COUNT, s, 4.0 * nuses + 4.0 * nlows);
+      CK(launch_kernel(k_count_lows, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, cnt));
+      CK_LAUNCH();
+    }
     exscan_u32(cnt, out.offs, nlows, s, nullptr, nullptr);
+    if (nuses) {
+      PROBE(P_UP_FILL, s, 4.0 * nuses + 4.0 * (nlows + 1.0) + 4.0 * nlows + 4.0 * nuses);
+      CK(launch_kernel(k_fill_uses, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses,
+          out.offs, cnt, out.uses));
+      CK_LAUNCH();
+    }
   } catch (...) {
     if (kept) cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s);
     throw;
-  }
-  if (nuses) {
-    PROBE(P_UP_FILL, s, 4.0 * nuses + 4.0 * (nlows + 1.0) + 4.0 * nlows + 4.0 * nuses);
-    CK(launch_kernel(k_fill_uses, dim3(grid_for(nuses)), dim3(BLOCK), 0, s, loh, nuses, out.offs,
-        cnt, out.uses));
-    CK_LAUNCH();
   }
   if (!kept) dev_free(cnt, s);
 }

@@ -43,3 +43,28 @@ def test_up_counts_return_to_zero(n):
             offs, adj, dirs = m.up(low, high)
             lph = lows.size // m.count(high)
             assert np.array_equal(adj, want // lph) and np.array_equal(dirs, want % lph)
+
+
+def test_up_counts_of_threads_on_one_stream():
+    """host threads that build rows of their own meshes on the same stream"""
+    import threading
+    import omega_h_v1_b200 as G
+
+    def work(k, out):
+        x, conn, _ = G.box(k, k, 0.1)
+        lows = conn.reshape(-1)
+        want = np.argsort(lows, kind="stable")
+        ok = True
+        for _ in range(20):
+            m = G.Mesh.reduced(3, x, conn)
+            offs, adj, dirs = m.up(0, 3)
+            ok = ok and np.array_equal(adj, want // 4) and np.array_equal(dirs, want % 4)
+        out.append(ok)
+
+    out = []
+    ts = [threading.Thread(target=work, args=(k, out)) for k in (3, 5, 8, 12)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert out == [True] * 4
