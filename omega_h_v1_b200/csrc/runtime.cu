@@ -863,6 +863,15 @@ __device__ inline void scan_store4(u32* __restrict__ a, size_t gi, u32 n, bool w
   if (gi + 3 < n) a[gi + 3] = x3;
 }
 
+// a count by one, after every write this thread has made before it, for any
+// thread on the device that sees the count and fences
+__device__ __forceinline__ u32 count_released(u32* n)
+{
+  u32 was;
+  asm volatile("atom.add.release.gpu.u32 %0, [%1], 1;" : "=r"(was) : "l"(n) : "memory");
+  return was;
+}
+
 template <int SCAN_T, int SCAN_ITEMS>
 __global__ void __launch_bounds__(SCAN_T)
 k_exscan(const __grid_constant__ ScanJobs jobs, unsigned long long* status,
@@ -1001,10 +1010,14 @@ k_exscan(const __grid_constant__ ScanJobs jobs, unsigned long long* status,
     __syncthreads();
     prefix = s_prefix;
   }
-  // counted once the look-back is over; the count is looked at after the
-  // stores, so its round trip is not waited for
+  // Counted once the look-back is over; the count is looked at after the
+  // stores, so its round trip is not waited for. It is released: the tile's
+  // published prefix (this thread's exchange) has been performed when the
+  // last tile sees it, so the zeros that one writes come after it. (Without
+  // the order an exchange still under way could land on a word already
+  // zeroed, and the next scan took the prefix it left for its own.)
   u32 done = 0;
-  if (!single && threadIdx.x == 0) done = atomicAdd(&ticket_and_err[2], 1u);
+  if (!single && threadIdx.x == 0) done = count_released(&ticket_and_err[2]);
   bool const marks = newid || list || comp_newid;
 #pragma unroll
   for (u32 c = 0; c < CH; ++c) {
@@ -1037,6 +1050,8 @@ k_exscan(const __grid_constant__ ScanJobs jobs, unsigned long long* status,
   // The last tile past its look-back returns the scratch to zero for the
   // next scan on the stream: no look-back reads a status word any more.
   if (!single && warp == 0 && __shfl_sync(0xffffffffu, done, 0) == ntiles - 1) {
+    __threadfence();  // after every tile's count, and so after its exchange
+    __syncwarp();
     for (u32 t = lane; t < ntiles; t += 32) status[t] = 0ull;
     if (lane == 0) {
       ticket_and_err[0] = 0;
