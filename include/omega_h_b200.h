@@ -308,6 +308,11 @@ void osh_b200_host_stats(unsigned long long* allocs, double* sync_wait_seconds) 
    expected result), 0 if it did not, or another error code; the device
    stays usable afterwards. */
 int osh_b200_selftest_scan_wait(unsigned spin_limit) OSH_PUBLIC;
+/* self-test of how a scan's give-up is reported: the nth scan that this
+   process issues from now on (1: the next; 0: none) is recorded on its
+   stream as one whose look-back gave up, though its result is right. The
+   call that issues it has to end with OSH_B200_E_TIMEOUT. */
+void osh_b200_selftest_scan_report(unsigned nth) OSH_PUBLIC;
 /* the passes' exclusive scan over device arrays (replaces uints_exscan,
    ints.cpp:45-59, a Thrust scan there): out[0..n] with out[0] = 0 and
    out[n] the total of in[0..n), 32-bit wrap-around sums, queued on `stream`

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <chrono>
+#include <set>
 
 #include "batch.hpp"
 
@@ -1253,6 +1254,11 @@ void adapt_batch(std::vector<Mesh*> const& ms, double size_floor, double good_qu
   try {
     while (run.step(cur, st, owned)) {
     }
+    check_device_timeouts(run.s);
+    std::set<cudaStream_t> alone;  // meshes changed in place, on their own streams
+    for (u32 k = 0; k < n; ++k)
+      if (!owned[k] && st[k].res.passes && alone.insert(cur[k]->s).second)
+        check_device_timeouts(cur[k]->s);
     stream_sync(run.s);
     for (u32 k = 0; k < n; ++k) {
       res[k] = st[k].res;

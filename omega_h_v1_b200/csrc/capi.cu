@@ -1206,6 +1206,8 @@ int osh_b200_selftest_scan_wait(unsigned spin_limit)
   API_CATCH(osh::last_error())
 }
 
+void osh_b200_selftest_scan_report(unsigned nth) { osh::selftest_scan_report(nth); }
+
 int osh_b200_exscan_u32(unsigned const* in, unsigned* out, unsigned n, void* stream, int check)
 {
   API_TRY

@@ -272,6 +272,16 @@ void adapt_concurrent(std::vector<Mesh*> const& ms, AdaptParams const& ap, u32 n
       }
       r.passes = last_adapt_stats().passes;
       r.elems_in = last_adapt_stats().elems_in;
+      // (the scans after the last read-back; the stream may go back below)
+      try {
+        check_device_timeouts(m.s);
+      } catch (Failure const& f) {
+        std::lock_guard<std::mutex> g(mu);
+        if (!first_error) {
+          first_error = f.code;
+          first_msg = f.what();
+        }
+      }
       cudaStreamSynchronize(m.s);
       m.s = orig;
       {

@@ -122,6 +122,7 @@ void Mesh::own_new_stream()
 
 void Mesh::use_stream(cudaStream_t stream)
 {
+  check_device_timeouts(s);
   stream_sync(s);
   if (own_stream) give_back_stream(s);
   own_stream = false;

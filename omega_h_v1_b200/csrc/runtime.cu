@@ -698,7 +698,7 @@ void Mailbox::init(cudaStream_t s)
   }
   device = d;
   void* h = nullptr;
-  size_t const bytes = POSTED * sizeof(u64) + (READ_SLOT + 16) * sizeof(u32);
+  size_t const bytes = POSTED * sizeof(u64) + (ERR_SLOT + 1) * sizeof(u32);
   CK(cudaMallocHost(&h, bytes));
   std::memset(h, 0, bytes);
   posted = static_cast<unsigned long long volatile*>(h);
@@ -745,14 +745,27 @@ void Mailbox::clear(cudaStream_t s)
 // Each word goes to the host with the post's number in the same 64-bit store,
 // so the host has it when it sees the number: no word waits for another, nor
 // for a fence across the bus and a flag after it (6 -> 3 us a post).
-__global__ void k_mailbox_post(u32 const* __restrict__ src, u32 n, unsigned long long* dst,
-    u32 seq)
+// Word n of a post is the stream's scan error (err; null: no scan yet).
+__global__ void k_mailbox_post(u32 const* __restrict__ src, u32 n, u32 const* __restrict__ err,
+    unsigned long long* dst, u32 seq)
 {
   pdl_wait();
   u32 i = threadIdx.x;
-  if (i < n)
-    reinterpret_cast<volatile unsigned long long*>(dst)[i] = (unsigned long long)seq << 32 | src[i];
+  if (i > n) return;
+  u32 const w = i < n ? src[i] : err ? *err : 0u;
+  reinterpret_cast<volatile unsigned long long*>(dst)[i] = (unsigned long long)seq << 32 | w;
 }
+
+namespace {
+// the scratch of a stream's scans: [ticket, error, done, pad] then two words
+// per tile
+struct ScanScratch {
+  u32* p = nullptr;
+  size_t words = 0;
+};
+ScanScratch find_scan_scratch(cudaStream_t s);
+[[noreturn]] void scan_gave_up(ScanScratch const& sc, cudaStream_t s);
+}  // namespace
 
 bool stream_captures(cudaStream_t s) { return capturing(s); }
 
@@ -780,14 +793,17 @@ void Mailbox::post(cudaStream_t s, u32 const* src, u32 nslots, u32 at)
   u32 const want = ++seq;
   g_syncs.fetch_add(1, std::memory_order_relaxed);
   auto t0 = std::chrono::steady_clock::now();
-  CK(launch_kernel(k_mailbox_post, dim3(1), dim3(64), 0, s, src, nslots, posted_dev, want));
+  ScanScratch const scan = find_scan_scratch(s);
+  u32 const* err = scan.p ? scan.p + 1 : nullptr;
+  CK(launch_kernel(k_mailbox_post, dim3(1), dim3(96), 0, s, src, nslots, err, posted_dev, want));
   CK_LAUNCH();
   u32 got = 0;
+  u32& gave_up = host[ERR_SLOT];
   auto arrived = [&] {
-    for (; got < nslots; ++got) {
+    for (; got <= nslots; ++got) {
       unsigned long long const w = posted[got];
       if ((u32)(w >> 32) != want) return false;
-      host[at + got] = (u32)w;
+      (got < nslots ? host[at + got] : gave_up) = (u32)w;
     }
     return true;
   };
@@ -800,7 +816,9 @@ void Mailbox::post(cudaStream_t s, u32 const* src, u32 nslots, u32 at)
     if (st == cudaErrorNotReady) continue;
     CK(st);
     if (arrived()) break;
+    gave_up = 0;
     CK(cudaMemcpyAsync(host + at, src, nslots * sizeof(u32), cudaMemcpyDeviceToHost, s));
+    if (err) CK(cudaMemcpyAsync(&gave_up, err, sizeof(u32), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     break;
   }
@@ -808,6 +826,8 @@ void Mailbox::post(cudaStream_t s, u32 const* src, u32 nslots, u32 at)
   auto dt = std::chrono::steady_clock::now() - t0;
   g_sync_ns.fetch_add((unsigned long long)std::chrono::duration_cast<std::chrono::nanoseconds>(
       dt).count(), std::memory_order_relaxed);
+  // (what was read may come of a scan that gave up: no pass goes on with it)
+  if (gave_up) scan_gave_up(scan, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1066,10 +1086,6 @@ namespace {
 // clears it, so no scan pays for a memset. Scans on one stream run one
 // after another; each stream has its own, freed by release_stream_scratch
 // when the stream goes.
-struct ScanScratch {
-  u32* p = nullptr;
-  size_t words = 0;
-};
 std::mutex g_scan_mu;
 std::map<std::pair<int, cudaStream_t>, ScanScratch>& scan_scratches()
 {
@@ -1086,16 +1102,37 @@ u32* stream_scan_scratch(size_t words, cudaStream_t s)
   ScanScratch& sc = all[{dev, s}];
   if (sc.words < words) {
     size_t want = std::max(words, (size_t)4096);
-    if (sc.p) CK(cudaFreeAsync(sc.p, s));
-    sc.p = nullptr;
-    sc.words = 0;
     void* q = nullptr;
     CK(cudaMallocAsync(&q, want * sizeof(u32), s));
     CK(cudaMemsetAsync(q, 0, want * sizeof(u32), s));
+    u32* const old = sc.p;
     sc.p = static_cast<u32*>(q);
     sc.words = want;
+    if (old) {
+      // (a give-up that nobody has read yet stays recorded)
+      CK(cudaMemcpyAsync(sc.p + 1, old + 1, sizeof(u32), cudaMemcpyDeviceToDevice, s));
+      CK(cudaFreeAsync(old, s));
+    }
   }
   return sc.p;
+}
+
+// the stream's scan scratch (p null: it has none)
+ScanScratch find_scan_scratch(cudaStream_t s)
+{
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> g(g_scan_mu);
+  auto& all = scan_scratches();
+  auto it = all.find({dev, s});
+  return it != all.end() ? it->second : ScanScratch();
+}
+
+// a scan of the stream gave up: its scratch made anew, and the failure
+[[noreturn]] void scan_gave_up(ScanScratch const& sc, cudaStream_t s)
+{
+  CK(cudaMemsetAsync(sc.p, 0, sc.words * sizeof(u32), s));
+  throw Failure(E_TIMEOUT, "a bounded device wait gave up (scan look-back)");
 }
 }  // namespace
 
@@ -1234,6 +1271,9 @@ void launch_scan_jobs(ScanJobs const& jobs, ScanShape sh, u32* scratch, u32 spin
 }
 }  // namespace
 
+static std::atomic<u32> g_report_scan{0};
+void selftest_scan_report(u32 nth) { g_report_scan.store(nth); }
+
 void exscan_jobs(ScanJob const* jobs, u32 njobs, cudaStream_t s)
 {
   for (u32 at = 0; at < njobs; at += MAX_SCAN_JOBS) {
@@ -1255,6 +1295,10 @@ void exscan_jobs(ScanJob const* jobs, u32 njobs, cudaStream_t s)
     u32* scratch = stream_scan_scratch(4 + 2 * (size_t)pack.tile0[pack.njobs], s);
     PROBE(P_EXSCAN, s, bytes);
     launch_scan_jobs(pack, sh, scratch, SCAN_SPIN_LIMIT, s);
+    u32 left = g_report_scan.load(std::memory_order_relaxed);
+    while (left && !g_report_scan.compare_exchange_weak(left, left - 1)) {
+    }
+    if (left == 1) CK(cudaMemsetAsync(scratch + 1, 1, sizeof(u32), s));
   }
 }
 
@@ -1269,24 +1313,12 @@ void exscan_u32(u32 const* in, u32* out, u32 n, cudaStream_t s, u32* total_to, u
 // check sees its own scans' timeouts and no other stream's.
 void check_device_timeouts(cudaStream_t s)
 {
-  int dev = 0;
-  CK(cudaGetDevice(&dev));
-  u32* p = nullptr;
-  {
-    std::lock_guard<std::mutex> g(g_scan_mu);
-    auto& all = scan_scratches();
-    auto it = all.find({dev, s});
-    if (it != all.end()) p = it->second.p;
-  }
-  if (!p) return;
+  ScanScratch const sc = find_scan_scratch(s);
+  if (!sc.p) return;
   u32* h = static_cast<u32*>(pinned_scratch());
-  CK(cudaMemcpyAsync(h, p + 1, sizeof(u32), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(h, sc.p + 1, sizeof(u32), cudaMemcpyDeviceToHost, s));
   stream_sync(s);
-  if (*h) {
-    CK(cudaMemsetAsync(p + 1, 0, sizeof(u32), s));
-    stream_sync(s);
-    throw Failure(E_TIMEOUT, "a bounded device wait gave up (scan look-back)");
-  }
+  if (*h) scan_gave_up(sc, s);
 }
 
 int selftest_scan_wait(u32 spin_limit)

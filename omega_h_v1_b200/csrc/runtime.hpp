@@ -136,6 +136,8 @@ void check_device_timeouts(cudaStream_t s);
 // one scan whose second tile waits for a first tile that never publishes,
 // with a wait limit of spin_limit polls: E_TIMEOUT when the wait gave up
 int selftest_scan_wait(u32 spin_limit);
+// the nth scan issued from now on (0: none) is recorded as one that gave up
+void selftest_scan_report(u32 nth);
 
 // out[i] = !(offs[i+1] - offs[i]) scanned (uints_negate_offsets, ints.cpp:227)
 // newid (optional): out[i] where entity i is kept, INV where it is not
@@ -268,7 +270,7 @@ void* pinned_scratch();
 // instead of waiting for a copy and a stream synchronisation, which woke the
 // host 6-20 us after the copy ended.
 struct Mailbox {
-  static constexpr u32 POSTED = 64;
+  static constexpr u32 POSTED = 65;  // up to 64 words and the scans' error
   // pinned and mapped, a word of the last post each: its number above its value
   unsigned long long volatile* posted = nullptr;
   unsigned long long* posted_dev = nullptr;  // the device's address of them
@@ -287,8 +289,10 @@ struct Mailbox {
   // nwords (at most 16) 32-bit words of any device array, the same way,
   // into host[READ_SLOT..]; returns that host address
   static constexpr u32 READ_SLOT = 64;
+  static constexpr u32 ERR_SLOT = READ_SLOT + 16;
   u32 const* read(cudaStream_t s, u32 const* src, u32 nwords);
-  // nslots words (at most 64) of src into host[at..]
+  // nslots words (at most 64) of src into host[at..]; throws E_TIMEOUT where
+  // a scan of the stream has given up since the last post or check
   void post(cudaStream_t s, u32 const* src, u32 nslots, u32 at);
 };
 
