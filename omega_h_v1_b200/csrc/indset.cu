@@ -87,6 +87,21 @@ __device__ inline Key key_decided(u32 depth, bool in)
   return (in ? KEY_IN : (Key)1) + min(depth, DEPTH_MAX);
 }
 
+// A word that another warp may be writing, or waiting for: warps wait on one
+// another through these words, so they are read and written at device scope
+// (a word says all there is to know of its entity: nothing else is ordered
+// with it).
+__device__ __forceinline__ Key key_read(Key const* p)
+{
+  Key k;
+  asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(k) : "l"(p));
+  return k;
+}
+__device__ __forceinline__ void key_write(Key* p, Key k)
+{
+  asm volatile("st.relaxed.gpu.u64 [%0], %1;" ::"l"(p), "l"(k));
+}
+
 // neighbours of an upward entry: 1 (a vertex's edge), 3 or 6 (an edge's
 // triangle or tet, the edge itself among them); NB: those a lane takes at once
 template <u32 PER>
@@ -142,7 +157,7 @@ __device__ inline Walk walk_neighbors(Nbrs const& g, u32 i, Key mykey, u32 lg, u
     load_neighbors<G, PER>(g, i, j, re, o);
 #pragma unroll
     for (u32 k = 0; k < NB; ++k)
-      ko[k] = o[k] == INV ? 0ull : FRESH ? __ldcg(&keys[o[k]]) : __ldca(&keys[o[k]]);
+      ko[k] = o[k] == INV ? 0ull : FRESH ? key_read(&keys[o[k]]) : __ldca(&keys[o[k]]);
 #pragma unroll
     for (u32 k = 0; k < NB; ++k) {
       if (!ko[k]) continue;
@@ -314,7 +329,7 @@ __device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list,
     if (!r.in && r.blocker != INV) return r.blocker;
     if (lg == 0) {
       Key const k = key_decided(r.depth + 1, !r.in);
-      __stcg(&keys[i], k);
+      key_write(&keys[i], k);
       settled(i, k);
     }
     if (!r.in && r.worse) {
@@ -327,13 +342,13 @@ __device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list,
         load_neighbors<G, PER>(g, i, j, re, o);
         Key ko[NB];
 #pragma unroll
-        for (u32 k = 0; k < NB; ++k) ko[k] = o[k] != INV ? __ldcg(&keys[o[k]]) : 0ull;
+        for (u32 k = 0; k < NB; ++k) ko[k] = o[k] != INV ? key_read(&keys[o[k]]) : 0ull;
 #pragma unroll
         for (u32 k = 0; k < NB; ++k) {
           if (exact && ko[k])  // (the smaller depth stays)
             atomicMin(&keys[o[k]], no);
           else if (key_undecided(ko[k]))
-            __stcg(&keys[o[k]], no);
+            key_write(&keys[o[k]], no);
         }
       }
     }
@@ -358,7 +373,7 @@ __device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list,
     // (one lane's reading for the group: a word may change between two)
 #pragma unroll
     for (u32 k = 0; k < ITEMS_AHEAD; ++k)
-      key[k] = lg == 0 && it[k] != INV ? __ldcg(&keys[it[k]]) : 0ull;
+      key[k] = lg == 0 && it[k] != INV ? key_read(&keys[it[k]]) : 0ull;
 #pragma unroll
     for (u32 k = 0; k < ITEMS_AHEAD; ++k) {
       Key const mine = __shfl_sync(FULL, key[k], gbase);
@@ -378,8 +393,8 @@ __device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list,
       Key mine = 0, ko = 0;
       if (q + lane < todo) {
         e = *slot(q + lane);
-        mine = __ldcg(&keys[e.x]);
-        ko = __ldcg(&keys[e.y]);
+        mine = key_read(&keys[e.x]);
+        ko = key_read(&keys[e.y]);
       }
       bool const have = e.y != INV;
       bool const put_out = have && !key_undecided(mine);
@@ -391,7 +406,7 @@ __device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list,
       if (put_out || (ready && !again)) {
         if (!put_out) {
           mine = key_decided(key_depth(ko) + 1, false);
-          __stcg(&keys[e.x], mine);
+          key_write(&keys[e.x], mine);
         }
         settled(e.x, mine);
       }
@@ -409,7 +424,7 @@ __device__ inline u32 decide_listed(Nbrs const& g, u32 const* __restrict__ list,
         u32 i = 0, blocker = INV;
         if (b + gi < cnt) {
           i = item[b + gi];
-          Key const k = __shfl_sync(gmask, lg == 0 ? __ldcg(&keys[i]) : 0ull, gbase);
+          Key const k = __shfl_sync(gmask, lg == 0 ? key_read(&keys[i]) : 0ull, gbase);
           blocker = walk(i, k, true);
         }
         append(i, blocker);
