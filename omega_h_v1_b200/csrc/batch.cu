@@ -761,6 +761,17 @@ constexpr u64 KEEP_UNION_ELEMS = 1u << 26;
 // quarter, 23 at an eighth, 22 never; 37 split after every pass.)
 constexpr u64 IDLE_ELEMS = 1000000;
 
+// Whether a mesh's global numbers are its caller's. They decide ties between
+// equal qualities, and a pass that changes the mesh puts its local indices in
+// their place (a swap leaves the vertices'), so they have to be kept for as
+// long as the mesh waits.
+bool own_numbers(Mesh const& m)
+{
+  for (u32 d = 0; d <= m.dim; ++d)
+    if (m.globals[d] && !m.globals_iota[d]) return true;
+  return false;
+}
+
 // the point of mesh_adapt's loop a pass acts on: refine (the quality floor
 // is read before the first), coarsen, shape
 u32 phase_of(u32 state) { return state == ST_INIT ? (u32)ST_REFINE : state; }
@@ -855,10 +866,14 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
   }
   // Meshes held apart are gathered by the point they are at, with the kept
   // unions at that point (a union of unions): consecutive items of at most
-  // max_union_elems elements. Kept unions alone stay as they are.
+  // max_union_elems elements. Kept unions alone stay as they are. Meshes with
+  // global numbers of their own are gathered by themselves, for one pass; a
+  // shape step, which may keep the vertices', takes each alone.
   list_residents();
   std::vector<std::pair<u32, u32>> alone;  // (phase, mesh): gathered with nothing
-  for (u32 p : {ST_REFINE, ST_COARSEN, ST_SHAPE}) {
+  for (u32 g = 0; g < 6; ++g) {
+    u32 const p = g % 3 == 0 ? ST_REFINE : g % 3 == 1 ? ST_COARSEN : ST_SHAPE;
+    bool const numbered = g >= 3;
     struct Item {
       Mesh* m;
       int r;  // a kept union's index, or -1: mesh k
@@ -868,12 +883,17 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
     std::vector<Item> items;
     bool apart = false;
     for (u32 k = 0; k < n; ++k)
-      if (!st[k].in && st[k].state < ST_DONE && phase_of(st[k].state) == p) {
+      if (!st[k].in && st[k].state < ST_DONE && phase_of(st[k].state) == p &&
+          own_numbers(*ms[k]) == numbered) {
+        if (numbered && p == ST_SHAPE) {
+          alone.push_back({p, k});
+          continue;
+        }
         items.push_back({ms[k], -1, k, ms[k]->count(ms[k]->dim)});
         apart = true;
       }
     if (!apart) continue;
-    for (size_t q = 0; q < rs.size(); ++q)
+    for (size_t q = 0; q < rs.size() && !numbered; ++q)
       if (phase_of_members(members[q]) == p)
         items.push_back({rs[q]->u, (int)q, 0, rs[q]->u->count(rs[q]->u->dim)});
     for (size_t at = 0; at < items.size();) {
@@ -900,6 +920,7 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
       r->u = concat_meshes(parts, s);
       stream_sync(s);
       bs.unions += 1;
+      r->once = numbered;
       r->dirty.assign(r->u->nseg, 0);
       r->elems.assign(r->u->nseg, 0);
       u32 seg = 0;
@@ -1023,7 +1044,9 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
     pass(*rs[q]->ctl, phase_of_members(members[q]), members[q], segs, rs[q].get());
     for (u32 k : members[q])
       if (st[k].state >= ST_DONE) done.push_back(k);
-    if (!done.empty() && (hand_back || done.size() == members[q].size()))
+    if (rs[q]->once)
+      take_out(*rs[q], members[q]);
+    else if (!done.empty() && (hand_back || done.size() == members[q].size()))
       take_out(*rs[q], done);
   }
   return any_live();

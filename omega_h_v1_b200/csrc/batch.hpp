@@ -114,6 +114,9 @@ struct Resident {
   std::unique_ptr<UnionCtl> ctl;
   std::vector<char> dirty;
   std::vector<u32> elems;  // each segment's elements when last counted
+  // split after its first pass: its meshes' global numbers are their own (a
+  // pass gives the whole union new ones, also of the meshes it leaves alone)
+  bool once = false;
   Resident() = default;
   Resident(Resident const&) = delete;
   Resident& operator=(Resident const&) = delete;
