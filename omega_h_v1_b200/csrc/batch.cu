@@ -829,6 +829,12 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
     for (u32 k : mk) p = std::min(p, phase_of(st[k].state));
     return p;
   };
+  // whether every live mesh of a union is at point p
+  auto all_at = [&](std::vector<u32> const& mk, u32 p) {
+    for (u32 k : mk)
+      if (st[k].state < ST_DONE && phase_of(st[k].state) != p) return false;
+    return phase_of_members(mk) == p;
+  };
   // meshes out of the union that holds them
   auto take_out = [&](Resident& r, std::vector<u32> const& mk) {
     double t = wall_s();
@@ -865,7 +871,10 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
       take_out(r, members[q]);
   }
   // Meshes held apart are gathered by the point they are at, with the kept
-  // unions at that point (a union of unions): consecutive items of at most
+  // unions all of whose meshes are at that point (a union of unions; one with
+  // meshes further on is left alone, as those would wait for every newcomer:
+  // jobs that came one a step to a server were all held back until no more
+  // came, 49 steps instead of 9): consecutive items of at most
   // max_union_elems elements. Kept unions alone stay as they are. Meshes with
   // global numbers of their own are gathered by themselves, for one pass; a
   // shape step, which may keep the vertices', takes each alone.
@@ -894,7 +903,7 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
       }
     if (!apart) continue;
     for (size_t q = 0; q < rs.size() && !numbered; ++q)
-      if (phase_of_members(members[q]) == p)
+      if (all_at(members[q], p))
         items.push_back({rs[q]->u, (int)q, 0, rs[q]->u->count(rs[q]->u->dim)});
     for (size_t at = 0; at < items.size();) {
       size_t end = at;
