@@ -852,11 +852,19 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
         owned[k] = 1;
       }
       st[k].in.reset();
+      st[k].left = hold;
     }
     bs.secs_split += wall_s() - t;
   };
-  // unions that are done, too large to keep, or mostly waiting: split
+  // whether segments of a union belong to meshes that left it
+  auto some_left = [&](size_t q) { return members[q].size() < rs[q]->u->nseg; };
+  // unions that are done, too large to keep, or mostly waiting: split; so are
+  // those that hold segments of meshes that left them, where others would
+  // join (a union of unions never holds such segments) or wait for the room
   list_residents();
+  bool come[ST_DONE] = {};  // meshes held apart at each point
+  for (u32 k = 0; k < n; ++k)
+    if (!st[k].in && st[k].state < ST_DONE) come[phase_of(st[k].state)] = true;
   for (size_t q = 0; q < rs.size(); ++q) {
     Resident& r = *rs[q];
     u32 const p = phase_of_members(members[q]);
@@ -866,7 +874,8 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
     for (u32 k : members[q])
       if (phase_of(st[k].state) == p) acting += r.elems[st[k].seg];
     if (p >= ST_DONE || total > KEEP_UNION_ELEMS ||
-        (max_union_elems && total > max_union_elems && members[q].size() > 1) ||
+        (max_union_elems && total > max_union_elems && r.u->nseg > 1) ||
+        (some_left(q) && (drop_left || (come[p] && all_at(members[q], p)))) ||
         (8 * acting < counted_elems && counted_elems - acting > IDLE_ELEMS))
       take_out(r, members[q]);
   }
@@ -903,7 +912,7 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
       }
     if (!apart) continue;
     for (size_t q = 0; q < rs.size() && !numbered; ++q)
-      if (all_at(members[q], p))
+      if (all_at(members[q], p) && !some_left(q))
         items.push_back({rs[q]->u, (int)q, 0, rs[q]->u->count(rs[q]->u->dim)});
     for (size_t at = 0; at < items.size();) {
       size_t end = at;

@@ -79,6 +79,9 @@ struct SegState {
   // (none: the mesh is held apart)
   std::shared_ptr<Resident> in;
   u32 seg = 0;
+  // the union it was last taken out of, which still holds its segment while
+  // other meshes are in it
+  std::weak_ptr<Resident> left;
 };
 
 // per-segment control arrays of a union and the host copies of their results
@@ -140,6 +143,8 @@ struct GroupRunner {
   // split a mesh out at the end of the step its loop ends in (a server's
   // jobs leave then); otherwise when the last mesh of its union is done
   bool hand_back = false;
+  // split every union that holds segments of meshes that left it
+  bool drop_left = false;
   // one step for every live mesh; ms[k] is replaced (and owned[k] set) when
   // it is split out of a union, the previous ms[k] deleted if it was owned
   // (null, not owned, while st[k].in holds the mesh). Returns whether any

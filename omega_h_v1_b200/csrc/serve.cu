@@ -88,8 +88,11 @@ struct Server {
   GroupRunner run;
   std::map<u32, std::unique_ptr<ServeJob>> jobs;
   std::deque<ServeJob*> queue;
-  // resident jobs, each mesh held apart and regrouped per pass
+  // resident jobs: their meshes are in unions kept between passes, or apart
   std::vector<ServeJob*> active;
+  // bytes of jobs handed back whose union still holds their segment: reserved
+  // until that union is gone
+  std::vector<std::pair<std::weak_ptr<Resident>, unsigned long long>> held;
   std::vector<Mesh*> ms;
   std::vector<SegState> st;
   std::vector<char> owned;
@@ -158,16 +161,31 @@ struct Server {
     }
   }
 
+  void release_held()
+  {
+    size_t w = 0;
+    for (auto& h : held)
+      if (h.first.expired())
+        reserved -= h.second;
+      else
+        held[w++] = h;
+    held.resize(w);
+  }
+
   void admit()
   {
     cudaStream_t s = run.s;
+    run.drop_left = false;
     for (;;) {
       ServeJob* j = nullptr;
       {
         std::lock_guard<std::mutex> g(mu);
         if (queue.empty()) break;
         j = queue.front();
-        if (!active.empty() && reserved + j->est_bytes > budget) break;
+        if (!active.empty() && reserved + j->est_bytes > budget) {
+          run.drop_left = true;  // (a step later there is room, where that makes any)
+          break;
+        }
         queue.pop_front();
       }
       reserved += j->est_bytes;
@@ -244,7 +262,7 @@ struct Server {
           j->finished = true;
           j->t_done = t;
         }
-        reserved -= j->est_bytes;
+        held.push_back({st[k].left, j->est_bytes});
         continue;
       }
       active[w] = active[k];
@@ -257,6 +275,7 @@ struct Server {
     ms.resize(w);
     st.resize(w);
     owned.resize(w);
+    release_held();
     secs_retire += now_s() - t_c;
     std::lock_guard<std::mutex> g(mu);
     publish();
