@@ -134,8 +134,10 @@ struct Resident {
 // are at the same point of their loop into unions of at most max_union_elems
 // current elements (0 = no limit) and runs that pass over each union, one
 // launch per stage. A union is kept between passes, with the adjacency they
-// carry; its meshes that got further wait for the others. Once most of its
-// elements wait (IDLE_ELEMS) its meshes are split out and gathered anew.
+// carry. In a batch its meshes that got further wait for the others; where
+// meshes are handed back one by one (hand_back), a step runs a pass for every
+// point of the loop some mesh of a union is at. Once most of its elements
+// wait (IDLE_ELEMS) its meshes are split out and gathered anew.
 struct GroupRunner {
   AdaptParams ap{1.0 / 3.0, 0.3, 4, 50};
   unsigned long long max_union_elems = 0;

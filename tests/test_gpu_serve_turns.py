@@ -9,16 +9,16 @@ ARGS = (1 / 3., 0.3, 4, 50)
 N, C, JOBS = 5, 0.6, 48
 
 
-def _submit(sv, seed):
+def _submit(sv, seed, n=N, c=C, pert=0.1):
     import omega_h_v1_b200 as G
-    coords, conn, _ = G.box(N, seed, 0.1)
-    return sv.submit(coords, conn, np.full(coords.size // 3, C / N))
+    coords, conn, _ = G.box(n, seed, pert)
+    return sv.submit(coords, conn, np.full(coords.size // 3, c / n))
 
 
-def _steps_alone(seed):
+def _steps_alone(seed, **kw):
     import omega_h_v1_b200 as G
     sv = G.Server(*ARGS, 8 << 30)
-    _submit(sv, seed)
+    _submit(sv, seed, **kw)
     steps = 1
     while sv.step():
         steps += 1
@@ -47,7 +47,17 @@ def test_a_job_does_not_wait_for_later_arrivals():
         step += 1
     assert len(took) == JOBS
     sv.close()
-    # a union's members are through a point of the loop together, and those
-    # that join it do so before its first member is past refinement
-    assert max(took.values()) <= 2 * alone + 2, (alone, took)
-    assert len(arrived) >= JOBS - 2 * alone - 2
+    assert max(took.values()) <= alone + 1, (alone, took)
+    assert len(arrived) >= JOBS - alone - 1
+
+
+def test_a_job_does_not_wait_for_a_slow_one():
+    import omega_h_v1_b200 as G
+    alone = _steps_alone(0, n=6, c=1.0)
+    sv = G.Server(*ARGS, 8 << 30)
+    a = _submit(sv, 0, n=6, c=1.0)
+    b = _submit(sv, 1, n=6, c=1.0, pert=0.3)   # as many passes as a job may take
+    for _ in range(alone):
+        sv.step()
+    assert sv.job_info(a)["finished"] and not sv.job_info(b)["finished"]
+    sv.close()
