@@ -11,9 +11,9 @@
 #include <map>
 #include <mutex>
 #include <tuple>
-#include <unordered_map>
 #include <vector>
 
+#include "kept_blocks.hpp"
 #include "runtime.hpp"
 
 namespace osh {
@@ -382,67 +382,28 @@ static void setup_pool()
   });
 }
 
-// Blocks of up to BLOCK_MAX bytes that dev_free gets back are kept for the
-// next dev_alloc on the same stream, by size class (four to an octave), up
-// to KEEP_MAX bytes a stream: a pass on a small mesh makes and drops some
-// forty arrays, and a call into the driver's pool for each took longer than
-// its kernels (0.6 to 1.9 us a call, 735 calls in a 6^3 adapt of 188
-// launches). Order is the stream's, as the driver's pool keeps it. The
-// blocks go back to that pool when the stream's scratch is released
-// (release_stream_scratch), when an allocation fails, and past KEEP_MAX. A
-// stream under capture goes to the driver's pool, whose calls are captured.
 namespace {
-constexpr size_t BLOCK_MAX = 4u << 20, KEEP_MAX = 256u << 20;
-constexpr u32 BLOCK_CLASSES = 1 + 13 * 4;  // 512 bytes; then 2^9 .. 2^22 in quarters
-
-u32 block_class(size_t bytes, size_t* rounded)
-{
-  if (bytes <= 512) {
-    *rounded = 512;
-    return 0;
-  }
-  u32 const l = 63 - (u32)__builtin_clzll((unsigned long long)(bytes - 1));  // >= 9
-  size_t const base = (size_t)1 << l, step = base / 4;
-  u32 const k = (u32)((bytes - 1 - base) / step);
-  *rounded = base + (k + 1) * step;
-  return 1 + (l - 9) * 4 + k;
-}
-
-size_t class_bytes(u32 c)
-{
-  if (!c) return 512;
-  size_t const base = (size_t)1 << (9 + (c - 1) / 4);
-  return base + ((c - 1) % 4 + 1) * (base / 4);
-}
-
-struct KeptBlocks {
-  std::vector<void*> free_of[BLOCK_CLASSES];
-  size_t bytes = 0;
-};
-
-struct BlockTable {
-  std::mutex mu;
-  std::map<std::pair<int, cudaStream_t>, KeptBlocks> kept;
-  std::unordered_map<void*, std::pair<int, u32>> made;  // (device, class) of each block
-  size_t kept_bytes[64] = {};
-};
 BlockTable& blocks()
 {
   static auto* t = new BlockTable();  // lives to exit
   return *t;
 }
 
-// (the table's lock held) every kept block of a stream back to the pool
-void drop_kept_blocks(BlockTable& t, std::map<std::pair<int, cudaStream_t>, KeptBlocks>::iterator it)
-{
-  for (auto& list : it->second.free_of)
-    for (void* p : list) {
-      t.made.erase(p);
-      cudaFreeAsync(p, it->first.second);
-    }
-  t.kept_bytes[it->first.first & 63] -= it->second.bytes;
-  t.kept.erase(it);
-}
+// the device's memory pool
+struct DriverPool {
+  bool full = false;
+  void* alloc(size_t bytes, void* s)
+  {
+    void* p = nullptr;
+    cudaError_t const e = cudaMallocAsync(&p, bytes, static_cast<cudaStream_t>(s));
+    if (e == cudaSuccess) return p;
+    cudaGetLastError();
+    full = e == cudaErrorMemoryAllocation;
+    return nullptr;
+  }
+  void free(void* p, void* s) { cudaFreeAsync(p, static_cast<cudaStream_t>(s)); }
+  void wait(void* s) { cudaStreamSynchronize(static_cast<cudaStream_t>(s)); }
+};
 
 bool capturing(cudaStream_t s)
 {
@@ -508,10 +469,26 @@ void give_back_stream(cudaStream_t s)
   cudaStreamDestroy(s);
 }
 
+// from the pool, with the blocks kept on the device given back to it where
+// that is needed (not under capture, where they could not be); E_NOMEM
+static void* pool_alloc(size_t bytes, cudaStream_t s)
+{
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  DriverPool pool;
+  void* p = capturing(s) ? pool.alloc(bytes, s) : alloc_or_drop(blocks(), pool, dev, bytes, s);
+  if (!p) {
+    char buf[128];
+    snprintf(buf, sizeof(buf), "device allocation of %zu bytes failed", bytes);
+    throw Failure(E_NOMEM, buf);
+  }
+  return p;
+}
+
+// A stream under capture goes to the driver's pool, whose calls are captured.
 void* dev_alloc(size_t bytes, cudaStream_t s)
 {
   setup_pool();
-  void* p = nullptr;
   if (bytes < 16) bytes = 16;
   g_allocs.fetch_add(1, std::memory_order_relaxed);
   int dev = 0;
@@ -521,38 +498,13 @@ void* dev_alloc(size_t bytes, cudaStream_t s)
   u32 cls = 0;
   if (small) {
     cls = block_class(bytes, &bytes);
-    std::lock_guard<std::mutex> g(t.mu);
-    auto it = t.kept.find({dev, s});
-    if (it != t.kept.end() && !it->second.free_of[cls].empty()) {
-      p = it->second.free_of[cls].back();
-      it->second.free_of[cls].pop_back();
-      it->second.bytes -= bytes;
-      t.kept_bytes[dev & 63] -= bytes;
-      return p;
-    }
+    if (void* p = t.take(dev, s, cls)) return p;
   }
-  cudaError_t e = cudaMallocAsync(&p, bytes, s);
-  if (e == cudaErrorMemoryAllocation) {
-    // once more with what this stream keeps
-    cudaGetLastError();
-    {
-      std::lock_guard<std::mutex> g(t.mu);
-      auto it = t.kept.find({dev, s});
-      if (it != t.kept.end()) drop_kept_blocks(t, it);
-    }
-    e = cudaMallocAsync(&p, bytes, s);
-  }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    char buf[128];
-    snprintf(buf, sizeof(buf), "device allocation of %zu bytes failed", bytes);
-    throw Failure(E_NOMEM, buf);
-  }
-  std::lock_guard<std::mutex> g(t.mu);
+  void* p = pool_alloc(bytes, s);
   if (small)
-    t.made[p] = {dev, cls};
+    t.made(p, dev, cls);
   else
-    t.made.erase(p);
+    t.not_a_block(p);
   return p;
 }
 
@@ -561,9 +513,9 @@ void pool_reserve(unsigned long long bytes)
   setup_pool();
   if (!bytes) return;
   void* p = nullptr;
-  cudaError_t e = cudaMallocAsync(&p, bytes, 0);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
+  try {
+    p = pool_alloc(bytes, 0);
+  } catch (Failure const&) {
     throw Failure(E_NOMEM, "could not reserve the requested device memory");
   }
   CK(cudaFreeAsync(p, 0));
@@ -584,11 +536,7 @@ void pool_stats(unsigned long long* reserved, unsigned long long* used,
   CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &h));
   if (reserved) *reserved = r;
   // the blocks kept for the next allocations are not in use
-  {
-    BlockTable& t = blocks();
-    std::lock_guard<std::mutex> g(t.mu);
-    u -= std::min<unsigned long long>(u, t.kept_bytes[dev & 63]);
-  }
+  u -= std::min<unsigned long long>(u, blocks().kept_bytes(dev));
   if (used) *used = u;
   if (used_high) *used_high = h;
   if (reset_high) {
@@ -599,26 +547,7 @@ void pool_stats(unsigned long long* reserved, unsigned long long* used,
 
 void dev_free(void* p, cudaStream_t s)
 {
-  if (!p) return;
-  BlockTable& t = blocks();
-  bool const keep = !capturing(s);
-  {
-    std::lock_guard<std::mutex> g(t.mu);
-    auto it = t.made.find(p);
-    if (it != t.made.end()) {
-      int const dev = it->second.first;
-      u32 const cls = it->second.second;
-      size_t const bytes = class_bytes(cls);
-      KeptBlocks& k = t.kept[{dev, s}];
-      if (keep && k.bytes + bytes <= KEEP_MAX) {
-        k.free_of[cls].push_back(p);
-        k.bytes += bytes;
-        t.kept_bytes[dev & 63] += bytes;
-        return;
-      }
-      t.made.erase(it);
-    }
-  }
+  if (!p || blocks().keep(p, s, !capturing(s))) return;
   CK(cudaFreeAsync(p, s));
 }
 
@@ -1102,8 +1031,7 @@ u32* stream_scan_scratch(size_t words, cudaStream_t s)
   ScanScratch& sc = all[{dev, s}];
   if (sc.words < words) {
     size_t want = std::max(words, (size_t)4096);
-    void* q = nullptr;
-    CK(cudaMallocAsync(&q, want * sizeof(u32), s));
+    void* q = pool_alloc(want * sizeof(u32), s);
     CK(cudaMemsetAsync(q, 0, want * sizeof(u32), s));
     u32* const old = sc.p;
     sc.p = static_cast<u32*>(q);
@@ -1161,13 +1089,14 @@ KeptScratch& kept_scratch(u32 key, size_t words, cudaStream_t s)
   KeptScratch& sc = all[{dev, s, key}];
   if (sc.words < words) {
     size_t want = std::max(words + words / 4, (size_t)4096);
-    if (sc.p) CK(cudaFreeAsync(sc.p, s));
-    void* q = nullptr;
-    CK(cudaMallocAsync(&q, want * sizeof(u32), s));
+    // (the old one stays in place until there is a new one)
+    void* q = pool_alloc(want * sizeof(u32), s);
     CK(cudaMemsetAsync(q, 0, want * sizeof(u32), s));
+    u32* const old = sc.p;
     sc.p = static_cast<u32*>(q);
     sc.words = want;
     sc.gen = 0;
+    if (old) CK(cudaFreeAsync(old, s));
   }
   return sc;
 }
@@ -1195,12 +1124,7 @@ void release_stream_scratch(cudaStream_t s)
 {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
-  {
-    BlockTable& t = blocks();
-    std::lock_guard<std::mutex> g(t.mu);
-    auto it = t.kept.find({dev, s});
-    if (it != t.kept.end()) drop_kept_blocks(t, it);
-  }
+  for (auto const& b : blocks().drop(dev, s)) cudaFreeAsync(b.p, s);
   {
     std::lock_guard<std::mutex> g(g_scan_mu);
     auto& all = scan_scratches();
