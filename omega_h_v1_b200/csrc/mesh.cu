@@ -41,6 +41,7 @@ Mesh::Mesh(u32 d, bool f, bool p, cudaStream_t stream,
     mb = std::shared_ptr<Mailbox>(new Mailbox(), release_mailbox);
     mb->init(s);
   }
+  if (!own_stream) begin_stream_use(s);
 }
 
 Mesh::~Mesh()
@@ -52,7 +53,10 @@ Mesh::~Mesh()
   // (a mailbox goes back with no kernel pending that writes it)
   if (own_stream || mb.use_count() == 1) cudaStreamSynchronize(s);
   mb.reset();
-  if (own_stream) give_back_stream(s);
+  if (own_stream)
+    give_back_stream(s);
+  else
+    end_stream_use(s);
 }
 
 Mesh* Mesh::spawn() const
@@ -114,8 +118,10 @@ void Mesh::own_new_stream()
 {
   stream_sync(s);
   if (own_stream) return;
+  cudaStream_t const was = s;
   s = take_stream();
   own_stream = true;
+  end_stream_use(was);
   mb = std::shared_ptr<Mailbox>(new Mailbox(), release_mailbox);
   mb->init(s);
 }
@@ -124,9 +130,13 @@ void Mesh::use_stream(cudaStream_t stream)
 {
   check_device_timeouts(s);
   stream_sync(s);
-  if (own_stream) give_back_stream(s);
+  if (own_stream)
+    give_back_stream(s);
+  else
+    end_stream_use(s);
   own_stream = false;
   s = stream;
+  begin_stream_use(s);
 }
 
 void Mesh::clear_contents()

@@ -419,6 +419,7 @@ constexpr size_t SPARE_MAX = 64;
 struct Spares {
   std::mutex mu;
   std::map<cudaStream_t, int> made_on;  // the device of each stream made here
+  std::map<cudaStream_t, u32> users;    // the meshes on each caller's stream
   std::map<int, std::vector<cudaStream_t>> streams;
   std::map<int, std::vector<Mailbox>> boxes;
 };
@@ -467,6 +468,29 @@ void give_back_stream(cudaStream_t s)
     }
   }
   cudaStreamDestroy(s);
+}
+
+void begin_stream_use(cudaStream_t s)
+{
+  if (!s || s == cudaStreamLegacy) return;
+  Spares& sp = spares();
+  std::lock_guard<std::mutex> g(sp.mu);
+  if (!sp.made_on.count(s)) ++sp.users[s];
+}
+
+void end_stream_use(cudaStream_t s)
+{
+  if (!s || s == cudaStreamLegacy) return;
+  Spares& sp = spares();
+  {
+    std::lock_guard<std::mutex> g(sp.mu);
+    auto it = sp.users.find(s);
+    if (it == sp.users.end() || --it->second) return;
+    sp.users.erase(it);
+  }
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  for (auto const& b : blocks().drop(dev, s)) cudaFreeAsync(b.p, s);
 }
 
 // from the pool, with the blocks kept on the device given back to it where
@@ -547,7 +571,9 @@ void pool_stats(unsigned long long* reserved, unsigned long long* used,
 
 void dev_free(void* p, cudaStream_t s)
 {
-  if (!p || blocks().keep(p, s, !capturing(s))) return;
+  if (!p) return;
+  // (one handle names every thread's own default stream: nothing kept there)
+  if (blocks().keep(p, s, s != cudaStreamPerThread && !capturing(s))) return;
   CK(cudaFreeAsync(p, s));
 }
 

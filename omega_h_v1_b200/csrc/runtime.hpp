@@ -124,6 +124,10 @@ void release_stream_scratch(cudaStream_t s);
 // released; its work may still run: the next user's comes after it)
 cudaStream_t take_stream();
 void give_back_stream(cudaStream_t s);
+// a mesh on a stream that is not its own, from its making (or its move there)
+// to its end: the blocks kept for a caller's stream go with its last mesh
+void begin_stream_use(cudaStream_t s);
+void end_stream_use(cudaStream_t s);
 u32* stream_marks(u32 key, size_t words, cudaStream_t s, u32* gen);
 
 // The same scan with caller-provided scratch of at least
