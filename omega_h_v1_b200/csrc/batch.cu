@@ -675,11 +675,11 @@ UnionCtl::~UnionCtl()
   cudaStream_t s = u.s;
   u.ctl = nullptr;
   cudaStreamSynchronize(s);
-  dev_free(active, s);
-  dev_free(floor, s);
-  dev_free(selected, s);
-  dev_free(elems, s);
-  dev_free(minkey, s);
+  dev_drop(active, s);
+  dev_drop(floor, s);
+  dev_drop(selected, s);
+  dev_drop(elems, s);
+  dev_drop(minkey, s);
   cudaFreeHost(h_u32);
   cudaFreeHost(h_key);
 }

@@ -126,7 +126,7 @@ struct DevOut {
   cudaStream_t s;
   DevOut(T* h, size_t count, cudaStream_t st) : d(osh::dalloc<T>(count, st)), host(h), n(count), s(st) {}
   void back() { CK(cudaMemcpyAsync(host, d, n * sizeof(T), cudaMemcpyDeviceToHost, s)); }
-  ~DevOut() { osh::dev_free(d, s); }
+  ~DevOut() { osh::dev_drop(d, s); }
 };
 }  // namespace
 

@@ -680,6 +680,9 @@ __device__ inline void load_corners(u32 const* __restrict__ voe, double const* _
 
 void* dev_alloc(size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
+// the same in a destructor, which may run while a failure unwinds: an error
+// (a stream whose capture failed, a device in error) is let go
+void dev_drop(void* p, cudaStream_t s) noexcept;
 
 template <class T>
 T* dalloc(size_t n, cudaStream_t s)

@@ -143,7 +143,7 @@ struct Counter {
     d = dalloc<u32>(1, s);
     CK(cudaMemsetAsync(d, 0, sizeof(u32), s));
   }
-  ~Counter() { dev_free(d, s); }
+  ~Counter() { dev_drop(d, s); }
   void zero() { CK(cudaMemsetAsync(d, 0, sizeof(u32), s)); }
   u32 get() { return read_u32(d, s); }
 };

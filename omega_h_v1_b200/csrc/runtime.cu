@@ -577,6 +577,15 @@ void dev_free(void* p, cudaStream_t s)
   CK(cudaFreeAsync(p, s));
 }
 
+void dev_drop(void* p, cudaStream_t s) noexcept
+{
+  try {
+    dev_free(p, s);
+  } catch (...) {
+    cudaGetLastError();
+  }
+}
+
 namespace {
 // a pinned word per host thread for read_u32: a copy into pageable memory
 // goes through the driver's staging buffer and takes several times longer.

@@ -286,8 +286,8 @@ struct Reader {
   {
     if (dtext) {
       cudaStreamSynchronize(s);
-      dev_free(dtext, s);
-      dev_free(dbad, s);
+      dev_drop(dtext, s);
+      dev_drop(dbad, s);
     }
     if (text) cudaFreeHost(text);
   }
@@ -599,7 +599,7 @@ struct Writer {
   {
     if (f) fclose(f);
     cudaStreamSynchronize(s);
-    dev_free(dtext, s);
+    dev_drop(dtext, s);
     if (htext) cudaFreeHost(htext);
   }
   void close()
