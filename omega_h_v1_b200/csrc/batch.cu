@@ -938,6 +938,8 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
       r->u = concat_meshes(parts, s);
       stream_sync(s);
       bs.unions += 1;
+      // (before any mesh is given up to the union: making the controls can fail)
+      r->ctl.reset(new UnionCtl(*r->u));
       r->once = numbered;
       r->dirty.assign(r->u->nseg, 0);
       r->elems.assign(r->u->nseg, 0);
@@ -967,7 +969,6 @@ bool GroupRunner::step(std::vector<Mesh*>& ms, std::vector<SegState>& st,
         }
         seg += o.u->nseg;
       }
-      r->ctl.reset(new UnionCtl(*r->u));
       bs.secs_concat += wall_s() - t;
       at = end;
     }
