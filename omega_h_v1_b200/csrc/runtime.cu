@@ -806,7 +806,8 @@ void Mailbox::post(cudaStream_t s, u32 const* src, u32 nslots, u32 at)
 // of spinning forever.
 
 // Tiles of SCAN_T threads (the tuning table's scan_threads, 256 or 512)
-// times SCAN_ITEMS items (scan_items, 8 or 16). With 8192-element tiles a
+// times SCAN_ITEMS items (scan_items, 8 or 16; 256 x 32 where a scan is long,
+// see LONG_SCAN). With 8192-element tiles a
 // 2M-element scan has 256 tiles, so a tile's look-back meets a published
 // prefix within a few steps (with 2048-element tiles the chain of
 // look-backs, not bandwidth, set the time of the adapt's scans). Scratch
@@ -833,7 +834,8 @@ constexpr u32 SCAN_SPIN_LIMIT = 1u << 24;
 // bytes: loads and stores are coalesced as they stand, the chunks' scans are
 // independent shuffles, and nothing is transposed through shared memory
 // (which took four shared-memory accesses an item and half the issue slots:
-// 15.6 us a launch over a 48^3 adapt, now 13). A launch of one tile needs no ticket, status or clean-up.
+// 28M items 61 us, now 53; 1.5M 8.4, now 7.2). A launch of one tile needs no
+// ticket, status or clean-up.
 __device__ inline void scan_store4(u32* __restrict__ a, size_t gi, u32 n, bool wide, u32 x0,
     u32 x1, u32 x2, u32 x3)
 {
@@ -1200,16 +1202,17 @@ namespace {
 // tiles of a job (one at least: an empty scan still writes out[0] = 0)
 u32 job_tiles(u32 n, u32 tile) { return n ? ceil_div(n, (u64)tile) : 1u; }
 
-// a tile's shape: threads (256 or 512) x items per thread (8 or 16)
+// a tile's shape: threads (256 or 512) x items per thread (8 or 16, or 32)
 struct ScanShape {
   u32 threads, items;
   u32 tile() const { return threads * items; }
 };
 ScanShape tuned_scan_shape() { return {tuned(TK_SCAN_THREADS), tuned(TK_SCAN_ITEMS)}; }
-// A large scan is bound by the tiles' look-backs rather than by its bytes,
-// so it takes the widest tile that keeps three blocks on an SM (28M items:
-// 59 us with 16 items a thread, 51 with 32; 6M: 14 and 12); below LONG_SCAN
-// items the two are level and the smaller tile starts sooner.
+// A long scan is bound by its tiles' waits on one another rather than by its
+// bytes. 256 threads of 32 items have the tile of 512 of 16, 8192 items, but
+// three of them fit an SM where two of the others do (28M items: 66 us with
+// 512 x 16, 53 with 256 x 32; 6M: 15.5 and 13.6). Below LONG_SCAN items the
+// two are level (4.0M: 12.2 both) and the tuning table's shape is taken.
 constexpr u64 LONG_SCAN = 4u << 20;
 ScanShape scan_shape_for(u64 items)
 {
