@@ -648,8 +648,13 @@ def run_batched(args, world, rank, local, cpu_sample=True):
     batch_launches = L.osh_b200_launch_count() - launches0
     clk = clocks.stop()
     fs = G.fp32_stats()
-    same = all(pd[i] == bd[i] == bd64[i] for i in range(len(jobs)))
-    same_conc = all(pd[i] == cd64[i] == cd32[i] for i in range(len(jobs)))
+    wrong = differing_meshes(pd, {"union_fp64": bd64, "union_fp32": bd,
+                                  "concurrent_fp64": cd64, "concurrent_fp32": cd32})
+    for leg, i in wrong:
+        print("bench: rank %d, leg %s: mesh %d (n = %d) differs from one mesh_adapt's"
+              % (rank, leg, i, jobs[i].n), file=sys.stderr)
+    same = not any(leg.startswith("union") for leg, _ in wrong)
+    same_conc = not any(leg.startswith("concurrent") for leg, _ in wrong)
     for b in bases:
         b.close()
     # whole-job figures: every rank's elements over the slowest rank's time
@@ -709,6 +714,21 @@ def run_batched(args, world, rank, local, cpu_sample=True):
     if cpu_sample and not args.no_cpu and rank == 0:
         out["cpu_baseline"] = batched_cpu_sample(jobs)
     return out
+
+
+def differing_meshes(plain, legs):
+    """(leg, mesh) for every mesh that a leg left with another digest than the
+    plain path's, or without one."""
+    return [(leg, i) for leg in sorted(legs) for i in sorted(plain)
+            if legs[leg].get(i) != plain[i]]
+
+
+def all_identical(out):
+    """Whether every identity flag of a line, at any depth, is true."""
+    if isinstance(out, dict):
+        return all(v is True if k in ("identical_to_plain", "identical_concurrent")
+                   else all_identical(v) for k, v in out.items())
+    return True
 
 
 def batched_summary(b):
@@ -1209,6 +1229,9 @@ def main():
     if world > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
+    if rank == 0 and not all_identical(out):
+        sys.exit("bench: a leg's meshes differ from the plain path's (identical_to_plain, "
+                 "identical_concurrent)")
 
 
 if __name__ == "__main__":
