@@ -8,6 +8,8 @@ import threading
 import numpy as np
 import pytest
 
+from conftest import build_gpu
+
 pytestmark = pytest.mark.gpu
 
 # one tile, a few, some hundred and some thousand of them
@@ -62,3 +64,24 @@ def test_mixed_sizes_on_four_streams():
         t.join()
     assert not left, left
     assert bad == [0] * THREADS
+
+
+def test_meshes_of_many_tiles_on_four_streams():
+    """Adapts whose scans have tens of tiles, side by side: each as alone."""
+    import omega_h_v1_b200 as G
+    args = (1 / 3., 0.3, 4, 50)
+    cases = [dict(n=n, seed=n, size=1.0 / n) for n in (32, 30, 28, 26, 24, 22, 20, 18)]
+    base = [build_gpu(**kw) for kw in cases]
+    want = []
+    for m in base:
+        c = m.clone()
+        c.adapt(*args)
+        want.append(c.digest())
+        c.close()
+    for _ in range(5):
+        ms = [m.clone() for m in base]
+        _, status, _ = G.adapt_concurrent(ms, *args, nthreads=4)
+        assert not any(status)
+        assert [m.digest() for m in ms] == want
+        for m in ms:
+            m.close()
