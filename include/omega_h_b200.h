@@ -326,8 +326,9 @@ int osh_b200_exscan_u32(unsigned const* in, unsigned* out, unsigned n, void* str
    cudaStream_t; 0 is the legacy default stream); the caller keeps it alive */
 void osh_b200_set_stream(osh_t m, void* stream) OSH_PUBLIC;
 /* before the caller destroys a stream it gave to osh_b200_set_stream: frees
-   the scratch the library keeps for that stream (in the stream's order), so
-   that it does not outlive it. No mesh may use the stream afterwards. */
+   the scratch the library keeps for that stream (in the stream's order; freed
+   blocks kept for it go with the last mesh on it), so that it does not outlive
+   it. No mesh may use the stream afterwards. */
 void osh_b200_release_stream(void* stream) OSH_PUBLIC;
 
 /* ---- launch shapes (tuning table) ------------------------------------------ */

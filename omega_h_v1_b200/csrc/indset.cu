@@ -21,13 +21,11 @@ PassStats& last_pass_stats()
   return s;
 }
 
-// control words of the single-launch rounds (mailbox slots 44-50)
+// a set's control words (mailbox slots 44-50; their layout is given at
+// k_indset), which come back with the slots before them
 constexpr u32 COOP_CTL_SLOT = 44, COOP_CTL_WORDS = 7;
-// (what the rounds read back: the words below; the control words' layout
-// is given at k_indset)
 static_assert(COOP_CTL_SLOT + COOP_CTL_WORDS == INDSET_FETCH_SLOTS, "mailbox slots");
 
-// also zeroes the control words of the rounds
 // neighbourhood walks: mode 0 = vertices via edges, mode 1 = edges via
 // elements (3D tets or 2D triangles)
 struct Nbrs {
@@ -573,8 +571,8 @@ void launch_indset(u32 n, Nbrs const& g, IndsetIn const& in, double const* good,
 }
 }  // namespace
 
-// number of upward uses walked per round (edges of vertices / elements of
-// edges), for the probe's byte count
+// number of upward uses (edges of vertices / elements of edges), for the mean
+// length of a row
 static u32 read_cached_uses(Mesh& m, u32 ent_dim)
 {
   return ent_dim == 0 ? 2u * m.counts[1] : deg(m.dim, 1) * m.counts[m.dim];

@@ -846,9 +846,9 @@ static u32* choose_refinement(Mesh& m, u32* cand, double qual_floor, double** qu
     m.mb->host[1] = max_u32(cand, ne, s) ? 1 : 0;
   }
   // The independent set runs without first reading back "any good
-  // candidate": with none it settles in its first batch of rounds to the
-  // empty set, and its first read-back brings the flags of mailbox slots
-  // 1-3 with it (one host wait fewer per pass).
+  // candidate": with none the set is empty, and the read-back of its outcome
+  // brings the flags of mailbox slots 1-3 with it (one host wait fewer per
+  // pass).
   u32* ind = nullptr;
   if (ne) {
     IndsetIn in = listed ? *listed : indset_in(m, ne, cand, q);

@@ -1001,7 +1001,9 @@ k_exscan(const __grid_constant__ ScanJobs jobs, unsigned long long* status,
   // published prefix (this thread's exchange) has been performed when the
   // last tile sees it, so the zeros that one writes come after it. (Without
   // the order an exchange still under way could land on a word already
-  // zeroed, and the next scan took the prefix it left for its own.)
+  // zeroed, and the next scan took the prefix it left for its own: on four
+  // busy streams some thousand words in 20,000 launches. It costs 2 us of 53
+  // at 28M items and 1 of 13 at 6M.)
   u32 done = 0;
   if (!single && threadIdx.x == 0) done = count_released(&ticket_and_err[2]);
   bool const marks = newid || list || comp_newid;

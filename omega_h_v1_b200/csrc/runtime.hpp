@@ -15,15 +15,15 @@ namespace osh {
 enum TuneKey : u32 {
   TK_CARRY_GROUP = 0,    // lanes per long carried upward row: 4, 8, 16
   TK_VERT_GROUP,         // lanes per vertex row, coarsening vertex kernels: 4, 8, 16
-  TK_INDSET_VERT_GROUP,  // lanes per vertex, independent-set rounds: 4, 8, 16
-  TK_INDSET_EDGE_GROUP,  // lanes per edge (3D), independent-set rounds: 1, 2, 4, 8
+  TK_INDSET_VERT_GROUP,  // lanes per vertex, independent set, long lists: 4, 8, 16
+  TK_INDSET_EDGE_GROUP,  // lanes per edge (3D), the same: 1, 2, 4, 8
   TK_QUALITY_BLOCK,      // threads per block, quality kernels: 64, 128, 256, 512
   TK_GATHER_BLOCK,       // threads per block, carry / search / copy kernels: 128, 256, 512
   TK_SCAN_ITEMS,         // items per thread of a scan tile: 8, 16
   TK_SCAN_THREADS,       // threads per scan tile: 256, 512
-  TK_INDSET_BLOCKS,      // blocks per SM of the one-launch independent set (each
-                         // round ends in a grid barrier that every block joins;
-                         // 0: as many as fit): 0, 1, 2, 4
+  TK_INDSET_BLOCKS,      // blocks per SM of the independent set's cooperative
+                         // launch, whose warps wait on one another (0: as many as
+                         // fit): 0, 1, 2, 4
   TK_SMALL_MESH_ELEMS,   // concurrent many-mesh adapt: meshes estimated below this
                          // many elements are adapted together in batch unions
                          // (0: none): 0, 25000, 50000 (default), 100000, 200000
