@@ -14,7 +14,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 
 #include "mesh.hpp"
 
@@ -501,7 +500,7 @@ __global__ void k_split_uses(u32 n, UseDiv div, u32 const* __restrict__ uses,
   dirs[j] = u - h * div.lph;
 }
 
-constexpr u32 KEPT_COUNTS = 1u << 20;  // (4 MB a stream)
+constexpr u32 KEPT_COUNTS = 1u << 20;  // (4 MB a stream and host thread)
 
 void up_from_down_unsorted(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* loh,
     UpAdj& out, cudaStream_t s)
@@ -510,16 +509,11 @@ void up_from_down_unsorted(u32 high, u32 low, u32 nhighs, u32 nlows, u32 const* 
   u32 nuses = nhighs * lph;
   out.offs = dalloc<u32>((size_t)nlows + 1, s);
   out.uses = dalloc<u32>(nuses, s);
-  // The counts of up to KEPT_COUNTS rows are the stream's kept ones, zero on
+  // The counts of up to KEPT_COUNTS rows are kept ones, zero on
   // entry (the fill takes them back down to zero): a memset waits for what
   // is before it and holds back what is after, 3 us of a small mesh's
   // derivation that its bandwidth does not explain.
-  // Host threads may share a stream: the one that has the counts has them
-  // until its fill is launched.
-  static std::mutex counts_of[16];
-  std::unique_lock<std::mutex> hold(counts_of[((uintptr_t)s >> 4) % 16], std::defer_lock);
   bool const kept = nlows <= KEPT_COUNTS && !stream_captures(s);
-  if (kept) hold.lock();
   u32* cnt = kept ? stream_zero_scratch(KEPT_USES, (size_t)nlows + 1, s)
                   : dalloc<u32>((size_t)nlows + 1, s);
   if (!kept) CK(cudaMemsetAsync(cnt, 0, sizeof(u32) * ((size_t)nlows + 1), s));

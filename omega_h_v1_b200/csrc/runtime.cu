@@ -1049,15 +1049,52 @@ k_exscan(const __grid_constant__ ScanJobs jobs, unsigned long long* status,
 }
 
 namespace {
-// Scratch of the scans issued on each stream ([ticket, error, done, pad]
-// then two words per tile), zero between scans: the scan kernel's last tile
-// clears it, so no scan pays for a memset. Scans on one stream run one
-// after another; each stream has its own, freed by release_stream_scratch
-// when the stream goes.
-std::mutex g_scan_mu;
-std::map<std::pair<int, cudaStream_t>, ScanScratch>& scan_scratches()
+// The calling host thread's number: small, its own while it runs, another
+// thread's after it. Host threads may share a stream, where each thread's
+// kernels run in its order but among the others': what one thread's kernel
+// leaves in a scratch for its next (counts, marks) must be out of the others'
+// reach, so every scratch is a (stream, host thread)'s. A thread that gets
+// another's number after its end comes after it on the stream.
+struct HostThread {
+  static std::mutex& mu()
+  {
+    static auto* m = new std::mutex();
+    return *m;
+  }
+  static std::vector<bool>& taken()
+  {
+    static auto* v = new std::vector<bool>();
+    return *v;
+  }
+  u32 id = 0;
+  HostThread()
+  {
+    std::lock_guard<std::mutex> g(mu());
+    while (id < taken().size() && taken()[id]) ++id;
+    if (id == taken().size()) taken().push_back(false);
+    taken()[id] = true;
+  }
+  ~HostThread()
+  {
+    std::lock_guard<std::mutex> g(mu());
+    taken()[id] = false;
+  }
+};
+u32 host_thread()
 {
-  static auto* m = new std::map<std::pair<int, cudaStream_t>, ScanScratch>();
+  static thread_local HostThread t;
+  return t.id;
+}
+
+// Scratch of the scans issued on each stream by each host thread ([ticket,
+// error, done, pad] then two words per tile), zero between scans: the scan
+// kernel's last tile clears it, so no scan pays for a memset. Freed by
+// release_stream_scratch when the stream goes.
+std::mutex g_scan_mu;
+using ScanKey = std::tuple<int, cudaStream_t, u32>;  // device, stream, host thread
+std::map<ScanKey, ScanScratch>& scan_scratches()
+{
+  static auto* m = new std::map<ScanKey, ScanScratch>();
   return *m;
 }
 
@@ -1067,7 +1104,7 @@ u32* stream_scan_scratch(size_t words, cudaStream_t s)
   CK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> g(g_scan_mu);
   auto& all = scan_scratches();
-  ScanScratch& sc = all[{dev, s}];
+  ScanScratch& sc = all[ScanKey{dev, s, host_thread()}];
   if (sc.words < words) {
     size_t want = std::max(words, (size_t)4096);
     void* q = pool_alloc(want * sizeof(u32), s);
@@ -1084,15 +1121,29 @@ u32* stream_scan_scratch(size_t words, cudaStream_t s)
   return sc.p;
 }
 
-// the stream's scan scratch (p null: it has none)
+// the calling thread's scan scratch on the stream (p null: it has none)
 ScanScratch find_scan_scratch(cudaStream_t s)
 {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> g(g_scan_mu);
   auto& all = scan_scratches();
-  auto it = all.find({dev, s});
+  auto it = all.find(ScanKey{dev, s, host_thread()});
   return it != all.end() ? it->second : ScanScratch();
+}
+
+// every host thread's
+std::vector<ScanScratch> stream_scan_scratches(cudaStream_t s)
+{
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::vector<ScanScratch> v;
+  std::lock_guard<std::mutex> g(g_scan_mu);
+  auto& all = scan_scratches();
+  for (auto it = all.lower_bound(ScanKey{dev, s, 0}); it != all.end() &&
+       std::get<0>(it->first) == dev && std::get<1>(it->first) == s; ++it)
+    if (it->second.p) v.push_back(it->second);
+  return v;
 }
 
 // a scan of the stream gave up: its scratch made anew, and the failure
@@ -1104,28 +1155,29 @@ ScanScratch find_scan_scratch(cudaStream_t s)
 }  // namespace
 
 namespace {
-// Per-stream scratch kept between calls, one per key (what it holds); see
-// stream_zero_scratch and stream_marks
+// Scratch kept between calls, one per stream, host thread and key (what it
+// holds); see stream_zero_scratch and stream_marks
 struct KeptScratch {
   u32* p = nullptr;
   size_t words = 0;
   u32 gen = 0;
 };
 std::mutex g_kept_mu;
-using KeptKey = std::tuple<int, cudaStream_t, u32>;
+using KeptKey = std::tuple<int, cudaStream_t, u32, u32>;  // the last two: host thread, key
 std::map<KeptKey, KeptScratch>& kept_scratches()
 {
   static auto* m = new std::map<KeptKey, KeptScratch>();
   return *m;
 }
 
-// at least `words` words for (this device, s, key), zeroed when (re)made
+// at least `words` words for (this device, s, this thread, key), zeroed when
+// (re)made
 KeptScratch& kept_scratch(u32 key, size_t words, cudaStream_t s)
 {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   auto& all = kept_scratches();
-  KeptScratch& sc = all[{dev, s, key}];
+  KeptScratch& sc = all[KeptKey{dev, s, host_thread(), key}];
   if (sc.words < words) {
     size_t want = std::max(words + words / 4, (size_t)4096);
     // (the old one stays in place until there is a new one)
@@ -1167,15 +1219,15 @@ void release_stream_scratch(cudaStream_t s)
   {
     std::lock_guard<std::mutex> g(g_scan_mu);
     auto& all = scan_scratches();
-    auto it = all.find({dev, s});
-    if (it != all.end()) {
+    for (auto it = all.lower_bound(ScanKey{dev, s, 0}); it != all.end() &&
+         std::get<0>(it->first) == dev && std::get<1>(it->first) == s;) {
       if (it->second.p) cudaFreeAsync(it->second.p, s);
-      all.erase(it);
+      it = all.erase(it);
     }
   }
   std::lock_guard<std::mutex> g(g_kept_mu);
   auto& all = kept_scratches();
-  for (auto it = all.lower_bound(KeptKey{dev, s, 0}); it != all.end() &&
+  for (auto it = all.lower_bound(KeptKey{dev, s, 0, 0}); it != all.end() &&
        std::get<0>(it->first) == dev && std::get<1>(it->first) == s;) {
     if (it->second.p) cudaFreeAsync(it->second.p, s);
     it = all.erase(it);
@@ -1272,17 +1324,17 @@ void exscan_u32(u32 const* in, u32* out, u32 n, cudaStream_t s, u32* total_to, u
   exscan_jobs(&j, 1, s);
 }
 
-// The scans of one stream record a look-back that gave up in word 1 of that
-// stream's scratch (the last tile clears words 0 and 2 only), so a stream's
-// check sees its own scans' timeouts and no other stream's.
+// The scans of one stream record a look-back that gave up in word 1 of their
+// scratch (the last tile clears words 0 and 2 only), so a stream's check sees
+// its own scans' timeouts and no other stream's.
 void check_device_timeouts(cudaStream_t s)
 {
-  ScanScratch const sc = find_scan_scratch(s);
-  if (!sc.p) return;
   u32* h = static_cast<u32*>(pinned_scratch());
-  CK(cudaMemcpyAsync(h, sc.p + 1, sizeof(u32), cudaMemcpyDeviceToHost, s));
-  stream_sync(s);
-  if (*h) scan_gave_up(sc, s);
+  for (ScanScratch const& sc : stream_scan_scratches(s)) {
+    CK(cudaMemcpyAsync(h, sc.p + 1, sizeof(u32), cudaMemcpyDeviceToHost, s));
+    stream_sync(s);
+    if (*h) scan_gave_up(sc, s);
+  }
 }
 
 int selftest_scan_wait(u32 spin_limit)

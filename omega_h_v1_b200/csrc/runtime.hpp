@@ -86,12 +86,12 @@ struct ScanJobs {
 };
 void exscan_jobs(ScanJob const* jobs, u32 njobs, cudaStream_t s);
 
-// Scratch kept per (device, stream, key) between calls, zeroed when made or
-// grown. stream_zero_scratch: the caller leaves it zero again after each use
-// (keys KEPT_ROWS0 and KEPT_ROWS1: the search rows' counts, KEPT_USES: the
-// upward rows', which the rows' fill counts back down to zero). stream_marks: entries stamped with a
-// generation of the (stream, key), returned in *gen (never 0) and new on
-// every call, so no entry of an earlier use passes for a mark of this one
+// Scratch kept per (device, stream, host thread, key) between calls, zeroed
+// when made or grown. stream_zero_scratch: the caller leaves it zero again
+// after each use (keys KEPT_ROWS0 and KEPT_ROWS1: the search rows' counts,
+// KEPT_USES: the upward rows', which the rows' fill counts back down to
+// zero). stream_marks: entries stamped with a generation of the scratch,
+// returned in *gen (never 0) and new on every call, so no entry of an earlier use passes for a mark of this one
 // (KEPT_MARKS: the products' vertices of a pass's searches; KEPT_FUSED + d:
 // the collapses' fused entities of dimension d; KEPT_SPLIT + d: a
 // refinement's split domain entities of dimension d).
