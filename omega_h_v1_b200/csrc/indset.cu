@@ -107,7 +107,9 @@ struct NbrBatch {
   static constexpr u32 USES = PER == 1 ? 2 : 1, NB = PER * USES;
 };
 
-// up to NB neighbours of entity i from its entries j, j + G, ... (INV: none)
+// up to NB neighbours of entity i from its entries j, j + G, ... (INV: none;
+// swaps in a tangled mesh can leave an edge whose ends are one vertex, which
+// is not its own neighbour)
 template <int G, u32 PER>
 __device__ inline void load_neighbors(Nbrs const& g, u32 i, u32 j, u32 re, u32* o)
 {
@@ -117,6 +119,9 @@ __device__ inline void load_neighbors(Nbrs const& g, u32 i, u32 j, u32 re, u32* 
     for (u32 k = 0; k < 2; ++k) u[k] = j + k * G < re ? g.uses[j + k * G] : INV;
 #pragma unroll
     for (u32 k = 0; k < 2; ++k) o[k] = u[k] != INV ? g.down[u[k] ^ 1u] : INV;
+#pragma unroll
+    for (u32 k = 0; k < 2; ++k)
+      if (o[k] == i) o[k] = INV;
   } else {
     u32 const use = g.uses[j];
     u32 const* ds = g.down + (use - use % PER);
@@ -149,6 +154,11 @@ __device__ inline Walk walk_neighbors(Nbrs const& g, u32 i, Key mykey, u32 lg, u
   Key bk = 0;
   bool in = false, worse = false;
   auto id_of = [&](u32 o) { return glob ? glob[o] : (u64)o; };
+  // (numbers that a caller gave twice: by index, so that no two wait for each other)
+  auto later = [&](u32 a, u32 b) {
+    u64 const x = id_of(a), y = id_of(b);
+    return x > y || (x == y && a > b);
+  };
   for (u32 j = rb + lg; j < re; j += STEP) {
     u32 o[NB];
     Key ko[NB];
@@ -160,9 +170,9 @@ __device__ inline Walk walk_neighbors(Nbrs const& g, u32 i, Key mykey, u32 lg, u
     for (u32 k = 0; k < NB; ++k) {
       if (!ko[k]) continue;
       if (key_undecided(ko[k])) {
-        if (ko[k] < mykey || (ko[k] == mykey && id_of(o[k]) > id_of(i)))
+        if (ko[k] < mykey || (ko[k] == mykey && later(o[k], i)))
           worse = true;
-        else if (blocker == INV || ko[k] > bk || (ko[k] == bk && id_of(o[k]) < id_of(blocker))) {
+        else if (blocker == INV || ko[k] > bk || (ko[k] == bk && later(blocker, o[k]))) {
           blocker = o[k];
           bk = ko[k];
         }
@@ -192,7 +202,7 @@ __device__ inline Walk walk_neighbors(Nbrs const& g, u32 i, Key mykey, u32 lg, u
     u32 const b2 = __shfl_xor_sync(gmask, blocker, o);
     Key const k2 = __shfl_xor_sync(gmask, bk, o);
     if (b2 != INV && b2 != blocker &&
-        (blocker == INV || k2 > bk || (k2 == bk && id_of(b2) < id_of(blocker)))) {
+        (blocker == INV || k2 > bk || (k2 == bk && later(blocker, b2)))) {
       blocker = b2;
       bk = k2;
     }
