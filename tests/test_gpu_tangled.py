@@ -50,10 +50,14 @@ def test_an_edge_of_one_vertex():
 
 def test_global_numbers_given_twice():
     """They leave ties of equal qualities open; the set is settled by index."""
-    m = build_gpu(5, pert=0, size=0.5 / 5, parallel=True)
+    m = build_gpu(8, pert=0, size=5.0 / 8, parallel=True)   # (exact coordinates: ties everywhere)
     for d in range(4):
         m.set_globals(d, np.zeros(m.count(d), np.uint64))
-    ind = m.refine_sets(0.0)["indset"]
-    assert ind.any()
-    edges = m.down(3, 1).reshape(-1, 6)
-    assert (ind[edges].sum(axis=1) <= 1).all()     # no two in one tet
+    sets = m.coarsen_sets(0.0, 1 / 3.)
+    ind, cand, edges = sets["indset"], sets["candidates"], m.down(1, 0).reshape(-1, 2)
+    a, b = edges.T
+    assert not (ind[a] & ind[b]).any()
+    near = np.zeros(m.count(0), bool)
+    near[a[ind[b] == 1]] = True
+    near[b[ind[a] == 1]] = True
+    assert cand.any() and (ind[cand == 1] | near[cand == 1]).all()
